@@ -409,8 +409,8 @@ def kernel_rooflines(pg, torch, grid, tables, nb, precision, stream):
     nx, ny, nz = grid.n
     hbytes = 8.0 * N * (2 * nb + 1)
     flops = N * nb * (2 * (nx + ny + nz) + 2)
-    hx = {"kernel": f"pg_hx mixed: {grid.hx_plan(nb)}" if mixed else "k_hx_fp64",
-          "bound": "hbm" if mixed else "fp64", "ms_per_launch": ms, "algorithmic_bytes": hbytes,
+    hx = {"kernel": f"pg_hx mixed: {grid.hx_plan(nb)}" if mixed else "pg_hx FP64: k_slice_axis x 3",
+          "bound": "hbm" if mixed else "integer pipes and tensor cores", "ms_per_launch": ms, "algorithmic_bytes": hbytes,
           "vectors_per_launch": nb, "l2": f"operands rotated over {kh} copies (more than twice the L2 between reuses)"}
     if mixed:
         hx.update(achieved=hbytes / (ms * 1e-3) / 1e9, peak=peaks["hbm_gbs"], unit="GB/s",
@@ -418,7 +418,8 @@ def kernel_rooflines(pg, torch, grid, tables, nb, precision, stream):
                   traffic=KERNEL_TRAFFIC.get(("hx", tuple(grid.n), nb, precision)))
     else:
         hx.update(achieved=flops / (ms * 1e-3) / 1e12, peak=1.0, unit="TFLOP/s", frac=flops / (ms * 1e-3) / 1e12,
-                  peak_source="FP64 FMA pipe of this GB300, measured with a DFMA loop (not in MEASURED_PEAKS.json)")
+                  peak_source="FP64 FMA pipe of this GB300, measured with a DFMA loop (not in MEASURED_PEAKS.json): the "
+                              "rate of plain FP64 multiply-adds; the slices run on the tensor cores and can exceed it")
     return gram, hx, comb
 
 

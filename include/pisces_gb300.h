@@ -268,7 +268,10 @@ pg_status pg_water_default_tables(int nw, const double* sites, const double* cha
 /* ------------------------------------------------------------------- H * X */
 
 /* Y = H X for nvec vectors: H = V + Tx (+) Ty (+) Tz.  precision PG_FP64:
- * FP64 arithmetic throughout; PG_MIXED: kinetic contractions as split-TF32
+ * FP64 throughout, the kinetic contractions from exact slices of both
+ * operands on the tensor cores (each rounded once); the call returns once
+ * its launches are queued, and pg_grid_check reports a completion wait that
+ * timed out.  PG_MIXED: kinetic contractions as split FP16 or TF32
  * tensor-core products accumulated in FP32, V*X in FP64.  nvec = 0 does
  * nothing and accepts null X and Y.  Replaces DVR::MatrixTimesVector applied
  * vector by vector (src/mtx.cpp:22-109, src/davdriver.cpp:67-78). */

@@ -180,6 +180,18 @@ inline __host__ __device__ int tc_kchunk(int n) {
   return ((kpad + nch - 1) / nch + 7) / 8 * 8;
 }
 
+// Right operand of an axis contraction: the digits of a row-major n x n
+// matrix as K-major core-matrix images (tc16_kmajor_off), one block per
+// (K chunk, N chunk) holding the slices one after the other, so that a
+// kernel fetches a block in one bulk copy.
+struct SliceMat {
+  const unsigned char* img = nullptr;  // in the grid's sl_img
+  int n = 0, tau = 0;            // entries are digits of A 2^tau
+  int nch = 1, kc = 16;          // K chunks and their width (a multiple of 16)
+  int nnc = 1, nc = 16;          // N chunks and their rows (a multiple of 16)
+  size_t block_bytes() const { return (size_t)7 * nc * kc * 2; }
+};
+
 }  // namespace pg
 
 // The grid handle: sizes, host copies of the 1-D data and device kinetic matrices.
@@ -192,6 +204,10 @@ struct pg_grid {
   std::vector<double> x[3];        // grid points per axis
   std::vector<double> t[3];        // full symmetric kinetic matrices, n x n row-major (host)
   pg::DevBuf<double> t_dev[3];     // same, FP64, on the device
+  // digit images of the kinetic matrices and of the eigenbasis transforms
+  // (forward Q^T, backward Q) for the FP64 axis contractions (pg_slice.cu)
+  pg::SliceMat t_sl[3], q_sl[3], qb_sl[3];
+  pg::DevBuf<unsigned char> sl_img;
   // TF32-rounded high part and the TF32-rounded remainder T - hi, each as
   // tensor-core operand images (tc_kmajor_off layout, one tc_npad x tc_kchunk
   // image per K chunk)
@@ -256,10 +272,11 @@ struct HxParams {
 };
 HxParams hx_params(const pg_grid* g, int nvec);
 // Single-axis contraction Y = A x_axis X for nvec vectors, A an n_axis x
-// n_axis matrix given in both FP64 and split-TF32 form; mode 0: Y = A X,
-// mode 1: Y += A X.  FP64 or tensor-core arithmetic per precision.
-pg_status axis_apply(const pg_grid* g, int axis, const double* A64, const float* Ahi, const float* Alo,
-                     const double* x, double* y, int nvec, int mode, int precision, cudaStream_t st);
+// n_axis matrix given in FP64, as digit images and in split-TF32 form; mode
+// 0: Y = A X, mode 1: Y += A X.  FP64 (slices) or split TF32 per precision.
+pg_status axis_apply(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const float* Ahi,
+                     const float* Alo, const double* x, double* y, int nvec, int mode, int precision,
+                     cudaStream_t st);
 // H*X without the public call's synchronous status check (pg_hx.cu); the
 // caller checks check_tc_error() at its own synchronisation points.
 // unit: every value of X is known to lie in [-1, 1] (the Davidson's

@@ -262,9 +262,8 @@ extern "C" pg_status pg_kinetic_precondition(const pg_grid* g, double* R, int k,
   PG_TRY(sg.alloc((size_t)k));
   PG_CUDA_TRY(cudaMemcpyAsync(sg.p, sigma, sizeof(double) * k, cudaMemcpyHostToDevice, st));
   PG_TRY(pg::kinetic_precondition(g, R, k, sg.p, w.p, w.p + (long)k * g->N, precision, st));
-  // the scratch is freed on return: finish with it first
-  PG_CUDA_TRY(cudaStreamSynchronize(st));
-  return precision == PG_MIXED ? pg::check_tc_error(g, st) : PG_OK;
+  // waits for the stream: the scratch is freed on return
+  return pg::check_tc_error(g, st);
 }
 
 extern "C" pg_status pg_grid_set_precond_kernel(pg_grid* g, int kind) {
@@ -517,9 +516,9 @@ pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double*
   for (int a = 0; a < 3; ++a) dmin += 0.5 * (M_PI / g->L[a]) * (M_PI / g->L[a]);
   if (pr == PG_MIXED && g->pc_kernel != 1 && kin_f16_ok(g) && (((uintptr_t)R | (uintptr_t)w1 | (uintptr_t)w2) & 15u) == 0)
     return kin_f16(g, R, w1, w2, k, sigma_dev, 0.1 * dmin, st);
-  PG_TRY(axis_apply(g, 2, g->q_dev[2].p, g->q_hi[2].p, g->q_lo[2].p, R, w1, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 1, g->q_dev[1].p, g->q_hi[1].p, g->q_lo[1].p, w1, w2, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 0, g->q_dev[0].p, g->q_hi[0].p, g->q_lo[0].p, w2, w1, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 2, g->q_sl[2], g->q_dev[2].p, g->q_hi[2].p, g->q_lo[2].p, R, w1, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 1, g->q_sl[1], g->q_dev[1].p, g->q_hi[1].p, g->q_lo[1].p, w1, w2, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 0, g->q_sl[0], g->q_dev[0].p, g->q_hi[0].p, g->q_lo[0].p, w2, w1, k, 0, pr, st));
   for (int v0 = 0; v0 < k; v0 += 16) {  // at most 16 vectors per launch
     const int kk = std::min(16, k - v0);
 #define PG_KIN_SCALE(NRV)                                                                                     \
@@ -534,9 +533,9 @@ pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double*
 #undef PG_KIN_SCALE
     PG_TRY(check_launch("k_kin_scale"));
   }
-  PG_TRY(axis_apply(g, 2, g->qb_dev[2].p, g->qb_hi[2].p, g->qb_lo[2].p, w1, w2, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 1, g->qb_dev[1].p, g->qb_hi[1].p, g->qb_lo[1].p, w2, w1, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 0, g->qb_dev[0].p, g->qb_hi[0].p, g->qb_lo[0].p, w1, R, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 2, g->qb_sl[2], g->qb_dev[2].p, g->qb_hi[2].p, g->qb_lo[2].p, w1, w2, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 1, g->qb_sl[1], g->qb_dev[1].p, g->qb_hi[1].p, g->qb_lo[1].p, w2, w1, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 0, g->qb_sl[0], g->qb_dev[0].p, g->qb_hi[0].p, g->qb_lo[0].p, w1, R, k, 0, pr, st));
   return PG_OK;
 }
 
@@ -1065,7 +1064,6 @@ pg_status solve_with(const pg_grid* g, const double* v, const pg_solve_params* p
   const pg_status conv_status = s;
   if (nconv < nr)  // not converged: report the current Ritz values
     for (int r = 0; r < nr && r < (int)d.sse.size(); ++r) evals[r] = d.sse[r];
-  if (p->precision == PG_MIXED) PG_TRY(check_tc_error(g, st));
   if (p->precision == PG_MIXED && p->refine == 1) {
     // FP64 Rayleigh-Ritz on the converged vectors: Z = H B with the FP64
     // operator, S = B^T Z, eigenpairs of S rotate the vectors.
@@ -1085,7 +1083,7 @@ pg_status solve_with(const pg_grid* g, const double* v, const pg_solve_params* p
   } else {
     PG_CUDA_TRY(cudaMemcpyAsync(evecs, B.p, sizeof(double) * N * nr, cudaMemcpyDeviceToDevice, st));
   }
-  PG_CUDA_TRY(cudaStreamSynchronize(st));
+  PG_TRY(check_tc_error(g, st));  // waits for the stream
   if (stats) {
     memset(stats, 0, sizeof(*stats));
     stats->nconv = nconv;

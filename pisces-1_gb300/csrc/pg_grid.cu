@@ -7,7 +7,7 @@
 #include <cstring>
 #include <vector>
 
-#include "pg_common.cuh"
+#include "pg_slice.cuh"
 
 namespace pg {
 
@@ -373,6 +373,13 @@ extern "C" pg_status pg_grid_create_dvr(const int n[3], const double L[3], int d
     pg::set_error("pg_grid_create: allocation of the status word failed");
     delete g;
     return PG_OOM;
+  }
+  {
+    const pg_status ss = pg::slice_grid(g);
+    if (ss != PG_OK) {
+      delete g;
+      return ss;
+    }
   }
   *out = g;
   return PG_OK;
