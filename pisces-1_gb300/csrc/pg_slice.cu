@@ -213,7 +213,6 @@ __global__ void __launch_bounds__(kST, 1)
   }
   const uint32_t lbo = 128, sbo = (uint32_t)koct * 128u;
   const uint32_t a_slice = (uint32_t)kLines * (uint32_t)A.kc * 2u;
-  const uint32_t idesc = (1u << 4) | ((uint32_t)(A.nc >> 3) << 17) | ((uint32_t)(kLines >> 4) << 24);
   for (int c = c_first; c < c_end && ok; ++c) {
     for (int h = 0; h < A.nch && ok; ++h) {
       if (A.rebuild || c == c_first) {
@@ -247,17 +246,24 @@ __global__ void __launch_bounds__(kST, 1)
       if (tid == 0) {
         if (mbar_wait(smem_u32(&bar_b), (uint32_t)(waits_b & 1))) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // neighbouring products go to different accumulators: a product
-          // into the accumulator of the one before it would wait for that one
+          // digit i of the lines against digits 0 .. 6 - i of the matrix,
+          // which lie one under the other in shared memory as one operand of
+          // (7 - i) nc rows, into accumulators i .. 6, which lie side by side:
+          // at most 256 columns an instruction (one product at a time read
+          // the lines' digits 28 times instead of 10: 7700 cycles a tile
+          // of 64 x 64 against 6600)
           for (int kk = 0; kk < (koct >> 1); ++kk) {
 #pragma unroll
             for (int i = 0; i < NS; ++i) {
               const uint64_t da = smem_desc(sA + (uint32_t)i * a_slice + (uint32_t)kk * 256u, lbo, sbo);
-#pragma unroll
-              for (int j = 0; i + j < pg::kSliceAcc; ++j)
-                mma_f16(tmem + (uint32_t)((i + j) * A.nc), da,
-                        smem_desc(sB + (uint32_t)j * A.slice_b + (uint32_t)kk * 256u, lbo, sbo), idesc,
+              for (int c0 = 0; c0 < (NS - i) * A.nc; c0 += 256) {
+                const int cols = (NS - i) * A.nc - c0 < 256 ? (NS - i) * A.nc - c0 : 256;
+                const uint32_t idesc =
+                    (1u << 4) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kLines >> 4) << 24);
+                mma_f16(tmem + (uint32_t)(i * A.nc + c0), da,
+                        smem_desc(sB + (uint32_t)(c0 >> 3) * sbo + (uint32_t)kk * 256u, lbo, sbo), idesc,
                         (h > 0 || kk > 0 || i > 0) ? 1u : 0u);
+              }
             }
           }
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
