@@ -273,16 +273,18 @@ struct HxParams {
 HxParams hx_params(const pg_grid* g, int nvec);
 // Single-axis contraction Y = A x_axis X for nvec vectors, A an n_axis x
 // n_axis matrix given in FP64, as digit images and in split-TF32 form; mode
-// 0: Y = A X, mode 1: Y += A X.  FP64 (slices) or split TF32 per precision.
+// 0: Y = A X, mode 1: Y += A X.  FP64 (slices, or in_order: chains of FP64
+// multiply-adds) or split TF32 per precision.
 pg_status axis_apply(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const float* Ahi,
                      const float* Alo, const double* x, double* y, int nvec, int mode, int precision,
-                     cudaStream_t st);
+                     cudaStream_t st, bool in_order = false);
 // H*X without the public call's synchronous status check (pg_hx.cu); the
 // caller checks check_tc_error() at its own synchronisation points.
 // unit: every value of X is known to lie in [-1, 1] (the Davidson's
 // orthonormal basis vectors), which lets the FP16-split kernel use a fixed
 // operand scale.
+// in_order (FP64): chains of FP64 multiply-adds instead of slices.
 pg_status hx(const pg_grid* g, const double* v, const double* x, double* y, int nvec, int precision,
-             cudaStream_t st, bool unit = false);
+             cudaStream_t st, bool unit = false, bool in_order = false);
 pg_status check_tc_error(const pg_grid* g, cudaStream_t st);
 }  // namespace pg

@@ -497,7 +497,8 @@ pg_status kinetic_precondition(pg_davidson* d, double* R, int k, const double* s
   const long N = d->pc_grid->N;
   PG_TRY(d->pc_w1.ensure((size_t)k * N));
   PG_TRY(d->pc_w2.ensure((size_t)k * N));
-  return pg::kinetic_precondition(d->pc_grid, R, k, sigma_dev, d->pc_w1.p, d->pc_w2.p, d->pc_precision, st);
+  return pg::kinetic_precondition(d->pc_grid, R, k, sigma_dev, d->pc_w1.p, d->pc_w2.p, d->pc_precision, st,
+                                  d->nroots > 1);
 }
 
 }  // namespace
@@ -509,16 +510,16 @@ pg_status kinetic_precondition(pg_davidson* d, double* R, int k, const double* s
 // form runs them as one FP16-split tensor-core kernel where the grid allows
 // (k_kin_f16), else as six axis passes and a scale kernel.
 pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double* sigma_dev, double* w1, double* w2,
-                               int pr, cudaStream_t st) {
+                               int pr, cudaStream_t st, bool in_order) {
   const long N = g->N;
   // the smallest kinetic level, a scale for the denominator floor
   double dmin = 0;
   for (int a = 0; a < 3; ++a) dmin += 0.5 * (M_PI / g->L[a]) * (M_PI / g->L[a]);
   if (pr == PG_MIXED && g->pc_kernel != 1 && kin_f16_ok(g) && (((uintptr_t)R | (uintptr_t)w1 | (uintptr_t)w2) & 15u) == 0)
     return kin_f16(g, R, w1, w2, k, sigma_dev, 0.1 * dmin, st);
-  PG_TRY(axis_apply(g, 2, g->q_sl[2], g->q_dev[2].p, g->q_hi[2].p, g->q_lo[2].p, R, w1, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 1, g->q_sl[1], g->q_dev[1].p, g->q_hi[1].p, g->q_lo[1].p, w1, w2, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 0, g->q_sl[0], g->q_dev[0].p, g->q_hi[0].p, g->q_lo[0].p, w2, w1, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 2, g->q_sl[2], g->q_dev[2].p, g->q_hi[2].p, g->q_lo[2].p, R, w1, k, 0, pr, st, in_order));
+  PG_TRY(axis_apply(g, 1, g->q_sl[1], g->q_dev[1].p, g->q_hi[1].p, g->q_lo[1].p, w1, w2, k, 0, pr, st, in_order));
+  PG_TRY(axis_apply(g, 0, g->q_sl[0], g->q_dev[0].p, g->q_hi[0].p, g->q_lo[0].p, w2, w1, k, 0, pr, st, in_order));
   for (int v0 = 0; v0 < k; v0 += 16) {  // at most 16 vectors per launch
     const int kk = std::min(16, k - v0);
 #define PG_KIN_SCALE(NRV)                                                                                     \
@@ -533,9 +534,9 @@ pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double*
 #undef PG_KIN_SCALE
     PG_TRY(check_launch("k_kin_scale"));
   }
-  PG_TRY(axis_apply(g, 2, g->qb_sl[2], g->qb_dev[2].p, g->qb_hi[2].p, g->qb_lo[2].p, w1, w2, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 1, g->qb_sl[1], g->qb_dev[1].p, g->qb_hi[1].p, g->qb_lo[1].p, w2, w1, k, 0, pr, st));
-  PG_TRY(axis_apply(g, 0, g->qb_sl[0], g->qb_dev[0].p, g->qb_hi[0].p, g->qb_lo[0].p, w1, R, k, 0, pr, st));
+  PG_TRY(axis_apply(g, 2, g->qb_sl[2], g->qb_dev[2].p, g->qb_hi[2].p, g->qb_lo[2].p, w1, w2, k, 0, pr, st, in_order));
+  PG_TRY(axis_apply(g, 1, g->qb_sl[1], g->qb_dev[1].p, g->qb_hi[1].p, g->qb_lo[1].p, w2, w1, k, 0, pr, st, in_order));
+  PG_TRY(axis_apply(g, 0, g->qb_sl[0], g->qb_dev[0].p, g->qb_hi[0].p, g->qb_lo[0].p, w1, R, k, 0, pr, st, in_order));
   return PG_OK;
 }
 
@@ -1107,7 +1108,7 @@ pg_status solve_with(const pg_grid* g, const double* v, const pg_solve_params* p
     pg_solve_stats s2;
     const pg_status s = solve_with(
         g, v, &q, evals, evecs, &s2, st,
-        [&](const double* x, double* y, int nvec) { return hx(g, v, x, y, nvec, PG_FP64, st, true); }, &ws);
+        [&](const double* x, double* y, int nvec) { return hx(g, v, x, y, nvec, PG_FP64, st, true, q.nroots > 1); }, &ws);
     if (stats) {
       stats->nconv = s2.nconv;
       stats->n_matvec += s2.n_matvec;
@@ -1159,9 +1160,11 @@ extern "C" pg_status pg_solve(const pg_grid* g, const double* v, const pg_solve_
   using namespace pg;
   cudaStream_t st = as_stream(stream);
   const int prec = p ? p->precision : PG_FP64;
+  const bool in_order = p && p->nroots > 1;
   return solve_with(
       g, v, p, evals, evecs, stats, st,
-      [&](const double* x, double* y, int nvec) { return hx(g, v, x, y, nvec, prec, st, true); }, nullptr);
+      [&](const double* x, double* y, int nvec) { return hx(g, v, x, y, nvec, prec, st, true, in_order); },
+      nullptr);
 }
 
 namespace pg {
@@ -1232,7 +1235,8 @@ extern "C" pg_status pg_cluster_solve(const int n[3], const double L[3], int nw,
   const double* vp = v.p;
   pg_status s = solve_with(
       g, vp, p, evals, vec.p, stats, st,
-      [&](const double* x, double* y, int nvec) { return hx(g, vp, x, y, nvec, prec, st, true); }, &ws);
+      [&](const double* x, double* y, int nvec) { return hx(g, vp, x, y, nvec, prec, st, true, p->nroots > 1); },
+      &ws);
   if (s != PG_OK && s != PG_NOT_CONVERGED) return s;
   if (evecs_host)
     PG_CUDA_TRY(cudaMemcpyAsync(evecs_host, vec.p, sizeof(double) * N * p->nroots, cudaMemcpyDeviceToHost, st));

@@ -5,7 +5,110 @@
 // (src/mtx.cpp:35-104 applies the same operator line by line with dspmv).
 // Three axis contractions from exact slices on the tensor cores
 // (pg_slice.cu): z with V X, then y and x added to Y.
+//
+// k_hx_fp64 and k_axis_fp64 are the same contractions as chains of FP64
+// multiply-adds in a fixed order, bound by that pipe (371 us against 54 at
+// 64^3 x 4).  They serve the FP64 solver of several roots, whose states come
+// out of a restart with signs that the rounding noise of the products
+// decides: with another product the states are the same to 1e-14, but a third
+// of them change sign, and a solve keeps the states it has always returned.
 #include "pg_slice.cuh"
+
+namespace {
+
+// One thread owns one grid point for up to four vectors (four independent
+// accumulators); operand loads are coalesced or warp-wide broadcasts.
+template <int NV>
+__global__ void __launch_bounds__(256) k_hx_fp64(int nx, int ny, int nz, const double* __restrict__ tx,
+                                                 const double* __restrict__ ty, const double* __restrict__ tz,
+                                                 const double* __restrict__ v, const double* __restrict__ X,
+                                                 double* __restrict__ Y, int nvec) {
+  const long N = (long)nx * ny * nz;
+  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int v0 = blockIdx.y * NV;
+  if (g >= N) return;
+  const int i = (int)(g % nx);
+  const long r = g / nx;
+  const int j = (int)(r % ny);
+  const int k = (int)(r / ny);
+  const int nv = nvec - v0 < NV ? nvec - v0 : NV;
+  const double* Xv = X + (long)v0 * N;
+  double acc[NV];
+  const double vg = v[g];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) acc[q] = q < nv ? vg * Xv[(long)q * N + g] : 0.0;
+  // x sweep: T[b][i] (coalesced over i), x[b,j,k] broadcast
+  {
+    const long base = (long)nx * (j + (long)ny * k);
+    for (int b = 0; b < nx; ++b) {
+      const double t = tx[(long)b * nx + i];
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+        if (q < nv) acc[q] += t * Xv[(long)q * N + base + b];
+    }
+  }
+  // y sweep: Ty[j][b] broadcast, x[i,b,k] coalesced
+  {
+    const long base = i + (long)nx * ny * k;
+    const double* trow = ty + (long)j * ny;
+    for (int b = 0; b < ny; ++b) {
+      const double t = trow[b];
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+        if (q < nv) acc[q] += t * Xv[(long)q * N + base + (long)nx * b];
+    }
+  }
+  // z sweep: Tz[k][b] broadcast, x[i,j,b] coalesced
+  {
+    const long base = i + (long)nx * j;
+    const long sz = (long)nx * ny;
+    const double* trow = tz + (long)k * nz;
+    for (int b = 0; b < nz; ++b) {
+      const double t = trow[b];
+#pragma unroll
+      for (int q = 0; q < NV; ++q)
+        if (q < nv) acc[q] += t * Xv[(long)q * N + base + sz * b];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    if (q < nv) Y[(long)(v0 + q) * N + g] = acc[q];
+}
+
+// Y (mode) A x_axis X: one axis contraction in FP64, mode 0 write, 1 add.
+template <int NV>
+__global__ void __launch_bounds__(256) k_axis_fp64(int nx, int ny, int nz, int axis, const double* __restrict__ A,
+                                                   const double* __restrict__ X, double* __restrict__ Y, int nvec,
+                                                   int mode) {
+  const long N = (long)nx * ny * nz;
+  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int v0 = blockIdx.y * NV;
+  if (g >= N) return;
+  const int i = (int)(g % nx);
+  const long r = g / nx;
+  const int j = (int)(r % ny);
+  const int k = (int)(r / ny);
+  const int na = axis == 0 ? nx : (axis == 1 ? ny : nz);
+  const int idx = axis == 0 ? i : (axis == 1 ? j : k);
+  const long stride = axis == 0 ? 1 : (axis == 1 ? nx : (long)nx * ny);
+  const long base = g - (long)idx * stride;
+  const int nv = nvec - v0 < NV ? nvec - v0 : NV;
+  double acc[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) acc[q] = (q < nv && mode == 1) ? Y[(long)(v0 + q) * N + g] : 0.0;
+  const double* arow = A + (long)idx * na;
+  for (int b = 0; b < na; ++b) {
+    const double t = arow[b];
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+      if (q < nv) acc[q] += t * X[(long)(v0 + q) * N + base + (long)b * stride];
+  }
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    if (q < nv) Y[(long)(v0 + q) * N + g] = acc[q];
+}
+
+}  // namespace
 
 namespace pg {
 
@@ -14,23 +117,34 @@ pg_status tc_axis(const pg_grid* g, int a, const float* Ahi, const float* Alo, c
 
 pg_status axis_apply(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const float* Ahi,
                      const float* Alo, const double* x, double* y, int nvec, int mode, int precision,
-                     cudaStream_t st) {
+                     cudaStream_t st, bool in_order) {
   PG_ARG(g && x && y && x != y && axis >= 0 && axis < 3 && (mode == 0 || mode == 1), "axis_apply: bad arguments");
   if (precision == PG_MIXED) return tc_axis(g, axis, Ahi, Alo, nullptr, x, y, nvec, mode, st);
-  return slice_axis(g, axis, S, A64, nullptr, x, y, nvec, mode, st);
+  if (!in_order) return slice_axis(g, axis, S, A64, nullptr, x, y, nvec, mode, st);
+  constexpr int NV = 4;
+  dim3 grid((unsigned)((g->N + 255) / 256), (unsigned)((nvec + NV - 1) / NV));
+  k_axis_fp64<NV><<<grid, 256, 0, st>>>(g->n[0], g->n[1], g->n[2], axis, A64, x, y, nvec, mode);
+  return check_launch("k_axis_fp64");
 }
 
 pg_status hx_mixed(const pg_grid* g, const double* v, const double* x, double* y, int nvec, cudaStream_t st,
                    bool check, bool unit);
 
 pg_status hx(const pg_grid* g, const double* v, const double* x, double* y, int nvec, int precision,
-             cudaStream_t st, bool unit) {
+             cudaStream_t st, bool unit, bool in_order) {
   PG_ARG(g && v && nvec >= 0, "pg_hx: bad arguments");
   if (nvec == 0) return PG_OK;  // an empty block may come with null X and Y
   PG_ARG(x && y, "pg_hx: null X or Y");
   PG_ARG(x != y, "pg_hx: X and Y must not alias");
   if (precision == PG_MIXED) return hx_mixed(g, v, x, y, nvec, st, false, unit);
   PG_ARG(precision == PG_FP64, "pg_hx: unknown precision %d", precision);
+  if (in_order) {
+    constexpr int NV = 4;
+    dim3 grid((unsigned)((g->N + 255) / 256), (unsigned)((nvec + NV - 1) / NV));
+    k_hx_fp64<NV><<<grid, 256, 0, st>>>(g->n[0], g->n[1], g->n[2], g->t_dev[0].p, g->t_dev[1].p, g->t_dev[2].p, v, x,
+                                       y, nvec);
+    return check_launch("k_hx_fp64");
+  }
   PG_TRY(slice_axis(g, 2, g->t_sl[2], g->t_dev[2].p, v, x, y, nvec, 2, st));
   PG_TRY(slice_axis(g, 1, g->t_sl[1], g->t_dev[1].p, nullptr, x, y, nvec, 1, st));
   return slice_axis(g, 0, g->t_sl[0], g->t_dev[0].p, nullptr, x, y, nvec, 1, st);

@@ -322,7 +322,7 @@ void pg_engine::run_job(Job& job, cudaStream_t st, pg::SolveWorkspace* ws, pg::D
       g, v.p, &p, res.evals, evecs.p, &res.stats, st,
       [&](const double* x, double* y, int nvec) {
         if (batch) return batched_hx(g, v.p, x, y, nvec, st, ready, done_ev);
-        return pg::hx(g, v.p, x, y, nvec, p.precision, st, true);
+        return pg::hx(g, v.p, x, y, nvec, p.precision, st, true, p.nroots > 1);
       },
       ws);
   {

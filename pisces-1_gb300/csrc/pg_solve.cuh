@@ -51,8 +51,8 @@ pg_status kin_f16(const pg_grid* g, double* R, double* w1, double* w2, int k, co
                   cudaStream_t st);
 
 // The kinetic preconditioner R <- (T - sigma_v)^-1 R in the given arithmetic
-// (pg_davidson.cu), scratch w1 and w2 of k vectors each.
+// (pg_davidson.cu), scratch w1 and w2 of k vectors each; in_order as for hx.
 pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double* sigma_dev, double* w1, double* w2,
-                               int precision, cudaStream_t st);
+                               int precision, cudaStream_t st, bool in_order = false);
 
 }  // namespace pg
