@@ -189,6 +189,7 @@ struct SliceMat {
   int n = 0, tau = 0;            // entries are digits of A 2^tau
   int nch = 1, kc = 16;          // K chunks and their width (a multiple of 16)
   int nnc = 1, nc = 16;          // N chunks and their rows (a multiple of 16)
+  bool plain = false;            // entries outside the slices' range: FP64 multiply-adds for every line
   size_t block_bytes() const { return (size_t)7 * nc * kc * 2; }
 };
 

@@ -9,11 +9,11 @@
 // (Potential::SelfConsistentPolarizability, src/Potential.cpp:1495-1628).
 //
 // Over the grid the dipoles are one dense product MU = E A (N x 3npp times
-// 3npp x 3npp).  The work is FP64 (the reference's precision), on this
-// part's FP64 pipe: tiled in shared memory, 64 points x 64 dipole components
-// per CTA, 4 x 4 outputs per thread.  V_pol is that product's epilogue: each
-// CTA forms the row dots E . MU of its tile, and a second pass sums the
-// column tiles of a point in a fixed order (no atomics; bit-stable).
+// 3npp x 3npp), in FP64 precision on the tensor cores from exact slices
+// (pg_slice.cu; 8 waters on 48^3: 1.89 ms as FP64 multiply-adds, 0.15 ms so).
+// V_pol is that product's read-out: each CTA forms the row dots E . MU of its
+// points, and a second pass sums the few partial dots of a point in a fixed
+// order (no atomics; bit-stable).
 //
 // The gradient (DVR::ComputeGradient, src/DVR.cpp:1099-1176, with
 // Potential::EvaluateDPPGTOPGradient / DerivElecField / MuCrossMu /
@@ -31,15 +31,17 @@
 #include <cstring>
 #include <vector>
 
+#include "pg_slice.cuh"
 #include "pg_solve.cuh"
 
 namespace {
 
-constexpr int kBM = 64;   // points per product tile
+constexpr int kBM = 64;   // rows of a product tile
 constexpr int kBN = 64;   // dipole components per product tile
 constexpr int kBK = 16;   // reduction depth per shared-memory stage
 constexpr int kGT = 256;  // threads per product CTA (16 x 16, 4 x 4 outputs each)
-constexpr size_t kChunkBytes = size_t(1) << 30;  // E (and MU) per chunk of points
+constexpr size_t kChunkBytes = size_t(1) << 30;  // E (and MU) per chunk of points of the gradient
+constexpr size_t kFieldBytes = size_t(64) << 20;  // E per chunk of points of the potential
 
 // ------------------------------------------------------------------ host side
 
@@ -107,6 +109,8 @@ pg_status check_model(const char* who, const pg_sites* t, const pg_scpol_model* 
 // Device copies of a model: positions of the polarisable sites, Epc and A.
 struct ModelDev {
   pg::DevBuf<double> pos, epc, inva;
+  pg::DevBuf<unsigned char> img;
+  pg::SliceMat mat;  // digit images of A
   pg_status upload(const pg_sites* t, const pg_scpol_model* m, cudaStream_t st) {
     const int n = 3 * m->npp;
     std::vector<double> p(n);
@@ -118,6 +122,15 @@ struct ModelDev {
     PG_CUDA_TRY(cudaMemcpyAsync(pos.p, p.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
     PG_CUDA_TRY(cudaMemcpyAsync(epc.p, m->epc, sizeof(double) * n, cudaMemcpyHostToDevice, st));
     PG_CUDA_TRY(cudaMemcpyAsync(inva.p, m->inva, sizeof(double) * n * n, cudaMemcpyHostToDevice, st));
+    double big = 0;
+    bool finite = true;
+    for (size_t e = 0; e < (size_t)n * n; ++e) {
+      finite &= std::isfinite(m->inva[e]);
+      big = std::max(big, fabs(m->inva[e]));
+    }
+    if (!finite) big = INFINITY;
+    PG_TRY(img.alloc(pg::slice_rows_shape(n, big, &mat)));
+    PG_TRY(pg::slice_rows_matrix(inva.p, img.p, &mat, st));
     // the host arrays may be released as soon as the call returns
     PG_CUDA_TRY(cudaStreamSynchronize(st));
     return PG_OK;
@@ -165,79 +178,6 @@ __global__ void k_scpol_field(long p0, long np, const int* __restrict__ list, in
     e[0] = g * rx + epc[3 * i];
     e[1] = g * ry + epc[3 * i + 1];
     e[2] = g * rz + epc[3 * i + 2];
-  }
-}
-
-// Y = E A for np points (E: np x n, A: n x n, both row-major).  kStore:
-// Y -> out[p*n + c]; otherwise out[ct*np + p] = sum over the 64 columns c of
-// column tile ct of E[p][c] Y[p][c] (fixed shuffle order).
-template <bool kStore>
-__global__ void __launch_bounds__(kGT) k_scpol_gemm(long np, int n, const double* __restrict__ E,
-                                                    const double* __restrict__ A, double* __restrict__ out) {
-  __shared__ double Es[kBK][kBM + 1];
-  __shared__ double As[kBK][kBN];
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  const long pb = (long)blockIdx.x * kBM;
-  const int cb = blockIdx.y * kBN;
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  for (int k0 = 0; k0 < n; k0 += kBK) {
-#pragma unroll
-    for (int e = t; e < kBM * kBK; e += kGT) {
-      const int pp = e / kBK, kk = e - pp * kBK;
-      const long p = pb + pp;
-      const int k = k0 + kk;
-      Es[kk][pp] = (p < np && k < n) ? E[p * n + k] : 0.0;
-    }
-#pragma unroll
-    for (int e = t; e < kBK * kBN; e += kGT) {
-      const int kk = e / kBN, cc = e - kk * kBN;
-      const int k = k0 + kk, c = cb + cc;
-      As[kk][cc] = (k < n && c < n) ? A[(long)k * n + c] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = Es[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = As[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  if (kStore) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long p = pb + ty + 16 * i;
-      if (p >= np) continue;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = cb + tx + 16 * j;
-        if (c < n) out[p * n + c] = acc[i][j];
-      }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long p = pb + ty + 16 * i;
-      double s = 0.0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = cb + tx + 16 * j;
-        if (p < np && c < n) s += E[p * n + c] * acc[i][j];
-      }
-#pragma unroll
-      for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-      if (tx == 0 && p < np) out[(long)blockIdx.y * np + p] = s;
-    }
   }
 }
 
@@ -488,24 +428,23 @@ pg_status scpol_add_points(const pg_grid* g, const pg_sites* t, const pg_scpol_m
   ModelDev md;
   PG_TRY(md.upload(t, m, st));
   const int n = 3 * m->npp;
-  const long chunk = chunk_points(count, n);
-  const int nct = (n + kBN - 1) / kBN;
+  // E of a chunk is read back while it is still in L2
+  const long chunk = std::min<long>(count, std::max<long>(152L * 128, (long)(kFieldBytes / (sizeof(double) * n)) / 128 * 128));
   pg::DevBuf<double> E, part;
   PG_TRY(E.alloc((size_t)chunk * n));
-  PG_TRY(part.alloc((size_t)chunk * nct));
+  PG_TRY(part.alloc((size_t)chunk * pg::slice_row_count(n)));
   for (long p0 = 0; p0 < count; p0 += chunk) {
     const long np = chunk < count - p0 ? chunk : count - p0;
     k_scpol_field<<<stride_blocks(np * m->npp), 256, 0, st>>>(p0, np, list, g->n[0], g->n[1], g->x_dev[0].p,
                                                              g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos.p, md.epc.p,
                                                              m->damp_type, m->damp, E.p);
     PG_TRY(pg::check_launch("k_scpol_field"));
-    k_scpol_gemm<false><<<dim3((unsigned)((np + kBM - 1) / kBM), nct), kGT, 0, st>>>(np, n, E.p, md.inva.p, part.p);
-    PG_TRY(pg::check_launch("k_scpol_gemm"));
-    k_scpol_finish<<<stride_blocks(np), 256, 0, st>>>(p0, np, list, nct, part.p, m->vpol_ww, v, vpol);
+    int rows = 0;
+    PG_TRY(slice_rows(np, md.mat, md.inva.p, E.p, part.p, kRowDot, &rows, g->tc_err.p, st));
+    k_scpol_finish<<<stride_blocks(np), 256, 0, st>>>(p0, np, list, rows, part.p, m->vpol_ww, v, vpol);
     PG_TRY(pg::check_launch("k_scpol_finish"));
   }
-  PG_CUDA_TRY(cudaStreamSynchronize(st));
-  return PG_OK;
+  return check_tc_error(g, st);  // waits for the stream
 }
 
 }  // namespace pg
@@ -585,15 +524,13 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
   PG_CUDA_TRY(cudaMemcpyAsync(dtiles.p, tl.data(), sizeof(int2) * ntiles, cudaMemcpyHostToDevice, st));
   PG_CUDA_TRY(cudaMemsetAsync(tot.p, 0, sizeof(double) * m1, st));
   PG_CUDA_TRY(cudaMemsetAsync(C.p, 0, sizeof(double) * n * n, st));
-  const int nct = (n + kBN - 1) / kBN;
   for (long p0 = 0; p0 < N; p0 += chunk) {
     const long np = chunk < N - p0 ? chunk : N - p0;
     k_scpol_field<<<stride_blocks(np * m->npp), 256, 0, st>>>(p0, np, nullptr, g->n[0], g->n[1], g->x_dev[0].p,
                                                              g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos.p, md.epc.p,
                                                              2, m->damp, E.p);
     PG_TRY(pg::check_launch("k_scpol_field"));
-    k_scpol_gemm<true><<<dim3((unsigned)((np + kBM - 1) / kBM), nct), kGT, 0, st>>>(np, n, E.p, md.inva.p, MU.p);
-    PG_TRY(pg::check_launch("k_scpol_gemm"));
+    PG_TRY(pg::slice_rows(np, md.mat, md.inva.p, E.p, MU.p, pg::kRowStore, nullptr, g->tc_err.p, st));
     const int sb = (int)((np + site_per - 1) / site_per);
     k_grad_sites<<<sb, 256, 0, st>>>(p0, np, site_per, g->n[0], g->n[1], g->x_dev[0].p, g->x_dev[1].p,
                                      g->x_dev[2].p, psi, MU.p, n, ns, srec.p, t->charge_damp, m->damp, spart.p);
@@ -609,7 +546,7 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
   std::vector<double> h(m1);
   PG_CUDA_TRY(cudaMemcpyAsync(h.data(), tot.p, sizeof(double) * m1, cudaMemcpyDeviceToHost, st));
   PG_CUDA_TRY(cudaMemcpyAsync(mcm, C.p, sizeof(double) * n * n, cudaMemcpyDeviceToHost, st));
-  PG_CUDA_TRY(cudaStreamSynchronize(st));
+  PG_TRY(pg::check_tc_error(g, st));  // waits for the stream
   std::memcpy(grad, h.data(), sizeof(double) * 3 * ns);
   std::memcpy(tmu, h.data() + 3 * ns, sizeof(double) * n);
   return PG_OK;

@@ -35,6 +35,7 @@ struct SliceArgs {
   long npts;     // points of one vector (index of V)
   int n, kc, nnc, nc;
   int h0, nch;   // K chunks [h0, h0 + nch) of this launch
+  int plain;     // every line by FP64 multiply-adds
   int rebuild;   // more than one K chunk per axis: the digit images are rebuilt for every N chunk
   int nc_per;    // N chunks per CTA (blockIdx.y takes the next ones)
   int scale;     // exponent of accumulator 6: kSliceUnit - tau - 1075 - kSliceGuard
@@ -42,7 +43,9 @@ struct SliceArgs {
   uint32_t slice_b;      // bytes of one slice in it
   uint32_t off_b, off_t; // shared-memory offsets of the matrix block and the transpose buffer
   uint32_t tmem_cols;
-  int mode;
+  int mode;              // 0: y = K, 1: y += K, 2: y = v x + K, 3: row dots x . K
+  long out0;             // mode 3: first output row of this launch, in values
+  long sa, sb;           // strides of A64 (output, input index)
 };
 
 template <int NU>
@@ -180,10 +183,11 @@ __global__ void __launch_bounds__(kST, 1)
     }
     return o;
   };
+  double dot = 0.0;     // mode 3
   double pa[4], pb[4];  // what the next batch is added to: y, or x and v
   auto prefetch = [&](const Out& o) {
     const double* s = A.mode == 1 ? y : x;
-    if (A.mode != 0) {
+    if (A.mode == 1 || A.mode == 2) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) pa[q] = q < o.cnt ? s[o.p + q * ostep] : 0.0;
     }
@@ -200,7 +204,7 @@ __global__ void __launch_bounds__(kST, 1)
   bool slow = false;
   auto settle = [&] {  // after the line maxima are complete
     emax = s_emax[line];
-    slow = emax != 0 && (emax < kExpLo || emax > kExpHi);
+    slow = A.plain || (emax != 0 && (emax < kExpLo || emax > kExpHi));
     if (slow) emax = 0;
   };
   if (A.nch > 1) {
@@ -318,9 +322,17 @@ __global__ void __launch_bounds__(kST, 1)
           const int i = c * A.nc + 4 * bt + q;
           double s = 0.0;
 #pragma unroll 1
-          for (int b = A.h0 * A.kc; i < A.n && b < k_end; ++b) s = fma(A64[(long)i * A.n + b], x[base + b * A.inner], s);
+          for (int b = A.h0 * A.kc; i < A.n && b < k_end; ++b) s = fma(A64[i * A.sa + b * A.sb], x[base + b * A.inner], s);
           k[q] = s;
         }
+      }
+      if (A.mode == 3) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = c * A.nc + 4 * bt + q;
+          if (valid && i < A.n) dot = fma(x[base + i], k[q], dot);
+        }
+        continue;
       }
       if (contig) {
         // 32 lines x 4 columns through the warp's buffer, so that four lanes
@@ -346,6 +358,16 @@ __global__ void __launch_bounds__(kST, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
+  if (A.mode == 3) {
+    // the four threads of a line, in order
+    double* sd = reinterpret_cast<double*>(smem + A.off_t);
+    __syncthreads();
+    sd[part * kLines + line] = dot;
+    __syncthreads();
+    if (part == 0 && valid)
+      y[A.out0 + (long)blockIdx.y * A.nlines + l0 + line] =
+          ((dot + sd[kLines + line]) + sd[2 * kLines + line]) + sd[3 * kLines + line];
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
@@ -361,13 +383,14 @@ struct SliceBuild {
   unsigned char* img[9];
   int emax[9];  // biased exponent of the matrix's largest value
   int n[9], kc[9], nc[9], nnc[9];
+  int trans;    // the images are those of A^T
 };
 __global__ void k_slice_matrix(const SliceBuild B) {
   const int m = blockIdx.y, n = B.n[m], kc = B.kc[m], nc = B.nc[m];
   const size_t block = (size_t)pg::kSliceN * nc * kc * 2;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
     const int i = e / n, k = e - i * n;
-    const unsigned long long f = pg::slice_fixed(B.A[m][e], B.emax[m]);
+    const unsigned long long f = pg::slice_fixed(B.A[m][B.trans ? k * n + i : e], B.emax[m]);
     const int c = i / nc, h = k / kc;
     unsigned char* p = B.img[m] + (size_t)(h * B.nnc[m] + c) * block + pg::tc16_kmajor_off(i - c * nc, k - h * kc, kc);
 #pragma unroll
@@ -451,18 +474,24 @@ pg_status slice_grid(pg_grid* g) {
   return PG_OK;
 }
 
-pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const double* v,
-                     const double* x, double* y, int nvec, int mode, cudaStream_t st) {
-  PG_ARG(S.img && S.n == g->n[axis], "slice_axis: no operand images");
+namespace {
+
+// Launches the contraction of nlines lines (stride inner); mode 3 writes
+// *rows rows of nlines partial dots.
+pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, const double* A64, bool trans,
+                       const double* v, const double* x, double* y, int mode, int* rows, int* err, cudaStream_t st) {
   SliceArgs a{};
   a.n = S.n;
-  a.inner = axis == 0 ? 1 : (axis == 1 ? g->n[0] : (long)g->n[0] * g->n[1]);
-  a.npts = g->N;
-  a.nlines = g->N / S.n * nvec;
-  a.kc = S.kc;
+  a.inner = inner;
+  a.npts = npts;
+  a.nlines = nlines;
+  a.plain = S.plain;
   a.rebuild = S.nch > 1;
+  a.kc = S.kc;
   a.nnc = S.nnc;
   a.nc = S.nc;
+  a.sa = trans ? 1 : S.n;
+  a.sb = trans ? S.n : 1;
   a.scale = kSliceUnit - kSliceGuard - S.tau - 1075;
   a.block_bytes = (uint32_t)S.block_bytes();
   a.slice_b = (uint32_t)(S.nc * S.kc * 2);
@@ -481,18 +510,66 @@ pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double
   const dim3 grid((unsigned)tiles, (unsigned)split);
   // at most two K chunks (160 values) per launch, so that the sums of one
   // accumulator stay below 2^24; a longer axis adds up in Y
-  for (int h0 = 0; h0 < S.nch; h0 += 2) {
+  int launches = 0;
+  for (int h0 = 0; h0 < S.nch; h0 += 2, ++launches) {
     a.h0 = h0;
     a.nch = std::min(2, S.nch - h0);
-    a.mode = h0 == 0 ? mode : 1;
+    a.mode = h0 == 0 || mode == 3 ? mode : 1;
+    a.out0 = (long)launches * split * nlines;
     cudaError_t e;
-    if (S.kc <= 32) e = launch_slice<1>(a, grid, smem, S.img, A64, v, x, y, g->tc_err.p, st);
-    else if (S.kc <= 64) e = launch_slice<2>(a, grid, smem, S.img, A64, v, x, y, g->tc_err.p, st);
-    else e = launch_slice<3>(a, grid, smem, S.img, A64, v, x, y, g->tc_err.p, st);
+    if (S.kc <= 32) e = launch_slice<1>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    else if (S.kc <= 64) e = launch_slice<2>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    else e = launch_slice<3>(a, grid, smem, S.img, A64, v, x, y, err, st);
     PG_CUDA_TRY(e);
     PG_TRY(check_launch("k_slice_axis"));
   }
+  if (rows) *rows = launches * split;
   return PG_OK;
+}
+
+}  // namespace
+
+pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const double* v,
+                     const double* x, double* y, int nvec, int mode, cudaStream_t st) {
+  PG_ARG(S.img && S.n == g->n[axis], "slice_axis: no operand images");
+  const long inner = axis == 0 ? 1 : (axis == 1 ? g->n[0] : (long)g->n[0] * g->n[1]);
+  return slice_launch(g->N / S.n * nvec, inner, g->N, S, A64, false, v, x, y, mode, nullptr, g->tc_err.p, st);
+}
+
+int slice_row_count(int n) {
+  SliceMat S;
+  slice_shape(n, &S);
+  return (S.nch + 1) / 2 * S.nnc;
+}
+
+size_t slice_rows_shape(int n, double big, SliceMat* S) {
+  slice_shape(n, S);
+  S->plain = !std::isfinite(big) || big > 1e200 || (big != 0 && big < 1e-200);
+  int ex = 0;
+  if (!S->plain) frexp(big, &ex);
+  S->tau = kSliceN * kSliceP - 1 - ex;
+  return (size_t)S->nch * S->nnc * S->block_bytes();
+}
+
+pg_status slice_rows_matrix(const double* A64, unsigned char* img, SliceMat* S, cudaStream_t st) {
+  PG_CUDA_TRY(cudaMemsetAsync(img, 0, (size_t)S->nch * S->nnc * S->block_bytes(), st));
+  SliceBuild B{};
+  B.A[0] = A64;
+  B.img[0] = img;
+  B.emax[0] = kSliceN * kSliceP - 1 - S->tau + 1022;
+  B.n[0] = S->n;
+  B.kc[0] = S->kc;
+  B.nc[0] = S->nc;
+  B.nnc[0] = S->nnc;
+  B.trans = 1;
+  S->img = img;
+  k_slice_matrix<<<dim3((unsigned)std::min(4096, (S->n * S->n + 255) / 256), 1), 256, 0, st>>>(B);
+  return check_launch("k_slice_matrix");
+}
+
+pg_status slice_rows(long nlines, const SliceMat& S, const double* A64, const double* x, double* y, SliceRows mode,
+                     int* rows, int* err, cudaStream_t st) {
+  return slice_launch(nlines, 1, nlines * S.n, S, A64, true, nullptr, x, y, mode, rows, err, st);
 }
 
 }  // namespace pg

@@ -123,4 +123,16 @@ pg_status slice_grid(pg_grid* g);
 pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const double* v,
                      const double* x, double* y, int nvec, int mode, cudaStream_t st);
 
+// Rows times a matrix: X is nlines x n (row-major), A n x n.
+// kRowStore: Y = X A.  kRowDot: Y holds *rows rows of nlines values whose sum
+// over the rows is x . (x A) for each line (at most slice_row_count(n)).
+// A64 and the images (slice_rows_matrix) on the device; err as tc_err.
+enum SliceRows { kRowStore = 0, kRowDot = 3 };
+int slice_row_count(int n);
+// shape and bytes of the images of an n x n matrix whose largest entry is big
+size_t slice_rows_shape(int n, double big, SliceMat* S);
+pg_status slice_rows_matrix(const double* A64, unsigned char* img, SliceMat* S, cudaStream_t st);
+pg_status slice_rows(long nlines, const SliceMat& S, const double* A64, const double* x, double* y, SliceRows mode,
+                     int* rows, int* err, cudaStream_t st);
+
 }  // namespace pg
