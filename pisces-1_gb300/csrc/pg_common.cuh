@@ -153,6 +153,21 @@ struct HostPinned {
   }
 };
 
+// A status word that kernels set and the host reads after a stream
+// synchronisation: page-locked host memory mapped into the device's address
+// space, so reading it takes no copy (a 4-byte device-to-host copy and its
+// wait cost about 15 us a call).  The words of all grids come from one small
+// block of the process.
+struct StatusWord {
+  int* p = nullptr;           // device address
+  volatile int* h = nullptr;  // host address
+  StatusWord() = default;
+  StatusWord(const StatusWord&) = delete;
+  StatusWord& operator=(const StatusWord&) = delete;
+  ~StatusWord();
+  pg_status alloc();
+};
+
 // Byte offset of element (r, k) of a tensor-core operand tile in shared
 // memory: no-swizzle K-major core matrices of 8 rows x 16 bytes (4 FP32/TF32
 // values), K-adjacent core matrices 128 bytes apart, 8-row groups kpad/4 *
@@ -195,6 +210,10 @@ struct SliceMat {
 
 }  // namespace pg
 
+namespace pg {
+struct SolveWorkspace;
+}
+
 // The grid handle: sizes, host copies of the 1-D data and device kinetic matrices.
 struct pg_grid {
   int dvrtype = 2;                 // 2: sine DVR; 3: periodic FFT kinetic (as dense circulant matrices)
@@ -221,7 +240,8 @@ struct pg_grid {
   pg::DevBuf<unsigned short> t16_lo[3];
   int t16_scale = 0;
   pg::DevBuf<double> x_dev[3];     // grid points on the device
-  pg::DevBuf<int> tc_err;          // set by the tensor-core H*X kernels if a completion wait times out
+  pg::StatusWord tc_err;           // set by the tensor-core kernels if a completion wait times out
+  bool same_t = false;             // the three axes share one kinetic matrix
   // eigenbasis of the kinetic matrices (the orthonormal DST-I, symmetric),
   // for the kinetic preconditioner: FP64, TF32 hi/lo, and the eigenvalues
   pg::DevBuf<double> q_dev[3];
@@ -259,9 +279,50 @@ struct pg_grid {
     alignas(64) unsigned char z[128];
   };
   mutable std::map<std::pair<const void*, int>, TensorMapPair> tmaps;
+  // device scratch of calls that wait for their stream before they return,
+  // and the buffers of pg_solve, kept between calls (pg_keep.cu); freed with
+  // the grid
+  mutable std::mutex scratch_m, solve_m;
+  mutable pg::DevBuf<unsigned char> scratch;
+  mutable std::shared_ptr<pg::SolveWorkspace> solve_ws;
+  mutable size_t solve_kept = 0;
+  ~pg_grid();
 };
 
 namespace pg {
+// Scratch of one call on stream st: the grid's kept buffer where no other
+// thread holds it and the size is within bounds, else an allocation of its
+// own.  The destructor waits for the stream, so that the next holder (on any
+// stream) finds the buffer idle.
+class ScratchLease {
+ public:
+  ScratchLease(const pg_grid* g, cudaStream_t st) : g_(g), st_(st) {}
+  ~ScratchLease();
+  pg_status get(size_t bytes, unsigned char** p);
+
+ private:
+  const pg_grid* g_;
+  cudaStream_t st_;
+  std::unique_lock<std::mutex> lock_;
+  DevBuf<unsigned char> own_;
+};
+
+// The grid's kept solve buffers for one pg_solve on stream st (a workspace of
+// its own where another thread is using them); on release they stay with the
+// grid if they are within bounds.
+class SolveLease {
+ public:
+  SolveLease(const pg_grid* g, cudaStream_t st);
+  ~SolveLease();
+  SolveWorkspace* ws() { return ws_.get(); }
+
+ private:
+  const pg_grid* g_;
+  cudaStream_t st_;
+  std::unique_lock<std::mutex> lock_;
+  std::shared_ptr<SolveWorkspace> ws_;
+};
+
 // Launch parameters of the mixed-form H*X for one grid shape and block size:
 // from the tuned table (pg_hx_tuned.inc, written by tune_hx.py), else the
 // built-in rules, then the grid's overrides.

@@ -257,12 +257,16 @@ extern "C" pg_status pg_kinetic_precondition(const pg_grid* g, double* R, int k,
   if (k == 0) return PG_OK;
   PG_ARG(R && sigma, "pg_kinetic_precondition: null R or sigma");
   cudaStream_t st = pg::as_stream(stream);
-  pg::DevBuf<double> w, sg;
-  PG_TRY(w.alloc((size_t)2 * k * g->N));
-  PG_TRY(sg.alloc((size_t)k));
-  PG_CUDA_TRY(cudaMemcpyAsync(sg.p, sigma, sizeof(double) * k, cudaMemcpyHostToDevice, st));
-  PG_TRY(pg::kinetic_precondition(g, R, k, sg.p, w.p, w.p + (long)k * g->N, precision, st));
-  // waits for the stream: the scratch is freed on return
+  // W1, W2 (each a multiple of 256 bytes) and sigma
+  const size_t wb = (sizeof(double) * k * (size_t)g->N + 255) / 256 * 256;
+  pg::ScratchLease scratch(g, st);
+  unsigned char* w = nullptr;
+  PG_TRY(scratch.get(2 * wb + sizeof(double) * k, &w));
+  double* sg = reinterpret_cast<double*>(w + 2 * wb);
+  PG_CUDA_TRY(cudaMemcpyAsync(sg, sigma, sizeof(double) * k, cudaMemcpyHostToDevice, st));
+  PG_TRY(pg::kinetic_precondition(g, R, k, sg, reinterpret_cast<double*>(w), reinterpret_cast<double*>(w + wb),
+                                  precision, st));
+  // waits for the stream: the scratch is the next call's
   return pg::check_tc_error(g, st);
 }
 
@@ -1159,12 +1163,14 @@ extern "C" pg_status pg_solve(const pg_grid* g, const double* v, const pg_solve_
                               double* evecs, pg_solve_stats* stats, void* stream) {
   using namespace pg;
   cudaStream_t st = as_stream(stream);
-  const int prec = p ? p->precision : PG_FP64;
-  const bool in_order = p && p->nroots > 1;
+  PG_ARG(g && v && p, "pg_solve: null argument");
+  const int prec = p->precision;
+  const bool in_order = p->nroots > 1;
+  SolveLease lease(g, st);
   return solve_with(
       g, v, p, evals, evecs, stats, st,
       [&](const double* x, double* y, int nvec) { return hx(g, v, x, y, nvec, prec, st, true, in_order); },
-      nullptr);
+      lease.ws());
 }
 
 namespace pg {

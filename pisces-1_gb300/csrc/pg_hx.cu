@@ -168,6 +168,6 @@ extern "C" pg_status pg_grid_check(const pg_grid* g, void* stream) {
   PG_ARG(g, "pg_grid_check: null grid");
   cudaStream_t st = pg::as_stream(stream);
   const pg_status s = pg::check_tc_error(g, st);
-  if (s == PG_DEVICE_TIMEOUT) PG_CUDA_TRY(cudaMemsetAsync(g->tc_err.p, 0, sizeof(int), st));
+  if (s == PG_DEVICE_TIMEOUT) *g->tc_err.h = 0;
   return s;
 }

@@ -573,8 +573,7 @@ F16Plan plan_f16(const pg_grid* g) {
   if (!g->t16_hi[0].p) return no("no FP16 kinetic images (an axis has more than 128 points)");
   if (nx > 96 || ny > 96 || nz > 96) return no("an axis has more than 96 points");
   if (nx % 2 != 0) return no("odd nx (bulk copies need 16-byte rows)");
-  for (int a = 1; a < 3; ++a)
-    if (g->n[a] != nx || g->t[a] != g->t[0]) return no("the axes do not share one kinetic matrix");
+  if (!g->same_t) return no("the axes do not share one kinetic matrix");
   F16Geom& G = P.G;
   G.nx = nx;
   G.ny = ny;

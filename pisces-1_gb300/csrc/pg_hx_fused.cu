@@ -784,7 +784,7 @@ cudaError_t fused_init() {
 }
 
 bool same_matrix(const pg_grid* g, int a, int b) {
-  return g->n[a] == g->n[b] && g->t[a] == g->t[b];
+  return g->same_t || (g->n[a] == g->n[b] && g->t[a] == g->t[b]);
 }
 
 FusedPlan plan_fused(const pg_grid* g) {

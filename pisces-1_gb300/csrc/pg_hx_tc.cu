@@ -800,10 +800,8 @@ pg_status hx_mixed(const pg_grid* g, const double* v, const double* x, double* y
 }
 
 pg_status check_tc_error(const pg_grid* g, cudaStream_t st) {
-  int herr = 0;
-  PG_CUDA_TRY(cudaMemcpyAsync(&herr, g->tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   PG_CUDA_TRY(cudaStreamSynchronize(st));
-  if (herr) {
+  if (*g->tc_err.h) {
     set_error("pg_hx: tensor-core completion wait timed out");
     return PG_DEVICE_TIMEOUT;
   }

@@ -106,33 +106,40 @@ pg_status check_model(const char* who, const pg_sites* t, const pg_scpol_model* 
   return PG_OK;
 }
 
-// Device copies of a model: positions of the polarisable sites, Epc and A.
+// Device copies of a model in a buffer of bytes(m) bytes: positions of the
+// polarisable sites, Epc, A and A's digit images.
 struct ModelDev {
-  pg::DevBuf<double> pos, epc, inva;
-  pg::DevBuf<unsigned char> img;
-  pg::SliceMat mat;  // digit images of A
-  pg_status upload(const pg_sites* t, const pg_scpol_model* m, cudaStream_t st) {
+  const double *pos = nullptr, *epc = nullptr, *inva = nullptr;
+  pg::SliceMat mat;
+  size_t img_bytes = 0;
+  static size_t up(size_t b) { return (b + 255) / 256 * 256; }
+  size_t bytes(const pg_scpol_model* m) {
     const int n = 3 * m->npp;
-    std::vector<double> p(n);
-    for (int i = 0; i < m->npp; ++i)
-      for (int c = 0; c < 3; ++c) p[3 * i + c] = t->sites[3 * m->pol_site[i] + c];
-    PG_TRY(pos.alloc(n));
-    PG_TRY(epc.alloc(n));
-    PG_TRY(inva.alloc((size_t)n * n));
-    PG_CUDA_TRY(cudaMemcpyAsync(pos.p, p.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
-    PG_CUDA_TRY(cudaMemcpyAsync(epc.p, m->epc, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-    PG_CUDA_TRY(cudaMemcpyAsync(inva.p, m->inva, sizeof(double) * n * n, cudaMemcpyHostToDevice, st));
     double big = 0;
     bool finite = true;
     for (size_t e = 0; e < (size_t)n * n; ++e) {
       finite &= std::isfinite(m->inva[e]);
       big = std::max(big, fabs(m->inva[e]));
     }
-    if (!finite) big = INFINITY;
-    PG_TRY(img.alloc(pg::slice_rows_shape(n, big, &mat)));
-    PG_TRY(pg::slice_rows_matrix(inva.p, img.p, &mat, st));
-    // the host arrays may be released as soon as the call returns
-    PG_CUDA_TRY(cudaStreamSynchronize(st));
+    img_bytes = pg::slice_rows_shape(n, finite ? big : INFINITY, &mat);
+    return up(img_bytes) + 2 * up(sizeof(double) * n) + up(sizeof(double) * n * n);
+  }
+  // the host arrays may be released once the call has waited for the stream
+  pg_status upload(const pg_sites* t, const pg_scpol_model* m, unsigned char* buf, cudaStream_t st) {
+    const int n = 3 * m->npp;
+    std::vector<double> p(n);
+    for (int i = 0; i < m->npp; ++i)
+      for (int c = 0; c < 3; ++c) p[3 * i + c] = t->sites[3 * m->pol_site[i] + c];
+    double* d = reinterpret_cast<double*>(buf + up(img_bytes));
+    pos = d;
+    PG_CUDA_TRY(cudaMemcpyAsync(d, p.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    d += up(sizeof(double) * n) / sizeof(double);
+    epc = d;
+    PG_CUDA_TRY(cudaMemcpyAsync(d, m->epc, sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    d += up(sizeof(double) * n) / sizeof(double);
+    inva = d;
+    PG_CUDA_TRY(cudaMemcpyAsync(d, m->inva, sizeof(double) * n * n, cudaMemcpyHostToDevice, st));
+    PG_TRY(pg::slice_rows_matrix(inva, buf, &mat, st));
     return PG_OK;
   }
 };
@@ -426,22 +433,25 @@ pg_status scpol_add_points(const pg_grid* g, const pg_sites* t, const pg_scpol_m
   PG_TRY(check_model("pg_potential_scpol_add", t, m));
   if (count == 0) return PG_OK;
   ModelDev md;
-  PG_TRY(md.upload(t, m, st));
   const int n = 3 * m->npp;
   // E of a chunk is read back while it is still in L2
   const long chunk = std::min<long>(count, std::max<long>(152L * 128, (long)(kFieldBytes / (sizeof(double) * n)) / 128 * 128));
-  pg::DevBuf<double> E, part;
-  PG_TRY(E.alloc((size_t)chunk * n));
-  PG_TRY(part.alloc((size_t)chunk * pg::slice_row_count(n)));
+  const size_t mb = md.bytes(m), eb = ModelDev::up(sizeof(double) * chunk * n);
+  ScratchLease scratch(g, st);
+  unsigned char* buf = nullptr;
+  PG_TRY(scratch.get(mb + eb + sizeof(double) * chunk * slice_row_count(n), &buf));
+  PG_TRY(md.upload(t, m, buf, st));
+  double* E = reinterpret_cast<double*>(buf + mb);
+  double* part = reinterpret_cast<double*>(buf + mb + eb);
   for (long p0 = 0; p0 < count; p0 += chunk) {
     const long np = chunk < count - p0 ? chunk : count - p0;
     k_scpol_field<<<stride_blocks(np * m->npp), 256, 0, st>>>(p0, np, list, g->n[0], g->n[1], g->x_dev[0].p,
-                                                             g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos.p, md.epc.p,
-                                                             m->damp_type, m->damp, E.p);
+                                                             g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos, md.epc,
+                                                             m->damp_type, m->damp, E);
     PG_TRY(pg::check_launch("k_scpol_field"));
     int rows = 0;
-    PG_TRY(slice_rows(np, md.mat, md.inva.p, E.p, part.p, kRowDot, &rows, g->tc_err.p, st));
-    k_scpol_finish<<<stride_blocks(np), 256, 0, st>>>(p0, np, list, rows, part.p, m->vpol_ww, v, vpol);
+    PG_TRY(slice_rows(np, md.mat, md.inva, E, part, kRowDot, &rows, g->tc_err.p, st));
+    k_scpol_finish<<<stride_blocks(np), 256, 0, st>>>(p0, np, list, rows, part, m->vpol_ww, v, vpol);
     PG_TRY(pg::check_launch("k_scpol_finish"));
   }
   return check_tc_error(g, st);  // waits for the stream
@@ -463,7 +473,9 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
          "pg_hf_gradient_grid: the reference gradient damps the polarisable sites by the effective radius only");
   cudaStream_t st = pg::as_stream(stream);
   ModelDev md;
-  PG_TRY(md.upload(t, m, st));
+  pg::DevBuf<unsigned char> mbuf;
+  PG_TRY(mbuf.alloc(md.bytes(m)));
+  PG_TRY(md.upload(t, m, mbuf.p, st));
   const int ns = t->nsites, n = 3 * m->npp;
   // site records: charges, Slater terms, polarisable index
   std::vector<SiteRec> rec(ns);
@@ -527,10 +539,10 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
   for (long p0 = 0; p0 < N; p0 += chunk) {
     const long np = chunk < N - p0 ? chunk : N - p0;
     k_scpol_field<<<stride_blocks(np * m->npp), 256, 0, st>>>(p0, np, nullptr, g->n[0], g->n[1], g->x_dev[0].p,
-                                                             g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos.p, md.epc.p,
+                                                             g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos, md.epc,
                                                              2, m->damp, E.p);
     PG_TRY(pg::check_launch("k_scpol_field"));
-    PG_TRY(pg::slice_rows(np, md.mat, md.inva.p, E.p, MU.p, pg::kRowStore, nullptr, g->tc_err.p, st));
+    PG_TRY(pg::slice_rows(np, md.mat, md.inva, E.p, MU.p, pg::kRowStore, nullptr, g->tc_err.p, st));
     const int sb = (int)((np + site_per - 1) / site_per);
     k_grad_sites<<<sb, 256, 0, st>>>(p0, np, site_per, g->n[0], g->n[1], g->x_dev[0].p, g->x_dev[1].p,
                                      g->x_dev[2].p, psi, MU.p, n, ns, srec.p, t->charge_damp, m->damp, spart.p);
