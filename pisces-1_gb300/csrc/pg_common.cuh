@@ -186,11 +186,15 @@ inline __host__ __device__ int tc_npad(int n) { return (n + 15) / 16 * 16; }
 inline __host__ __device__ int tc_kpad(int n) { return (n + 7) / 8 * 8; }
 // K chunk of the tensor-core contraction: the B chunk (npad x kc) and the A
 // tile (128 x kc), both as TF32 hi/lo, must fit 220 KB of shared memory;
-// n <= 112 gives one chunk (kc = kpad).  The operand images are stored as
-// ceil(kpad / kc) consecutive chunk images of npad x kc.
+// n <= 112 gives one chunk (kc = kpad).  Longer axes take chunks for which
+// two CTAs fit an SM (112 KB each): one fills its tile or writes its results
+// while the other multiplies.  The chunks do not change the order of the
+// sums.  The operand images are stored as ceil(kpad / kc) consecutive chunk
+// images of npad x kc.
 inline __host__ __device__ int tc_kchunk(int n) {
   const int npad = tc_npad(n), kpad = tc_kpad(n);
-  const int kc_max = (220 * 1024 / (8 * (npad + 128))) / 8 * 8;
+  int kc_max = (220 * 1024 / (8 * (npad + 128))) / 8 * 8;
+  if (kpad > kc_max) kc_max = (112 * 1024 / (8 * (npad + 128))) / 8 * 8;
   const int nch = (kpad + kc_max - 1) / kc_max;
   return ((kpad + nch - 1) / nch + 7) / 8 * 8;
 }

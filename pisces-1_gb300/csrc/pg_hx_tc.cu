@@ -28,6 +28,7 @@
 namespace {
 
 constexpr int kThreads = 512;  // 16 warps: the A fill and the epilogue each take one round of loads at 64^3
+constexpr int kHalfThreads = 256;  // several K chunks: two CTAs per SM
 constexpr int kTileM = 128;
 constexpr int kMaxN = 256;  // n_axis limit: the MMA N extent (rows of the axis matrix, padded to 16)
 constexpr int kBatch = 16;  // global loads a thread keeps in flight while filling A
@@ -87,6 +88,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* out) {
   for (int j = 0; j < 16; ++j) out[j] = __uint_as_float(r[j]);
 }
 
+// FP32 -> FP64 with integer operations (the conversion instruction takes 64
+// cycles of the FP64 pipe a warp, these about 20 of the integer pipe); a
+// subnormal takes the instruction.
+__device__ __forceinline__ double f32_to_f64_exact(float v) {
+  const uint32_t u = __float_as_uint(v);
+  const uint32_t sign = u & 0x80000000u, m = u & 0x7fffffu, e = (u >> 23) & 0xffu;
+  if (e == 0 || e == 255) return m ? (double)v : __hiloint2double((int)(sign | (e ? 0x7ff00000u : 0u)), 0);
+  return __hiloint2double((int)(sign | ((e + 896u) << 20) | (m >> 3)), (int)(m << 29));
+}
+
 struct AxisMap {
   int n;          // length of the contracted axis
   long stride;    // element stride along the axis
@@ -139,7 +150,7 @@ __device__ __forceinline__ void epilogue_x16(const float (&d)[16], float* stg, i
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const long c = c0w + 2 * (h + u) + half;
-      if (c < ncols && i < n) Y[(long)nx * c + i] = prev[u] + (double)val[u];
+      if (c < ncols && i < n) Y[(long)nx * c + i] = prev[u] + f32_to_f64_exact(val[u]);
     }
   }
   __syncwarp();  // the block is rewritten by the warp's next chunk
@@ -234,8 +245,8 @@ namespace {
 using pg::TcJob;
 using pg::TcJobs;
 
-template <int AXIS>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int AXIS, int TH>
+__global__ void __launch_bounds__(TH, kThreads / TH)
     k_hx_tc(int nx, int ny, int nz, AxisMap am, int npad, int kc, int nch, uint32_t tmem_cols,
             const float* __restrict__ t_hi, const float* __restrict__ t_lo, const __grid_constant__ TcJobs jobs,
             int mode, uint32_t stage_off, int* __restrict__ err) {
@@ -323,8 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (nch > 1 && !first && tid == 0) load_b(ch);  // the previous chunk's MMAs have completed
       first = false;
       // ---- A operand: 128 columns x kc, split into TF32 hi/lo
-      static_assert(kThreads / 32 == kTileM / 8, "one row group of the A tile per warp");
-      fill_a<AXIS, 1>(warp, lane, X, c0, ncols, k0, kc, n, am.stride, nx, ny, N, sAh, sAl);
+      fill_a<AXIS, kThreads / TH>(warp, lane, X, c0, ncols, k0, kc, n, am.stride, nx, ny, N, sAh, sAl);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       bool bok = true;
@@ -375,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const long base = cvalid ? col_base<AXIS>(c, nx, ny, N) : 0;
     const long gshift = cvalid ? (c / (N / n)) * N : 0;  // vector offset: grid point = address - gshift
     // one 16-row chunk per warp and round: 16 loads in flight, then the stores
-    for (int ck = group; ck * 16 < npad; ck += kThreads / 128) {
+    for (int ck = group; ck * 16 < npad; ck += TH / 128) {
       float d[16];
       tmem_ld16(tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(ck * 16), d);
       if (AXIS == 0 && stage_off != kNoStage) {
@@ -396,7 +406,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int i = ck * 16 + j;
-          if (i < n) Y[base + (long)i * am.stride] = prev[j] + (double)d[j];
+          if (i < n) Y[base + (long)i * am.stride] = prev[j] + f32_to_f64_exact(d[j]);
         }
       }
     }
@@ -595,7 +605,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1)
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int r = ck * 16 + j;
-            if (r < n) Y[base + (long)r * am.stride] = prev[j] + (double)d[j];
+            if (r < n) Y[base + (long)r * am.stride] = prev[j] + f32_to_f64_exact(d[j]);
           }
         }
       }
@@ -637,15 +647,19 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (g_num_sms <= 0) g_num_sms = 148;
-    const void* fns[6] = {(const void*)k_hx_tc<0>,      (const void*)k_hx_tc<1>,      (const void*)k_hx_tc<2>,
-                          (const void*)k_hx_tc_pipe<0>, (const void*)k_hx_tc_pipe<1>, (const void*)k_hx_tc_pipe<2>};
+    constexpr int kFns = 9;
+    const void* fns[kFns] = {(const void*)k_hx_tc<0, kThreads>,     (const void*)k_hx_tc<1, kThreads>,
+                             (const void*)k_hx_tc<2, kThreads>,     (const void*)k_hx_tc<0, kHalfThreads>,
+                             (const void*)k_hx_tc<1, kHalfThreads>, (const void*)k_hx_tc<2, kHalfThreads>,
+                             (const void*)k_hx_tc_pipe<0>,          (const void*)k_hx_tc_pipe<1>,
+                             (const void*)k_hx_tc_pipe<2>};
     int lim = optin;
-    for (int k = 0; k < 6 && e == cudaSuccess; ++k) {
+    for (int k = 0; k < kFns && e == cudaSuccess; ++k) {
       cudaFuncAttributes fa;
       e = cudaFuncGetAttributes(&fa, fns[k]);
       if (e == cudaSuccess) lim = std::min(lim, optin - (int)fa.sharedSizeBytes);
     }
-    for (int k = 0; k < 6 && e == cudaSuccess; ++k)
+    for (int k = 0; k < kFns && e == cudaSuccess; ++k)
       e = cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     g_max_dyn = lim;
     return e;
@@ -682,7 +696,11 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
   }
   // one persistent CTA of kThreads per SM, or the tuned count
   const long cap = ctas > 0 && ctas < g_num_sms ? ctas : g_num_sms;
-  const int grid = (int)(tiles < cap ? tiles : cap);
+  // several K chunks and more tiles than SMs: two CTAs of half the threads per
+  // SM (160^3 x 16: 2.25 -> 1.67 ms; with one tile per SM or fewer the wide
+  // CTA is faster, 128x64x40 x 3: 55 us against 60)
+  const bool half = nch > 1 && tiles > cap;
+  const int grid = (int)std::min<long>(tiles, half ? 2 * cap : cap);
   int* err = g->tc_err.p;
   const size_t a_region = (size_t)2 * kTileM * kc * 4, b_region = (size_t)2 * npad * kc * 4;
   // several tiles per CTA: the pipelined form overlaps them (form 0), or as tuned
@@ -710,7 +728,8 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
   }
   // x-axis epilogue blocks of all 16 warps: in the A tile (free once a tile's
   // MMAs have completed) when it is large enough, else after it
-  const size_t stage = (size_t)kThreads / 32 * kStageWarpBytes;
+  const int th = half ? kHalfThreads : kThreads;
+  const size_t stage = (size_t)th / 32 * kStageWarpBytes;
   uint32_t stage_off = kNoStage;
   size_t smem_t = smem;
   if (a == 0) {
@@ -721,19 +740,12 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
       smem_t = smem + stage;
     }
   }
-  switch (a) {
-    case 0:
-      PG_CUDA_TRY(launch_dependent(k_hx_tc<0>, dim3(grid), dim3(kThreads), smem_t, st, g->n[0], g->n[1], g->n[2], am,
-                                   npad, kc, nch, cols, Ahi, Alo, jobs, mode, stage_off, err));
-      break;
-    case 1:
-      PG_CUDA_TRY(launch_dependent(k_hx_tc<1>, dim3(grid), dim3(kThreads), smem_t, st, g->n[0], g->n[1], g->n[2], am,
-                                   npad, kc, nch, cols, Ahi, Alo, jobs, mode, stage_off, err));
-      break;
-    default:
-      PG_CUDA_TRY(launch_dependent(k_hx_tc<2>, dim3(grid), dim3(kThreads), smem_t, st, g->n[0], g->n[1], g->n[2], am,
-                                   npad, kc, nch, cols, Ahi, Alo, jobs, mode, stage_off, err));
-  }
+  const auto k = half ? (a == 0   ? k_hx_tc<0, kHalfThreads>
+                         : a == 1 ? k_hx_tc<1, kHalfThreads>
+                                  : k_hx_tc<2, kHalfThreads>)
+                      : (a == 0 ? k_hx_tc<0, kThreads> : a == 1 ? k_hx_tc<1, kThreads> : k_hx_tc<2, kThreads>);
+  PG_CUDA_TRY(launch_dependent(k, dim3(grid), dim3(th), smem_t, st, g->n[0], g->n[1], g->n[2], am, npad, kc, nch, cols,
+                               Ahi, Alo, jobs, mode, stage_off, err));
   return check_launch("k_hx_tc");
 }
 
