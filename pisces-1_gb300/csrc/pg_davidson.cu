@@ -315,11 +315,11 @@ constexpr int kPinSig = kPinLam + 16;          // preconditioner shifts (2 x 16)
 constexpr int kPinTotal = kPinSig + 32;
 static_assert(kRsq + 16 <= 96, "hsq region");
 
-pg_status ensure_scratch(pg_davidson* d, int ndim, int maxsub, int nroots) {
+pg_status ensure_scratch(pg_davidson* d, int ndim, int maxsub, int nroots, cudaStream_t st) {
   // grow-only scratch: a reused handle allocates only while its problems grow
   PG_TRY(d->dcoef.ensure((size_t)std::max(maxsub * maxsub, 2 * kMaxGramOut)));
   PG_TRY(d->dgram.ensure((size_t)kMaxGramOut));
-  PG_TRY(d->rs.ensure());
+  PG_TRY(d->rs.ensure(st));
   PG_TRY(d->pip_skip.ensure(1));
   PG_TRY(d->hpin.ensure(kPinTotal));
   if (d->dfloat) {
@@ -331,7 +331,10 @@ pg_status ensure_scratch(pg_davidson* d, int ndim, int maxsub, int nroots) {
     PG_TRY(d->dsq.alloc(kScalars));
     std::vector<double> init(kScalars, 0.0);
     for (int i = 0; i < 16; ++i) init[kOnes + i] = 1.0;
-    PG_CUDA_TRY(cudaMemcpy(d->dsq.p, init.data(), sizeof(double) * kScalars, cudaMemcpyHostToDevice));
+    // on the solve's stream: a copy on the legacy stream may still be in flight
+    // when a non-blocking stream's kernels read it
+    PG_CUDA_TRY(cudaMemcpyAsync(d->dsq.p, init.data(), sizeof(double) * kScalars, cudaMemcpyHostToDevice, st));
+    PG_CUDA_TRY(cudaStreamSynchronize(st));
   }
   d->ndim = ndim;
   d->maxsub = maxsub;
@@ -606,7 +609,7 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
   if (corrflag == 3) PG_ARG(d->pc_grid->N == ndim, "pg_davidson_rci: preconditioner grid does not match ndim");
 
   if (d->status == 0) {  // first call (src/Davidson.cpp:145-193)
-    PG_TRY(ensure_scratch(d, ndim, maxsub, nroots));
+    PG_TRY(ensure_scratch(d, ndim, maxsub, nroots, st));
     d->pc_olsen = false;
     if (corrflag == 3) {  // is V identically zero? (diag(H) equals the kinetic diagonal)
       const pg_grid* g = d->pc_grid;

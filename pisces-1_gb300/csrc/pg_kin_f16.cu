@@ -784,7 +784,8 @@ static pg_status kin_counters(const pg_grid* g, cudaStream_t st, KinCounters** o
     }
     std::unique_ptr<DevBuf<unsigned>> b(new DevBuf<unsigned>());
     PG_TRY(b->alloc(sizeof(KinCounters) / sizeof(unsigned)));
-    PG_CUDA_TRY(cudaMemset(b->p, 0, sizeof(KinCounters)));
+    // zeroed on the stream that uses it: other streams do not wait for the legacy one
+    PG_CUDA_TRY(cudaMemsetAsync(b->p, 0, sizeof(KinCounters), st));
     it = g->fused_cnt.emplace(key, std::move(b)).first;
   }
   *out = reinterpret_cast<KinCounters*>(it->second->p);

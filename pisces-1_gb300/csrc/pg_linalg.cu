@@ -529,11 +529,13 @@ pg_status reduce(const double* partial, int nb, int no, double* out, bool sqrt_m
 
 }  // namespace
 
-pg_status RedScratch::ensure() {
+pg_status RedScratch::ensure(cudaStream_t st) {
   if (!partial.p) PG_TRY(partial.alloc((size_t)kRedBlocks * kMaxGramOut));
   if (!counter.p) {
     PG_TRY(counter.alloc(1));
-    PG_CUDA_TRY(cudaMemset(counter.p, 0, sizeof(unsigned)));
+    // complete before any stream can use it (none waits for the legacy stream)
+    PG_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned), st));
+    PG_CUDA_TRY(cudaStreamSynchronize(st));
   }
   return PG_OK;
 }
@@ -578,7 +580,7 @@ pg_status gram(long N, const double* P, int na, const double* Q, int nb, double*
                cudaStream_t st, bool dfloat, const double* Pt, const double* Qt, const int* skip) {
   PG_ARG(na > 0 && nb > 0 && na * nb <= kMaxGramOut && na + nb <= 144, "gram: %d x %d outputs exceed the limits",
          na, nb);
-  PG_TRY(rs.ensure());
+  PG_TRY(rs.ensure(st));
   PG_TRY(opt_in_smem());
   const long chunk = chunk_for(N, kRedBlocks, kTP);
   const int blocks = (int)((N + chunk - 1) / chunk);
@@ -611,7 +613,7 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
                   cudaStream_t st, bool dfloat, const double* Pt, double* Yt, const int* skip) {
   PG_ARG(nr > 0 && nr <= kMaxCombine && na >= 0 && na * nr <= 128 * kMaxCombine, "combine: bad sizes na=%d nr=%d",
          na, nr);
-  PG_TRY(rs.ensure());
+  PG_TRY(rs.ensure(st));
   PG_TRY(opt_in_smem());
   const long chunk = chunk_for(N, kStreamBlocks, kT);
   const int blocks = (int)((N + chunk - 1) / chunk);
@@ -779,7 +781,7 @@ pg_status ritz_df(long N, const double* Bt, const double* Zt, int m, const doubl
                   double* U, double* W, int nr, double* sq, RedScratch& rs, cudaStream_t st) {
   PG_ARG(m > 0 && nr > 0 && nr <= kMaxCombine && m * nr <= 128 * kMaxCombine && Bt && Zt,
          "ritz_df: bad sizes m=%d nr=%d", m, nr);
-  PG_TRY(rs.ensure());
+  PG_TRY(rs.ensure(st));
   const long chunk = chunk_for(N, kStreamBlocks, kT);
   const int blocks = (int)((N + chunk - 1) / chunk);
   const size_t smem = sizeof(float) * 2 * (size_t)m * nr;

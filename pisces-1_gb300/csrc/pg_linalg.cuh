@@ -20,7 +20,7 @@ constexpr int kMaxCombine = 16;  // columns produced by one combine launch
 struct RedScratch {
   DevBuf<double> partial;     // kRedBlocks * kMaxGramOut
   DevBuf<unsigned> counter;   // arrival count of reduce_in_last_block (zero between launches)
-  pg_status ensure();
+  pg_status ensure(cudaStream_t st);
 };
 
 // Ends a kernel whose block b has written its partial row partial[b*no + o],

@@ -5,7 +5,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,nvec", [((130, 40, 39), 14), ((33, 128, 40), 16), ((20, 36, 161), 28), ((256, 16, 9), 70)])
+@pytest.mark.parametrize("n,nvec", [((130, 40, 39), 14), ((33, 128, 40), 16), ((20, 36, 161), 28), ((256, 16, 9), 140)])
 def test_block_equals_single_vectors(pg, n, nvec):
     import torch
     g = pg.Grid(n, tuple(0.6 * (m + 1) for m in n))
