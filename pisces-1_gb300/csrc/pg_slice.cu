@@ -3,15 +3,22 @@
 // kinetic preconditioner of the FP64 form are three and six of these.
 //
 // Grid lines along the axis are the rows of the left operand: a CTA takes
-// 128 of them, converts their values to digit images once (each line scaled
-// by its own largest exponent), and multiplies them with the matrix's digit
-// images, which the bulk copy engine fetches from L2.  The tensor core's
+// 128 of them (fewer on small grids), converts their values to digit images
+// once (each line scaled by its own largest exponent), and multiplies them
+// with the matrix's digit images, which the bulk copy engine fetches from L2.  The tensor core's
 // accumulators (7 x nc columns of TMEM) are read back one line per lane.
 //
 // Bounds: per point and axis about 35 integer operations to make the digits,
 // 60 to join the accumulators and one or two FP64 operations (V X, the sum
 // into Y), against n FP64 multiply-adds before; the FP64 pipe is about 60
-// times slower than the integer pipes here.
+// times slower than the integer pipes here.  A tile of 128 lines of 64 points
+// spends 4000 cycles on loading, 6000 on digits and 13000 on the read-out;
+// the products run beside the read-out.
+//
+// H X, FP64 multiply-adds / one accumulator set and K chunks of 64 (digits
+// made again for each 64 outputs) / as here, us: 32^3 33.5 / 30.7 / 20.8,
+// 64^3 x 4 371 / 52.8 / 54.4, 83x90x71 x 6 1814 / 245 / 173, 96^3 x 8 3428 /
+// 498 / 342, 160^3 x 16 (K chunks) 63060 / 5586 / 5543.
 #include <algorithm>
 #include <cmath>
 
@@ -21,9 +28,8 @@
 namespace {
 
 constexpr int kLines = 128;  // MMA M
-constexpr int kST = 512;     // threads: four per line
-constexpr int kTransPitch = 5;
-constexpr int kTransBytes = (kST / 32) * 32 * kTransPitch * 8;  // 32 lines x 4 columns per warp
+constexpr int kST = 512;     // threads that fill and read out
+constexpr int kTransMost = (kST / 32) * 32 * 5 * 8;  // transpose buffer: 32 lines x 4 columns per warp
 
 // A line whose largest exponent lies outside [kExpLo, kExpHi] (subnormal or
 // huge values, infinities, NaN) is multiplied with FP64 multiply-adds instead.
@@ -34,53 +40,69 @@ struct SliceArgs {
   long inner;    // stride of the axis
   long npts;     // points of one vector (index of V)
   int n, kc, nnc, nc;
+  int lc;        // lines per CTA: 128, or 64 or 32 where that still leaves one CTA per SM at most
   int h0, nch;   // K chunks [h0, h0 + nch) of this launch
   int plain;     // every line by FP64 multiply-adds
-  int rebuild;   // more than one K chunk per axis: the digit images are rebuilt for every N chunk
   int nc_per;    // N chunks per CTA (blockIdx.y takes the next ones)
   int scale;     // exponent of accumulator 6: kSliceUnit - tau - 1075 - kSliceGuard
   uint32_t block_bytes;  // one (K, N) block of the matrix image
-  uint32_t slice_b;      // bytes of one slice in it
-  uint32_t off_b, off_t; // shared-memory offsets of the matrix block and the transpose buffer
+  uint32_t off_b, off_t; // shared-memory offsets of the matrix blocks and the transpose buffer
+  int tc;                // columns transposed at a time: 4, or 2 where shared memory is short
   uint32_t tmem_cols;
   int mode;              // 0: y = K, 1: y += K, 2: y = v x + K, 3: row dots x . K
   long out0;             // mode 3: first output row of this launch, in values
   long sa, sb;           // strides of A64 (output, input index)
 };
 
-template <int NU>
-__global__ void __launch_bounds__(kST, 1)
+// kChunks false: the whole axis in one K chunk (n <= 96).  The lines' digits
+// are made once; the matrix comes in chunks of nc columns, double buffered,
+// into two halves of tensor memory, so that a chunk's products run while the
+// one before is read out.
+// kChunks true: K chunks of at most 80, N chunks of 64; the digits are made
+// again for every N chunk.
+// The products of the former are issued by a warp of its own (the 17th), which
+// waits for the matrix blocks and for the accumulators to be read: issued
+// by a thread that also reads out, two chunks of 64^3 took 5600 cycles before
+// its read-out began.
+template <int NU, bool kChunks>
+__global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     k_slice_axis(const SliceArgs A, const unsigned char* __restrict__ img, const double* __restrict__ A64,
                  const double* __restrict__ v, const double* __restrict__ x, double* y, int* __restrict__ err) {
   constexpr int NS = pg::kSliceN;
+  constexpr int kBuf = kChunks ? 1 : 2;  // matrix blocks and accumulator sets
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bar_b, bar_mma;
+  __shared__ __align__(8) uint64_t bar_b[kBuf], bar_mma[kBuf], bar_read[kBuf];
   __shared__ uint32_t tmem_base;
   __shared__ int s_emax[kLines];
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int line = tid & (kLines - 1), part = tid >> 7;
   const int c_first = blockIdx.y * A.nc_per;
   const int c_end = c_first + A.nc_per < A.nnc ? c_first + A.nc_per : A.nnc;
   const uint32_t sA = smem_u32(smem), sB = sA + A.off_b;
 
-  auto load_b = [&](int c, int h) {  // one thread: block (h, c) of the matrix image
+  auto load_b = [&](int c, int h, int b) {  // one thread: block (h, c) of the matrix image into buffer b
     uint64_t state;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 %0, [%1], %2;"
                  : "=l"(state)
-                 : "r"(smem_u32(&bar_b)), "r"(A.block_bytes)
+                 : "r"(smem_u32(&bar_b[b])), "r"(A.block_bytes)
                  : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sB),
-                 "l"(img + (size_t)((A.h0 + h) * A.nnc + c) * A.block_bytes), "r"(A.block_bytes), "r"(smem_u32(&bar_b))
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     sB + (uint32_t)b * A.block_bytes),
+                 "l"(img + (size_t)((A.h0 + h) * A.nnc + c) * A.block_bytes), "r"(A.block_bytes),
+                 "r"(smem_u32(&bar_b[b]))
                  : "memory");
   };
   if (tid == 0) {
     s_fail = 0;
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_b)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_mma)));
+    for (int b = 0; b < kBuf; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_b[b])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_mma[b])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_read[b])), "r"(kST / 32));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    load_b(c_first, 0);  // constant data: before the kernel ahead has finished
+    // constant data: before the kernel ahead has finished
+    for (int b = 0; b < kBuf && c_first + b < c_end; ++b) load_b(c_first + b, 0, b);
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
@@ -95,18 +117,21 @@ __global__ void __launch_bounds__(kST, 1)
   pg::pdl_release();
   const uint32_t tmem = tmem_base;
 
-  const long l0 = blockIdx.x * (long)kLines;
   const bool contig = A.inner == 1;
-  const bool valid = l0 + line < A.nlines;
-  const long base = [&] {  // first point of this thread's line
-    const long l = valid ? l0 + line : 0;
+  const long l0 = blockIdx.x * (long)A.lc;
+  const int lend = A.nlines - l0 < A.lc ? (int)(A.nlines - l0) : A.lc;  // lines of this CTA
+  // filling: this thread's line, and its octets part, part + parts, ...
+  const int line = tid & (A.lc - 1), part = tid / A.lc, parts = kST / A.lc;
+  // read-out: this thread's TMEM lane
+  const int row = 32 * (warp & 3) + lane, wpart = warp >> 2;
+  auto first_point = [&](int r) {  // of line r of the tile
+    const long l = r < lend ? l0 + r : 0;
     return contig ? l * A.n : (l / A.inner) * A.inner * A.n + l % A.inner;
-  }();
+  };
   const int koct = A.kc >> 3;
   const int k_end = (A.h0 + A.nch) * A.kc < A.n ? (A.h0 + A.nch) * A.kc : A.n;
 
   double val[NU][8];
-  // this thread's octets (part, part + 4, ...) of K chunk h
   auto load_chunk = [&](int h) {
     const int k0 = (A.h0 + h) * A.kc;
     const int kn = A.n - k0 < A.kc ? A.n - k0 : A.kc;
@@ -115,8 +140,7 @@ __global__ void __launch_bounds__(kST, 1)
       // images' place), odd pitch
       double* raw = reinterpret_cast<double*>(smem);
       const int pitch = A.kc | 1;
-      const long lend = A.nlines - l0 < kLines ? A.nlines - l0 : kLines;
-      for (int r = warp; r < kLines; r += kST / 32)
+      for (int r = warp; r < A.lc; r += kST / 32)
         for (int k = lane; k < A.kc; k += 32) {
           const bool in = r < lend && k < kn;
           const double* src = x + (in ? (l0 + r) * A.n + k0 + k : 0);
@@ -125,21 +149,22 @@ __global__ void __launch_bounds__(kST, 1)
                        : "memory");
         }
       asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
+      named_sync(1, kST);
 #pragma unroll
       for (int u = 0; u < NU; ++u) {
-        const int o = part + 4 * u;
+        const int o = part + parts * u;
 #pragma unroll
         for (int q = 0; q < 8; ++q) val[u][q] = o < koct ? raw[line * pitch + 8 * o + q] : 0.0;
       }
     } else {
+      const double* src = x + first_point(line);
 #pragma unroll
       for (int u = 0; u < NU; ++u) {
-        const int o = part + 4 * u;
+        const int o = part + parts * u;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int k = 8 * o + q;
-          val[u][q] = (valid && o < koct && k < kn) ? x[base + (long)(k0 + k) * A.inner] : 0.0;
+          val[u][q] = (line < lend && o < koct && k < kn) ? src[(long)(k0 + k) * A.inner] : 0.0;
         }
       }
     }
@@ -157,153 +182,133 @@ __global__ void __launch_bounds__(kST, 1)
       }
     if (em) atomicMax(&s_emax[line], (int)em);
   };
-
-  // The four outputs of a read-out batch are y[p + q step], q < cnt: four
-  // columns of the thread's own line, or, where lines are contiguous and the
-  // batch is transposed, one column of four lines.
-  struct Out {
-    long p;
-    int cnt;
-  };
-  const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-  double* tb = reinterpret_cast<double*>(smem + A.off_t) + warp * 32 * kTransPitch;
-  const int nbatch = A.nc >> 2;
-  const long lt = l0 + 32 * (warp & 3) + (lane >> 2);
-  const long ostep = contig ? 8L * A.n : A.inner;
-  const int rows_left = lt < A.nlines ? (int)((A.nlines - lt + 7) / 8 < 4 ? (A.nlines - lt + 7) / 8 : 4) : 0;
-  auto out_of = [&](int c, int bt) {
-    Out o;
-    const int i = c * A.nc + 4 * bt;
-    if (contig) {
-      o.p = lt * A.n + i + (lane & 3);
-      o.cnt = i + (lane & 3) < A.n ? rows_left : 0;
-    } else {
-      o.p = base + i * A.inner;
-      o.cnt = valid ? (A.n - i < 4 ? A.n - i : 4) : 0;
+  // a line's scale, once its maximum is complete; slow: by FP64 multiply-adds
+  auto is_slow = [&](int em) { return A.plain || (em != 0 && (em < kExpLo || em > kExpHi)); };
+  const uint32_t lbo = 128, sbo = (uint32_t)koct * 128u;
+  const uint32_t a_slice = (uint32_t)kLines * (uint32_t)A.kc * 2u;
+  // digits: one 16-byte row of a core matrix per slice and octet
+  auto convert = [&] {
+    const int em = s_emax[line];
+    const bool slow = is_slow(em);
+    const int emax = slow ? 0 : em;
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+      const int o = part + parts * u;
+      if (o < koct) {
+        uint32_t w[NS][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const unsigned long long f0 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q], emax);
+          const unsigned long long f1 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q + 1], emax);
+#pragma unroll
+          for (int i = 0; i < NS; ++i) w[i][q] = pg::slice_digit2(f0, f1, i);
+        }
+        const uint32_t dst = (uint32_t)((line >> 3) * koct + o) * 128u + (uint32_t)(line & 7) * 16u;
+#pragma unroll
+        for (int i = 0; i < NS; ++i)
+          *reinterpret_cast<uint4*>(smem + (uint32_t)i * a_slice + dst) =
+              make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+      }
     }
-    return o;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  };
+  // One thread: the products of the digits with matrix block b into
+  // accumulator set b, once the block has landed.  Digit i of the lines meets
+  // digits 0 .. 6 - i of the matrix, which lie one under the other in shared
+  // memory as one operand of (7 - i) nc rows, in accumulators i .. 6, which
+  // lie side by side: at most 256 columns an instruction (one product at a
+  // time read the lines' digits 28 times instead of 10, and took 7700 cycles
+  // a tile of 64 x 64; so, and with the descriptors counted up, 4600).
+  auto issue = [&](int b, uint32_t parity, bool first) {
+    if (!mbar_wait(smem_u32(&bar_b[b]), parity)) {
+      s_fail = 1;
+      mbar_arrive(smem_u32(&bar_mma[b]));  // nothing was issued: release the others
+      return;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint64_t dA = smem_desc(sA, lbo, sbo), dB = smem_desc(sB + (uint32_t)b * A.block_bytes, lbo, sbo);
+    const uint32_t id0 = (1u << 4) | ((uint32_t)(kLines >> 4) << 24);
+    const uint32_t d0 = tmem + (uint32_t)b * (A.tmem_cols >> 1);
+    for (int kk = 0; kk < (koct >> 1); ++kk) {
+#pragma unroll
+      for (int i = 0; i < NS; ++i) {
+        const uint64_t da = dA + (((uint32_t)i * a_slice + (uint32_t)kk * 256u) >> 4);
+        const int all = (NS - i) * A.nc;
+        const uint32_t acc = (!first || kk > 0 || i > 0) ? 1u : 0u;
+        mma_f16(d0 + (uint32_t)(i * A.nc), da, dB + (uint32_t)kk * 16u,
+                id0 | ((uint32_t)((all < 256 ? all : 256) >> 3) << 17), acc);
+        if (kChunks && all > 256)
+          mma_f16(d0 + (uint32_t)(i * A.nc + 256), da, dB + (uint32_t)kk * 16u + (((256u >> 3) * sbo) >> 4),
+                  id0 | ((uint32_t)((all - 256) >> 3) << 17), acc);
+      }
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+        smem_u32(&bar_mma[b])));
+  };
+  // The four outputs of a read-out batch: four columns of the thread's own
+  // line, or, where lines are contiguous and the batch is transposed, columns
+  // of neighbouring lines; addresses p + step[q].
+  const bool reads = 32 * (warp & 3) < A.lc;  // this warp's lanes hold lines
+  const bool valid = row < lend;
+  const long base = first_point(row);
+  const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+  const int tc = A.tc;
+  double* tb = reinterpret_cast<double*>(smem + A.off_t) + warp * 32 * (tc + 1);
+  const int nbatch = A.nc >> 2;
+  const int tcol = lane & (tc - 1), tline = lane / tc;  // transposed: lane = (line of 32 / tc, column)
+  const int rows_t = lend - 32 * (warp & 3) - tline;    // lines from this lane's on
+  const long istep = contig ? 1 : A.inner;
+  const long pbase = contig ? (l0 + 32 * (warp & 3) + tline) * A.n + tcol : base;
+  const long vector0 = base - base % A.npts;  // a line lies within one vector
+  const long step1 = !contig ? A.inner : (tc == 4 ? 8L : 16L) * A.n;
+  const long step2 = !contig ? 2 * A.inner : (tc == 4 ? 16L * A.n : 2L);
+  const long step3 = step1 + step2;
+  auto outputs = [&](int i) {  // which of the four exist, column i on
+    if (!contig) return valid ? (A.n - i >= 4 ? 15 : (1 << (A.n - i > 0 ? A.n - i : 0)) - 1) : 0;
+    if (tc == 4) return i + tcol < A.n ? (rows_t > 0) | (rows_t > 8) << 1 | (rows_t > 16) << 2 | (rows_t > 24) << 3 : 0;
+    const int lines = (rows_t > 0) | (rows_t > 16) << 1;
+    return (i + tcol < A.n ? lines : 0) | (i + tcol + 2 < A.n ? lines << 2 : 0);
   };
   double dot = 0.0;     // mode 3
   double pa[4], pb[4];  // what the next batch is added to: y, or x and v
-  auto prefetch = [&](const Out& o) {
-    const double* s = A.mode == 1 ? y : x;
-    if (A.mode == 1 || A.mode == 2) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) pa[q] = q < o.cnt ? s[o.p + q * ostep] : 0.0;
-    }
-    if (A.mode == 2) {
-      const long pv = o.p % A.npts;  // a line lies within one vector
-#pragma unroll
-      for (int q = 0; q < 4; ++q) pb[q] = q < o.cnt ? v[pv + q * ostep] : 0.0;
+  auto prefetch = [&](int i, long p) {
+    if ((A.mode != 1 && A.mode != 2) || !reads) return;
+    const double* s = (A.mode == 1 ? y : x) + p;
+    const int m = outputs(i);
+    pa[0] = m & 1 ? s[0] : 0.0;
+    pa[1] = m & 2 ? s[step1] : 0.0;
+    pa[2] = m & 4 ? s[step2] : 0.0;
+    pa[3] = m & 8 ? s[step3] : 0.0;
+    if (A.mode == 2) {  // never with contiguous lines
+      const double* w = v + (p - vector0);
+      pb[0] = m & 1 ? w[0] : 0.0;
+      pb[1] = m & 2 ? w[step1] : 0.0;
+      pb[2] = m & 4 ? w[step2] : 0.0;
+      pb[3] = m & 8 ? w[step3] : 0.0;
     }
   };
-
-  bool ok = true;
-  int waits_b = 0, waits_m = 0;
-  int emax = 0;
-  bool slow = false;
-  auto settle = [&] {  // after the line maxima are complete
-    emax = s_emax[line];
-    slow = A.plain || (emax != 0 && (emax < kExpLo || emax > kExpHi));
-    if (slow) emax = 0;
-  };
-  if (A.nch > 1) {
-    for (int h = 0; h < A.nch; ++h) {
-      load_chunk(h);
-      chunk_emax();
-      __syncthreads();
-    }
-    settle();
-  }
-  const uint32_t lbo = 128, sbo = (uint32_t)koct * 128u;
-  const uint32_t a_slice = (uint32_t)kLines * (uint32_t)A.kc * 2u;
-  for (int c = c_first; c < c_end && ok; ++c) {
-    for (int h = 0; h < A.nch && ok; ++h) {
-      if (A.rebuild || c == c_first) {
-        load_chunk(h);
-        if (A.nch == 1) chunk_emax();
-        __syncthreads();  // the staging area is read; with one chunk also the maxima
-        if (A.nch == 1) settle();
-        // digits: one 16-byte row of a core matrix per slice and octet
-#pragma unroll
-        for (int u = 0; u < NU; ++u) {
-          const int o = part + 4 * u;
-          if (o < koct) {
-            uint32_t w[NS][4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const unsigned long long f0 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q], emax);
-              const unsigned long long f1 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q + 1], emax);
-#pragma unroll
-              for (int i = 0; i < NS; ++i) w[i][q] = pg::slice_digit2(f0, f1, i);
-            }
-            const uint32_t dst = (uint32_t)((line >> 3) * koct + o) * 128u + (uint32_t)(line & 7) * 16u;
-#pragma unroll
-            for (int i = 0; i < NS; ++i)
-              *reinterpret_cast<uint4*>(smem + (uint32_t)i * a_slice + dst) =
-                  make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
-          }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      }
-      __syncthreads();
-      if (tid == 0) {
-        if (mbar_wait(smem_u32(&bar_b), (uint32_t)(waits_b & 1))) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // digit i of the lines against digits 0 .. 6 - i of the matrix,
-          // which lie one under the other in shared memory as one operand of
-          // (7 - i) nc rows, into accumulators i .. 6, which lie side by side:
-          // at most 256 columns an instruction (one product at a time read
-          // the lines' digits 28 times instead of 10: 7700 cycles a tile
-          // of 64 x 64 against 6600)
-          for (int kk = 0; kk < (koct >> 1); ++kk) {
-#pragma unroll
-            for (int i = 0; i < NS; ++i) {
-              const uint64_t da = smem_desc(sA + (uint32_t)i * a_slice + (uint32_t)kk * 256u, lbo, sbo);
-              for (int c0 = 0; c0 < (NS - i) * A.nc; c0 += 256) {
-                const int cols = (NS - i) * A.nc - c0 < 256 ? (NS - i) * A.nc - c0 : 256;
-                const uint32_t idesc =
-                    (1u << 4) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kLines >> 4) << 24);
-                mma_f16(tmem + (uint32_t)(i * A.nc + c0), da,
-                        smem_desc(sB + (uint32_t)(c0 >> 3) * sbo + (uint32_t)kk * 256u, lbo, sbo), idesc,
-                        (h > 0 || kk > 0 || i > 0) ? 1u : 0u);
-              }
-            }
-          }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-              smem_u32(&bar_mma)));
-        } else {
-          s_fail = 1;
-          mbar_arrive(smem_u32(&bar_mma));  // nothing was issued: release the others
-        }
-      }
-      ++waits_b;
-      if (h + 1 == A.nch) prefetch(out_of(c, part));
-      ok = __syncthreads_and(mbar_wait(smem_u32(&bar_mma), (uint32_t)(waits_m & 1)) && !*(volatile int*)&s_fail) != 0;
-      ++waits_m;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tid == 0 && ok) {  // the next block while this one is read out
-        if (h + 1 < A.nch) load_b(c, h + 1);
-        else if (c + 1 < c_end) load_b(c + 1, 0);
-      }
-    }
-    if (!ok) {
-      if (tid == 0) atomicExch(err, 1);
-      break;
-    }
-    // read-out: this thread's line (its TMEM lane), four columns at a time
-    for (int bt = part; bt < nbatch; bt += 4) {
+  // first column and address of this warp's first batch of N chunk c
+  auto first_col = [&](int c) { return c * A.nc + 4 * wpart; };
+  auto first_at = [&](int c) { return pbase + (long)first_col(c) * istep; };
+  auto readout = [&](int c, uint32_t tset, bool more) {
+    if (!reads) return;
+    const int em = s_emax[row];
+    const bool slow = is_slow(em);
+    const int emax = slow ? 0 : em;
+    int i = first_col(c);
+    long p = first_at(c);
+    for (int bt = wpart; bt < nbatch; bt += 4, i += 16, p += 16 * istep) {
       uint32_t r[pg::kSliceAcc][4];
 #pragma unroll
       for (int d = 0; d < pg::kSliceAcc; ++d)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(r[d][0]), "=r"(r[d][1]), "=r"(r[d][2]), "=r"(r[d][3])
-                     : "r"(trow + (uint32_t)(d * A.nc + 4 * bt)));
+                     : "r"(trow + tset + (uint32_t)(d * A.nc + 4 * bt)));
       double a0[4], b0[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) a0[q] = pa[q], b0[q] = pb[q];
-      const Out o = out_of(c, bt);
-      if (bt + 4 < nbatch) prefetch(out_of(c, bt + 4));
+      if (bt + 4 < nbatch) prefetch(i + 16, p + 16 * istep);
+      else if (more) prefetch(first_col(c + 1), first_at(c + 1));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
       for (int d = 0; d < pg::kSliceAcc; ++d)  // the values are read after the wait
@@ -319,54 +324,126 @@ __global__ void __launch_bounds__(kST, 1)
       if (slow && valid) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int i = c * A.nc + 4 * bt + q;
           double s = 0.0;
 #pragma unroll 1
-          for (int b = A.h0 * A.kc; i < A.n && b < k_end; ++b) s = fma(A64[i * A.sa + b * A.sb], x[base + b * A.inner], s);
+          for (int b = A.h0 * A.kc; i + q < A.n && b < k_end; ++b)
+            s = fma(A64[(i + q) * A.sa + b * A.sb], x[base + b * A.inner], s);
           k[q] = s;
         }
       }
       if (A.mode == 3) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int i = c * A.nc + 4 * bt + q;
-          if (valid && i < A.n) dot = fma(x[base + i], k[q], dot);
-        }
+        for (int q = 0; q < 4; ++q)
+          if (valid && i + q < A.n) dot = fma(x[base + i + q], k[q], dot);
         continue;
       }
       if (contig) {
-        // 32 lines x 4 columns through the warp's buffer, so that four lanes
-        // write one line's 32 bytes
+        // through the warp's buffer, so that neighbouring lanes write
+        // neighbouring values of a line
+        if (tc == 4) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) tb[lane * kTransPitch + q] = k[q];
-        __syncwarp();
+          for (int q = 0; q < 4; ++q) tb[lane * 5 + q] = k[q];
+          __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) k[q] = tb[(8 * q + (lane >> 2)) * kTransPitch + (lane & 3)];
-        __syncwarp();
+          for (int q = 0; q < 4; ++q) k[q] = tb[(8 * q + tline) * 5 + tcol];
+          __syncwarp();
+        } else {
+#pragma unroll
+          for (int g = 0; g < 4; g += 2) {
+            tb[lane * 3] = k[g];
+            tb[lane * 3 + 1] = k[g + 1];
+            __syncwarp();
+            k[g] = tb[tline * 3 + tcol];
+            k[g + 1] = tb[(16 + tline) * 3 + tcol];
+            __syncwarp();
+          }
+        }
       }
+      const int m = outputs(i);
+      double* out = y + p;
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (q < o.cnt) {
-          double* p = y + o.p + q * ostep;
-          if (A.mode == 0) *p = k[q];
-          else if (A.mode == 1) *p = a0[q] + k[q];
-          else *p = fma(b0[q], a0[q], k[q]);
+        if (m >> q & 1) {
+          const double w = A.mode == 0 ? k[q] : (A.mode == 1 ? a0[q] + k[q] : fma(b0[q], a0[q], k[q]));
+          out[q == 0 ? 0 : (q == 1 ? step1 : (q == 2 ? step2 : step3))] = w;
         }
     }
-    // the accumulators are read before the next chunk's products
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  };
+  bool ok = true;
+  if constexpr (!kChunks) {
+    if (warp < kST / 32) {
+      load_chunk(0);
+      chunk_emax();
+      named_sync(1, kST);  // the maxima are complete, the staging area is read
+      convert();
+    }
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp < kST / 32) {
+      prefetch(first_col(c_first), first_at(c_first));
+      for (int c = c_first; c < c_end; ++c) {
+        const int b = (c - c_first) & 1;
+        ok = mbar_wait(smem_u32(&bar_mma[b]), (uint32_t)((c - c_first) >> 1 & 1)) && !*(volatile int*)&s_fail && ok;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (ok) readout(c, (uint32_t)b * (A.tmem_cols >> 1), c + 1 < c_end);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_read[b]));
+      }
+    } else if (lane == 0) {
+      for (int c = c_first; c < c_end; ++c) {
+        const int b = (c - c_first) & 1, use = (c - c_first) >> 1;
+        if (use > 0) {
+          // the matrix block is free once its products are done, the
+          // accumulators once they are read
+          ok = mbar_wait(smem_u32(&bar_mma[b]), (uint32_t)((use - 1) & 1)) && ok;
+          load_b(c, 0, b);
+          ok = mbar_wait(smem_u32(&bar_read[b]), (uint32_t)((use - 1) & 1)) && ok;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        issue(b, (uint32_t)(use & 1), true);
+      }
+    }
+  } else {
+    for (int h = 0; h < A.nch; ++h) {
+      load_chunk(h);
+      chunk_emax();
+      __syncthreads();
+    }
+    uint32_t turn = 0;
+    for (int c = c_first; c < c_end && ok; ++c) {
+      for (int h = 0; h < A.nch && ok; ++h, ++turn) {
+        load_chunk(h);
+        __syncthreads();  // the staging area is read
+        convert();
+        __syncthreads();
+        if (tid == 0) issue(0, turn & 1u, h == 0);
+        if (h + 1 == A.nch) prefetch(first_col(c), first_at(c));
+        ok = __syncthreads_and(mbar_wait(smem_u32(&bar_mma[0]), turn & 1u) && !*(volatile int*)&s_fail) != 0;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (tid == 0 && ok) {  // the next block while this one is read out
+          if (h + 1 < A.nch) load_b(c, h + 1, 0);
+          else if (c + 1 < c_end) load_b(c + 1, 0, 0);
+        }
+      }
+      if (!ok) break;
+      readout(c, 0u, false);
+      // the accumulators are read before products into them
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncthreads();
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
   }
+  if (!ok && lane == 0) atomicExch(err, 1);
   if (A.mode == 3) {
     // the four threads of a line, in order
     double* sd = reinterpret_cast<double*>(smem + A.off_t);
     __syncthreads();
-    sd[part * kLines + line] = dot;
+    if (warp < kST / 32) sd[wpart * kLines + row] = dot;
     __syncthreads();
-    if (part == 0 && valid)
-      y[A.out0 + (long)blockIdx.y * A.nlines + l0 + line] =
-          ((dot + sd[kLines + line]) + sd[2 * kLines + line]) + sd[3 * kLines + line];
+    if (wpart == 0 && valid)
+      y[A.out0 + (long)blockIdx.y * A.nlines + l0 + row] =
+          ((dot + sd[kLines + row]) + sd[2 * kLines + row]) + sd[3 * kLines + row];
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -399,26 +476,35 @@ __global__ void k_slice_matrix(const SliceBuild B) {
   }
 }
 
-template <int NU>
+constexpr int kSmemMost = 226 * 1024;
+
+template <int NU, bool kChunks>
 cudaError_t launch_slice(const SliceArgs& a, dim3 grid, size_t smem, const unsigned char* img, const double* A64,
                          const double* v, const double* x, double* y, int* err, cudaStream_t st) {
   static const cudaError_t attr =
-      cudaFuncSetAttribute(k_slice_axis<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+      cudaFuncSetAttribute(k_slice_axis<NU, kChunks>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
   if (attr != cudaSuccess) return attr;
-  return pg::launch_dependent(k_slice_axis<NU>, grid, dim3(kST), smem, st, a, img, A64, v, x, y, err);
+  return pg::launch_dependent(k_slice_axis<NU, kChunks>, grid, dim3(kST + (kChunks ? 0 : 32)), smem, st, a, img, A64, v, x, y, err);
 }
 
 }  // namespace
 
 namespace pg {
 
+// Up to 96 points: one K chunk, N chunks of 32 (two sets of 7 accumulators in
+// 512 columns of tensor memory; the lines' digits and two blocks of the
+// matrix's in shared memory), or of 16 where shared memory asks for it (above
+// 80 points) and on short axes, whose small grids then spread over more CTAs.
+// The digits of 81 to 96 points made once instead of twice: 96^3 x 8 498 ->
+// 342 us; 32 points in two chunks on CTAs of their own: 30 -> 21 us a product.
+// Longer axes: K chunks of at most 80, N chunks of 64.
 static void slice_shape(int n, SliceMat* S) {
   S->n = n;
-  // K chunks of at most 80: 128 lines' digits and 64 matrix rows' fit shared memory
-  S->nch = (n + 79) / 80;
+  S->nch = n <= 96 ? 1 : (n + 79) / 80;
   S->kc = ((n + S->nch - 1) / S->nch + 15) / 16 * 16;
   const int npad = (n + 15) / 16 * 16;
-  S->nnc = (npad + 63) / 64;  // 7 accumulators of at most 64 columns in TMEM
+  const int most = S->nch > 1 ? 64 : (n > 80 || n <= 32 ? 16 : 32);
+  S->nnc = (npad + most - 1) / most;
   S->nc = ((npad + S->nnc - 1) / S->nnc + 15) / 16 * 16;
 }
 
@@ -486,7 +572,6 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   a.npts = npts;
   a.nlines = nlines;
   a.plain = S.plain;
-  a.rebuild = S.nch > 1;
   a.kc = S.kc;
   a.nnc = S.nnc;
   a.nc = S.nc;
@@ -494,17 +579,23 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   a.sb = trans ? S.n : 1;
   a.scale = kSliceUnit - kSliceGuard - S.tau - 1075;
   a.block_bytes = (uint32_t)S.block_bytes();
-  a.slice_b = (uint32_t)(S.nc * S.kc * 2);
-  const uint32_t abytes = (uint32_t)(kSliceN * kLines * S.kc * 2);
-  a.off_b = abytes;
-  // with several K chunks the digit images are rebuilt for every N chunk, so
-  // the transpose buffer may take their place
-  a.off_t = S.nch > 1 ? 0u : abytes + a.block_bytes;
-  const size_t smem = abytes + a.block_bytes + (S.nch > 1 ? 0 : kTransBytes);
+  const bool chunks = S.nch > 1;
+  a.off_b = (uint32_t)(kSliceN * kLines * S.kc * 2);
+  const size_t images = a.off_b + (size_t)(chunks ? 1 : 2) * a.block_bytes;
+  // with K chunks the digits are made again for every N chunk: the transpose
+  // buffer may take their place
+  a.tc = chunks || images + kTransMost <= (size_t)kSmemMost ? 4 : 2;
+  a.off_t = chunks ? 0u : (uint32_t)images;
+  const size_t smem = images + (chunks ? 0 : (size_t)(kST / 32) * 32 * (a.tc + 1) * 8);
   a.tmem_cols = 32;
   while (a.tmem_cols < (uint32_t)(kSliceAcc * S.nc)) a.tmem_cols <<= 1;
-  const long tiles = (a.nlines + kLines - 1) / kLines;
-  // few tiles: the N chunks of a tile go to CTAs of their own
+  if (!chunks) a.tmem_cols <<= 1;  // two sets
+  // Few lines: fewer per CTA (the digits and the read-out are shared among
+  // more SMs; the products cost the same), then the N chunks of a tile to CTAs
+  // of their own.
+  a.lc = kLines;
+  while (a.lc > 32 && (nlines + a.lc / 2 - 1) / (a.lc / 2) <= 152) a.lc /= 2;
+  const long tiles = (nlines + a.lc - 1) / a.lc;
   const int split = tiles * S.nnc <= 152 ? S.nnc : 1;
   a.nc_per = (S.nnc + split - 1) / split;
   const dim3 grid((unsigned)tiles, (unsigned)split);
@@ -517,9 +608,10 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
     a.mode = h0 == 0 || mode == 3 ? mode : 1;
     a.out0 = (long)launches * split * nlines;
     cudaError_t e;
-    if (S.kc <= 32) e = launch_slice<1>(a, grid, smem, S.img, A64, v, x, y, err, st);
-    else if (S.kc <= 64) e = launch_slice<2>(a, grid, smem, S.img, A64, v, x, y, err, st);
-    else e = launch_slice<3>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    if (chunks) e = launch_slice<3, true>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    else if (S.kc <= 32) e = launch_slice<1, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    else if (S.kc <= 64) e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    else e = launch_slice<3, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
     PG_CUDA_TRY(e);
     PG_TRY(check_launch("k_slice_axis"));
   }
