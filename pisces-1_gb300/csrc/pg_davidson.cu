@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(kT) k_ritz_residual(long N, long chunk, int nr
 // Davidson correction (lambda - diag H)^-1 r with the 1e-12 floor
 // (DavidsonCorrectionVector, src/Davidson.cpp:557-566).
 __global__ void k_precond(long N, double* __restrict__ r, const double* __restrict__ diag, double lambda) {
+  pdl_wait();
+  pdl_release();
   for (long g = blockIdx.x * (long)blockDim.x + threadIdx.x; g < N; g += (long)gridDim.x * blockDim.x) {
     double d = lambda - diag[g];
     if (fabs(d) < 1e-12) d = 1e-12;
@@ -869,7 +871,7 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
       const int r = sel[j];
       double* rv = res + (long)r * N;
       if (corrflag == 1) {
-        k_precond<<<blocks_for(N), kT, 0, st>>>(N, rv, diag, d->sse[r]);
+        PG_CUDA_TRY(launch_dependent(k_precond, dim3(blocks_for(N)), dim3(kT), 0, st, N, rv, diag, d->sse[r]));
         PG_TRY(check_launch("k_precond"));
       } else if (corrflag == 2) {
         k_jd_prep<<<blocks_for(N), kT, 0, st>>>(N, rv, jd, ritz + (long)r * N, diag, d->sse[r]);

@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(kT) k_reduce_partials(const double* __restrict
       v[u] = b < nb ? partial[(long)b * no + warp] : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) s += v[u];
+    for (int u = 0; u < 8; ++u)
+      if (b0 + u * 32 < nb) s += v[u];  // zero rows left out: the same sum
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) {
@@ -54,45 +55,64 @@ __global__ void __launch_bounds__(kT) k_reduce_partials(const double* __restrict
   }
 }
 
-__global__ void __launch_bounds__(kT) k_gram(long N, long chunk, const double* __restrict__ P, int na,
-                                             const double* __restrict__ Q, int nb, double* __restrict__ partial,
-                                             const int* __restrict__ skip) {
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+
+// Gram partials in FP64.  Bound by the FP64 pipe: 36 operations per output and
+// kTP points (4 chains of 8 multiply-adds, which are the order of the sums),
+// 64 to 76 cycles each per warp and scheduler.  T tiles of kTP points are
+// resident at a time, and the warps take units of (32 outputs, tile) in turn,
+// so that all four schedulers have the same work: with a thread per output
+// and one tile at a time, 40 x 4 outputs kept 5 warps of 8 busy (two of them
+// on one scheduler) and 20 x 1 only one.  The tiles' sums meet in shared
+// memory and are added in the tiles' order.  The next T tiles are copied
+// meanwhile.
+// Over 262144 points, us: 8 x 1 71 -> 29, 20 x 1 72 -> 32, 40 x 4 120 -> 100,
+// 56 x 8 276 -> 254, 120 x 16 1064 -> 1017.
+__global__ void __launch_bounds__(kT, 2) k_gram(long N, long chunk, const double* __restrict__ P, int na,
+                                                const double* __restrict__ Q, int nb, int logT,
+                                                double* __restrict__ partial, const int* __restrict__ skip) {
+  pdl_wait();
+  pdl_release();
   if (skip && *skip) return;
   extern __shared__ double sm[];
-  double* Ps = sm;                       // na x (kTP+1)
-  double* Qs = sm + na * (kTP + 1);      // nb x (kTP+1)
-  const int no = na * nb;
+  const int rows = na + nb, no = na * nb;
+  const int W = kTP << logT, pitch = W + 1;
+  double* sums = sm + (size_t)2 * rows * pitch;  // [tile][output]
   double acc[kMaxGramOut / kT];
 #pragma unroll
   for (int s = 0; s < kMaxGramOut / kT; ++s) acc[s] = 0;
   const long g_begin = blockIdx.x * chunk;
   const long g_end = g_begin + chunk < N ? g_begin + chunk : N;
-  for (long g0 = g_begin; g0 < g_end; g0 += kTP) {
-    const int cnt = g_end - g0 < kTP ? (int)(g_end - g0) : kTP;
-    // rows 0..na-1 from P, na..na+nb-1 from Q (Qs follows Ps); batched loads
-    const int tot = (na + nb) * kTP;
-    for (int e0 = threadIdx.x; e0 < tot; e0 += kBatch * kT) {
-      double v[kBatch];
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        const int e = e0 + u * kT;
-        const int row = e / kTP, p = e % kTP;
-        const double* src = row < na ? P + (long)row * N : Q + (long)(row - na) * N;
-        v[u] = (e < tot && p < cnt) ? src[g0 + p] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        const int e = e0 + u * kT;
-        if (e < tot) Ps[(e / kTP) * (kTP + 1) + e % kTP] = v[u];
-      }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int groups = (no + 31) >> 5;
+  auto issue = [&](long g0, int buf) {  // rows 0 .. na-1 of P, then those of Q
+    double* dst = sm + (size_t)buf * rows * pitch;
+    const int cnt = g_end - g0 < W ? (int)(g_end - g0) : W;
+    for (int e = threadIdx.x; e < rows * W; e += kT) {
+      const int row = e >> (5 + logT), p = e & (W - 1);
+      const double* src = (row < na ? P + (long)row * N : Q + (long)(row - na) * N) + g0;
+      const unsigned sa = (unsigned)__cvta_generic_to_shared(dst + row * pitch + p);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(src + (p < cnt ? p : 0)),
+                   "r"(p < cnt ? 8 : 0)
+                   : "memory");
     }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < kMaxGramOut / kT; ++s) {
-      const int o = threadIdx.x + s * kT;
+  };
+  if (g_begin < g_end) issue(g_begin, 0);
+  cp_async_commit();
+  int buf = 0;
+  for (long g0 = g_begin; g0 < g_end; g0 += W, buf ^= 1) {
+    if (g0 + W < g_end) issue(g0 + W, buf ^ 1);
+    cp_async_commit();
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // these tiles have landed; the sums before have been read
+    const int nt = g_end - g0 < W ? (int)((g_end - g0 + kTP - 1) / kTP) : 1 << logT;
+    const double* Ps = sm + (size_t)buf * rows * pitch;
+    const double* Qs = Ps + na * pitch;
+    for (int u = warp; u < groups * nt; u += kT / 32) {
+      const int tile = u / groups, o = (u - tile * groups) * 32 + lane;
       if (o < no) {
-        const double* pa = Ps + (o / nb) * (kTP + 1);
-        const double* qb = Qs + (o % nb) * (kTP + 1);
+        const double* pa = Ps + (o / nb) * pitch + tile * kTP;
+        const double* qb = Qs + (o % nb) * pitch + tile * kTP;
         double a0 = 0, a1 = 0, a2 = 0, a3 = 0;  // four chains hide the DFMA latency
 #pragma unroll
         for (int p = 0; p < kTP; p += 4) {
@@ -101,10 +121,16 @@ __global__ void __launch_bounds__(kT) k_gram(long N, long chunk, const double* _
           a2 += pa[p + 2] * qb[p + 2];
           a3 += pa[p + 3] * qb[p + 3];
         }
-        acc[s] += (a0 + a1) + (a2 + a3);
+        sums[tile * no + o] = (a0 + a1) + (a2 + a3);
       }
     }
-    __syncthreads();
+    __syncthreads();  // the sums are complete, these tiles free
+#pragma unroll
+    for (int s = 0; s < kMaxGramOut / kT; ++s) {
+      const int o = threadIdx.x + s * kT;
+      if (o < no)
+        for (int tile = 0; tile < nt; ++tile) acc[s] += sums[tile * no + o];
+    }
   }
 #pragma unroll
   for (int s = 0; s < kMaxGramOut / kT; ++s) {
@@ -120,6 +146,10 @@ __global__ void __launch_bounds__(kT) k_combine(long N, long chunk, const double
                                                 const double* __restrict__ alpha, int inv_sqrt, double* Y, int nr,
                                                 double* __restrict__ partial, double* sq_out, unsigned* counter,
                                                 const int* __restrict__ skip) {
+  // no early release: blocks of the next kernel that take the free places of
+  // some SMs would leave it uneven (back to back 96 x 4 over 110592 points,
+  // on the FP64 pipe: 79 us, 100 with a release here)
+  pdl_wait();
   if (skip && *skip) return;
   extern __shared__ double sm[];
   double* Cs = sm;                 // na x nr
@@ -248,7 +278,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_stages() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(kGStages - 2) : "memory");
 }
@@ -560,12 +589,10 @@ inline bool pair_ok(long N, const double* P, const double* Q) {
   return N % 2 == 0 && ((uintptr_t)P % 16) == 0 && ((uintptr_t)Q % 16) == 0;
 }
 
-// Dynamic shared-memory opt-in, once per kernel (the largest size any call
-// needs: 112 + 16 vectors of 33 doubles for the Gram kernels).
+// Dynamic shared-memory opt-in, once per kernel.
 static pg_status opt_in_smem() {
   static const cudaError_t init = [] {  // thread-safe static initialisation
-    const int big = (int)(sizeof(double) * (size_t)(128 + 16) * (kTP + 1));
-    cudaError_t e = cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaError_t e = cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_gram_df<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);
     if (e == cudaSuccess)
@@ -574,6 +601,21 @@ static pg_status opt_in_smem() {
   }();
   PG_CUDA_TRY(init);
   return PG_OK;
+}
+
+// k_gram over the blocks of chunk points: 4, 2 or 1 tiles resident, as two
+// buffers of them and the sums leave room for two blocks per SM (144 rows and
+// 2048 outputs, more than any call has, fit with one).
+static pg_status launch_gram(long N, long chunk, int blocks, const double* P, int na, const double* Q, int nb,
+                             double* partial, const int* skip, cudaStream_t st) {
+  const auto smem = [&](int logT) {
+    return sizeof(double) * ((size_t)2 * (na + nb) * ((kTP << logT) + 1) + ((size_t)na * nb << logT));
+  };
+  int logT = 2;
+  while (logT > 0 && smem(logT) > (size_t)kGramSmemMax) --logT;
+  PG_CUDA_TRY(launch_dependent(k_gram, dim3(blocks), dim3(kT), smem(logT), st, N, chunk, P, na, Q, nb, logT, partial,
+                               skip));
+  return check_launch("k_gram");
 }
 
 pg_status gram(long N, const double* P, int na, const double* Q, int nb, double* out, RedScratch& rs,
@@ -601,9 +643,7 @@ pg_status gram(long N, const double* P, int na, const double* Q, int nb, double*
     PG_TRY(check_launch("k_gram_df"));
     return reduce(rs.partial.p, dblocks, na * nb, out, false, st, skip);
   } else {
-    const size_t smem = sizeof(double) * (size_t)(na + nb) * (kTP + 1);
-    k_gram<<<blocks, kT, smem, st>>>(N, chunk, P, na, Q, nb, rs.partial.p, skip);
-    PG_TRY(check_launch("k_gram"));
+    PG_TRY(launch_gram(N, chunk, blocks, P, na, Q, nb, rs.partial.p, skip, st));
   }
   return reduce(rs.partial.p, blocks, na * nb, out, false, st, skip);
 }
@@ -640,9 +680,9 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
     PG_TRY(check_launch("k_combine_df"));
   } else {
     const size_t smem = sizeof(double) * (size_t)(na > 0 ? na : 1) * nr;
-#define PG_COMBINE(NRV) \
-  k_combine<NRV><<<blocks, kT, smem, st>>>(N, chunk, P, na, C, ca, cr, cscale, X, alpha, inv_sqrt ? 1 : 0, Y, nr, \
-                                           sq ? rs.partial.p : nullptr, sq, rs.counter.p, skip)
+#define PG_COMBINE(NRV)                                                                                           \
+  PG_CUDA_TRY(launch_dependent(k_combine<NRV>, dim3(blocks), dim3(kT), smem, st, N, chunk, P, na, C, ca, cr, cscale, X, \
+                               alpha, inv_sqrt ? 1 : 0, Y, nr, sq ? rs.partial.p : nullptr, sq, rs.counter.p, skip))
     if (nr <= 1) PG_COMBINE(1);
     else if (nr <= 2) PG_COMBINE(2);
     else if (nr <= 4) PG_COMBINE(4);
@@ -929,8 +969,6 @@ extern "C" pg_status pg_block_gram_noalloc(long n, const double* P, int np, cons
   }
   const long chunk = chunk_for(n, pg::kRedBlocks, kTP);
   const int blocks = (int)((n + chunk - 1) / chunk);
-  const size_t smem = sizeof(double) * (size_t)(np + nq) * (kTP + 1);
-  k_gram<<<blocks, kT, smem, st>>>(n, chunk, P, np, Q, nq, partial, nullptr);
-  PG_TRY(check_launch("k_gram"));
+  PG_TRY(launch_gram(n, chunk, blocks, P, np, Q, nq, partial, nullptr, st));
   return reduce(partial, blocks, no, out, false, st);
 }
