@@ -258,6 +258,119 @@ __device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al,
   sh = t;
 }
 
+// Two FP32 numbers in one register pair, for the packed FP32 instructions: the
+// same roundings at the same rate, but half the issue slots, which leaves
+// slots for the integer work beside them.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 d, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(d));
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// a - b (b times -1 is exact, so one rounding)
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) { return f2_fma(b, 0xbf800000bf800000ull, a); }
+
+// df_fma for two sums at once: the one value a = (ah, al), given as the pairs
+// (ah, ah), (-ah, -ah) and (-al, -al), times two coefficients.  The error of
+// the product is kept negated; the roundings are df_fma's.
+__device__ __forceinline__ void df_fma2(f32x2& sh, f32x2& sl, f32x2 ah, f32x2 nah, f32x2 nal, f32x2 bh, f32x2 bl) {
+  const f32x2 p = f2_mul(ah, bh);
+  f32x2 e = f2_fma(nah, bh, p);
+  e = f2_fma(nah, bl, e);
+  e = f2_fma(nal, bh, e);
+  const f32x2 t = f2_add(sh, p);
+  const f32x2 bp = f2_sub(t, sh);
+  const f32x2 err = f2_add(f2_sub(sh, f2_sub(t, bp)), f2_sub(p, bp));
+  sl = f2_add(sl, f2_sub(err, e));
+  sh = t;
+}
+
+// FP32 -> FP64 with integer operations (exact for normal numbers and zero;
+// FP32 subnormals flush to a signed zero; Inf and NaN are kept): keeps the
+// conversion off the FP64 pipe, which retires about two operations per SM
+// per clock on this part.
+__device__ __forceinline__ double f32_to_f64_int(float v) {
+  const uint32_t u = __float_as_uint(v);
+  const uint32_t sign = u & 0x80000000u, e = (u >> 23) & 0xffu, mt = u & 0x7fffffu;
+  uint32_t hi = sign | ((e + 896u) << 20) | (mt >> 3);
+  uint32_t lo = mt << 29;
+  hi = e == 0 ? sign : hi;
+  lo = e == 0 ? 0u : lo;
+  hi = e == 255 ? (sign | 0x7ff00000u | (mt >> 3) | (mt ? 0x80000u : 0u)) : hi;
+  lo = e == 255 ? 0u : lo;
+  return __hiloint2double((int)hi, (int)lo);
+}
+
+// (double)h + (double)l rounded to nearest, with FP32 and integer operations:
+// an FP64 conversion or addition costs 64 to 76 cycles a warp and scheduler
+// here.  s = h + l in FP32 and its error e (two-sum, exact); then e, in units
+// of the result's last place, is rounded to an integer and added to s's bits.
+// Not for sums outside [2^-75, 2^127], or where the addition crosses below a
+// power of two (its last place is then half as large): by FP64, as the caller
+// asks for FP32 subnormals (kFlush: zero, as f32_to_f64_int).
+template <bool kFlush>
+__device__ __noinline__ double df_join_slow(float h, float l) {
+  if (kFlush) return f32_to_f64_int(h) + f32_to_f64_int(l);
+  return (double)h + (double)l;
+}
+template <bool kFlush>
+__device__ __forceinline__ double df_join(float h, float l) {
+  const float s = h + l;
+  const float bp = s - h;
+  const float e = (h - (s - bp)) + (l - bp);
+  const uint32_t u = __float_as_uint(s);
+  const uint32_t ex = u & 0x7f800000u;
+  // e / 2^(exponent of s - 52), with the sign of s: at most 2^28 in magnitude
+  const float v = e * __uint_as_float((0x99000000u - ex) ^ (u & 0x80000000u));
+  if (ex - (52u << 23) > (202u << 23) || ((u & 0x7fffffu) == 0 && v < 0.f)) return df_join_slow<kFlush>(h, l);
+  const long long r = (long long)(((unsigned long long)((u & 0x7fffffffu) >> 3) + (896ull << 20)) << 32 | (u << 29)) +
+                      __float2int_rn(v);
+  return __longlong_as_double(r | (long long)((unsigned long long)(u & 0x80000000u) << 32));
+}
+
+// Sums K values (a power of two) over the lanes as steps of 16, 8, .. to kLast
+// of v[lane] + v[lane + step] would, several values to a register as lanes
+// become free: value k ends in lane k (32 / K) for K <= 32 / kLast, else value
+// k in v[k % (K kLast / 32)] of lane kLast (k / (K kLast / 32)).
+template <int K, int kLast, typename T>
+__device__ __forceinline__ void packed_sums(T (&v)[K], int lane) {
+  int n = K;
+#pragma unroll
+  for (int o = 16; o >= kLast; o >>= 1) {
+    if (n > 1) {
+#pragma unroll
+      for (int i = 0; i < K / 2; ++i) {
+        if (i < n / 2) {
+          const bool up = lane & o;
+          const T keep = up ? v[i + n / 2] : v[i], send = up ? v[i] : v[i + n / 2];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      n >>= 1;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+}
+
 // Gram partials in double-float, written as double (hi + lo): same contract
 // as k_gram.  A thread owns a kGA x kGB block of outputs (kGA rows of P
 // against kGB rows of Q) for one slice of the points of each tile, so every
@@ -267,6 +380,11 @@ __device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al,
 // in place once they land), keeping two tiles in flight behind the one being
 // multiplied.  At the end the slices of each output block are summed in a
 // fixed order.
+// Bound by the FP32 pipe in the multiply loop (12 operations per output and
+// point) and by the issue slots of copies and conversions beside it.  Those
+// had a warp to a row (36 point pairs: two rounds for 36 of 64 lanes), and the
+// ends 48 FP64 operations a thread; without them, us over 884736 points: 16 x 4
+// 83 -> 74, 40 x 4 188 -> 147, 56 x 8 404 -> 293, 96 x 4 563 -> 347.
 constexpr int kGA = 4, kGB = 4, kGStages = 3;
 constexpr int kGramSmemMax = 112 * 1024;
 
@@ -326,7 +444,6 @@ __global__ void __launch_bounds__(kT, 2) k_gram_df(long N, long chunk, const dou
   const long g_end = g_begin + chunk < N ? g_begin + chunk : N;
   const int ntiles = g_end > g_begin ? (int)((g_end - g_begin + tp - 1) / tp) : 0;
   const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
   const int blk = tid / S, slice = tid - blk * S;
   const bool active = blk < nblk;
   const int a0 = (blk % ablk) * kGA, b0 = (blk / ablk) * kGB;
@@ -341,33 +458,42 @@ __global__ void __launch_bounds__(kT, 2) k_gram_df(long N, long chunk, const dou
 #pragma unroll
     for (int j = 0; j < kGB; ++j) sh[i][j] = sl[i][j] = 0.f;
 
-  // staging: warp w copies rows w, w + 8, ...; its lanes stride over the row
+  // staging: the threads take the tile's point pairs (points) row by row, kT
+  // at a time, so that no lane idles where a row's are not a multiple of 32;
+  // addresses count up
+  const int per = kPair ? hp : tp, total = rows * per;
+  constexpr int kStep = kPair ? 2 : 1;
+  const int row0 = tid / per, q0 = tid - row0 * per, drow = kT / per, dq = kT - drow * per;
+  const long jump = (long)drow * N + kStep * dq, wrap = N - (long)kStep * per;
+  const double* first = (row0 < na ? P + (long)row0 * N : Q + (long)(row0 - na) * N) + g_begin + kStep * q0;
+  const long to_q = Q - (P + (long)na * N);  // from where row na of P would be to row 0 of Q
   auto issue = [&](int tile) {
-    double* dst = stage0 + (size_t)(tile % kGStages) * stage_elems;
-    const long g0 = g_begin + (long)tile * tp;
-    const int cnt = g_end - g0 < tp ? (int)(g_end - g0) : tp;
-    for (int row = warp; row < rows; row += kT / 32) {
-      const double* src = (row < na ? P + (long)row * N : Q + (long)(row - na) * N) + g0;
-      double* d = dst + (size_t)row * tp;
+    double* d = stage0 + (size_t)(tile % kGStages) * stage_elems + kStep * tid;
+    const long g0 = (long)tile * tp;
+    const int cnt = g_end - g_begin - g0 < tp ? (int)(g_end - g_begin - g0) : tp;
+    const double* src = first + g0;
+    int row = row0, p = kStep * q0;
+    for (int e = tid; e < total; e += kT, d += kStep * kT) {
       if (kPair) {
-        for (int q = lane; q < hp; q += 32) {
-          const int p = 2 * q;
-          if (p + 1 < cnt) {
-            cp_async16(d + p, src + p);
-          } else if (p < cnt) {
-            cp_async8(d + p, src + p);
-            d[p + 1] = 0.0;
-          } else {
-            d[p] = 0.0;
-            d[p + 1] = 0.0;
-          }
+        if (p + 1 < cnt) {
+          cp_async16(d, src);
+        } else if (p < cnt) {
+          cp_async8(d, src);
+          d[1] = 0.0;
+        } else {
+          d[0] = 0.0;
+          d[1] = 0.0;
         }
       } else {
-        for (int p = lane; p < tp; p += 32) {
-          if (p < cnt) cp_async8(d + p, src + p);
-          else d[p] = 0.0;
-        }
+        if (p < cnt) cp_async8(d, src);
+        else d[0] = 0.0;
       }
+      const bool in_p = row < na;
+      row += drow;
+      p += kStep * dq;
+      src += jump;
+      if (p >= kStep * per) p -= kStep * per, src += wrap, ++row;
+      if (in_p && row >= na) src += to_q;
     }
   };
   for (int t = 0; t < kGStages - 1; ++t) {
@@ -378,23 +504,21 @@ __global__ void __launch_bounds__(kT, 2) k_gram_df(long N, long chunk, const dou
     cp_async_wait_stages();  // this thread's copies of tile `it` have landed
     double* cur = stage0 + (size_t)(it % kGStages) * stage_elems;
     // convert the points this thread copied, in place, to (hi, lo) pairs
-    for (int row = warp; row < rows; row += kT / 32) {
-      if (row < na ? split_p : split_q) continue;  // a twin row: already (hi, lo)
-      double* d = cur + (size_t)row * tp;
+    // (a twin's rows already are)
+    const int conv0 = split_p ? na * per : 0, conv1 = split_q ? na * per : total;
+    for (int e = tid; e < conv1; e += kT) {
+      if (e < conv0) continue;
+      double* d = cur + (size_t)kStep * e;
       if (kPair) {
-        for (int q = lane; q < hp; q += 32) {
-          const double2 d2 = *reinterpret_cast<const double2*>(d + 2 * q);
-          float h0, l0, h1, l1;
-          df_split(d2.x, h0, l0);
-          df_split(d2.y, h1, l1);
-          *reinterpret_cast<float4*>(d + 2 * q) = make_float4(h0, l0, h1, l1);
-        }
+        const double2 d2 = *reinterpret_cast<const double2*>(d);
+        float h0, l0, h1, l1;
+        df_split(d2.x, h0, l0);
+        df_split(d2.y, h1, l1);
+        *reinterpret_cast<float4*>(d) = make_float4(h0, l0, h1, l1);
       } else {
-        for (int p = lane; p < tp; p += 32) {
-          float h, l;
-          df_split(d[p], h, l);
-          *reinterpret_cast<float2*>(d + p) = make_float2(h, l);
-        }
+        float h, l;
+        df_split(d[0], h, l);
+        *reinterpret_cast<float2*>(d) = make_float2(h, l);
       }
     }
     __syncthreads();  // tile `it` converted; everyone is done with tile it-1
@@ -430,7 +554,7 @@ __global__ void __launch_bounds__(kT, 2) k_gram_df(long N, long chunk, const dou
     for (int i = 0; i < kGA; ++i)
 #pragma unroll
       for (int j = 0; j < kGB; ++j)
-        red[((size_t)slice * nblk + blk) * (kGA * kGB) + i * kGB + j] = (double)sh[i][j] + (double)sl[i][j];
+        red[((size_t)slice * nblk + blk) * (kGA * kGB) + i * kGB + j] = df_join<false>(sh[i][j], sl[i][j]);
   }
   __syncthreads();
   const int no = na * nb;
@@ -444,33 +568,90 @@ __global__ void __launch_bounds__(kT, 2) k_gram_df(long N, long chunk, const dou
   }
 }
 
+// The coefficients of up to NR outputs as double-float: [row][pair of outputs]
+// (hi, hi, lo, lo), zero past nr; for one output [row] (hi, lo).
+template <int NR, typename Get>
+__device__ __forceinline__ void load_coefs(float* Cs, int na, int nr, const Get& get) {
+  for (int e = threadIdx.x; e < na * NR; e += kT) {
+    const int a = e / NR, r = e % NR;
+    float h = 0.f, l = 0.f;
+    if (r < nr) df_split(get(a, r), h, l);
+    float* c = NR == 1 ? Cs + 2 * a : Cs + 4 * (a * (NR / 2) + r / 2) + r % 2;
+    c[0] = h;
+    c[NR == 1 ? 1 : 2] = l;
+  }
+}
+template <int NR>
+constexpr size_t coef_bytes(int na) { return sizeof(float) * 2 * (size_t)(na > 0 ? na : 1) * NR; }
+
+// NR double-float sums of one point, two to a register pair.
+template <int NR>
+struct DfSums {
+  f32x2 h[NR / 2], l[NR / 2];
+  __device__ __forceinline__ DfSums(const float (&sh)[NR], const float (&sl)[NR]) {
+#pragma unroll
+    for (int j = 0; j < NR / 2; ++j) h[j] = f2_pack(sh[2 * j], sh[2 * j + 1]), l[j] = f2_pack(sl[2 * j], sl[2 * j + 1]);
+  }
+  // += (ph, pl) times row a of the coefficients
+  __device__ __forceinline__ void add(float ph, float pl, const float* Cs, int a) {
+    const f32x2 ah = f2_pack(ph, ph), nah = f2_pack(-ph, -ph), nal = f2_pack(-pl, -pl);
+    const ulonglong2* c = reinterpret_cast<const ulonglong2*>(Cs) + a * (NR / 2);
+#pragma unroll
+    for (int j = 0; j < NR / 2; ++j) {
+      const ulonglong2 b = c[j];
+      df_fma2(h[j], l[j], ah, nah, nal, b.x, b.y);
+    }
+  }
+  __device__ __forceinline__ void get(float (&sh)[NR], float (&sl)[NR]) const {
+#pragma unroll
+    for (int j = 0; j < NR / 2; ++j) {
+      f2_unpack(h[j], sh[2 * j], sh[2 * j + 1]);
+      f2_unpack(l[j], sl[2 * j], sl[2 * j + 1]);
+    }
+  }
+};
+template <>
+struct DfSums<1> {
+  float h, l;
+  __device__ __forceinline__ DfSums(const float (&sh)[1], const float (&sl)[1]) : h(sh[0]), l(sl[0]) {}
+  __device__ __forceinline__ void add(float ph, float pl, const float* Cs, int a) {
+    const float2 c = reinterpret_cast<const float2*>(Cs)[a];
+    df_fma(h, l, ph, pl, c.x, c.y);
+  }
+  __device__ __forceinline__ void get(float (&sh)[1], float (&sl)[1]) const { sh[0] = h, sl[0] = l; }
+};
+
 // Combine in double-float: same contract as k_combine (coefficients and
 // alpha are FP64 and split once per block; Y is written as double).
 // kTwinIn: the rows of P are double-float twins (float2 (hi, lo) per point)
 // and are read without converting; kTwinOut: each output is also written as
 // its twin to Yt.  Compile-time flags: a runtime choice inside the unrolled
-// loop doubles the registers of the kernel and halves its occupancy.  Up to 4
-// outputs the kernel fits 64 registers (4 blocks per SM, no spills).
+// loop doubles the registers of the kernel and halves its occupancy.
+// Bound by the FP32 pipe: 12 operations per output and row, two outputs to an
+// instruction, whose coefficients are one 16-byte read; the pairs become FP64
+// without the FP64 pipe, and the norms' FP64 sums over the lanes share
+// instructions.  With a read and a branch per coefficient, and conversions
+// and every sum in FP64, us over 884736 points: 40 x 4 132 -> 107, 56 x 8
+// 371 -> 234, 12 x 12 173 -> 117, 120 x 16 1370 -> 898; 40 x 1 74 -> 66 (rows
+// read ahead).
 template <int NR, bool kTwinIn, bool kTwinOut>
 __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long chunk, const double* P, int na,
                                                    const double* __restrict__ C, int ca, int cr, double cscale,
                                                    const double* X, const double* __restrict__ alpha, int inv_sqrt,
                                                    double* Y, int nr, float2* Yt, double* __restrict__ partial,
                                                    double* sq_out, unsigned* counter, const int* __restrict__ skip) {
+  // the next kBatch rows are on their way while these are multiplied; not with
+  // 4 outputs, where four blocks per SM (64 registers) are worth more (16 x 4
+  // over 884736 points: 48 us, 56 with three blocks and the rows ahead)
+  constexpr bool kAhead = NR != 4;
   pdl_wait();
   pdl_release();
   if (skip && *skip) return;
-  extern __shared__ float smf[];
-  float* Ch = smf;              // na x nr
-  float* Cl = smf + na * nr;
+  extern __shared__ __align__(16) float smf[];
+  float* Cs = smf;  // [row][pair]: (hi, hi, lo, lo); NR 1: [row] (hi, lo)
   __shared__ float alh[NR], all[NR];
   __shared__ double red[kT / 32][NR];
-  for (int e = threadIdx.x; e < na * nr; e += kT) {
-    float h, l;
-    df_split(cscale * C[(long)(e / nr) * ca + (long)(e % nr) * cr], h, l);
-    Ch[e] = h;
-    Cl[e] = l;
-  }
+  load_coefs<NR>(Cs, na, nr, [&](int a, int r) { return cscale * C[(long)a * ca + (long)r * cr]; });
   if (threadIdx.x < nr) {
     double a = 0;
     if (alpha) a = inv_sqrt ? 1.0 / sqrt(alpha[threadIdx.x]) : alpha[threadIdx.x];
@@ -498,10 +679,16 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long
         df_fma(sh[r], sl[r], alh[r], all[r], xh, xl);
       }
     }
-    for (int a0 = 0; a0 < na; a0 += kBatch) {
-      double pv[kBatch];
+    DfSums<NR> sum(sh, sl);
+    const double* row = P + g;
+    double pv[kBatch], nv[kBatch];
+    auto rows = [&](double (&w)[kBatch], int a0) {
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) pv[u] = a0 + u < na ? P[(long)(a0 + u) * N + g] : 0.0;
+      for (int u = 0; u < kBatch; ++u) w[u] = a0 + u < na ? row[(long)(a0 + u) * N] : 0.0;
+    };
+    rows(pv, 0);
+    for (int a0 = 0; a0 < na; a0 += kBatch) {
+      if (kAhead) rows(nv, a0 + kBatch);
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
         if (a0 + u >= na) break;
@@ -512,32 +699,31 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long
         } else {
           df_split(pv[u], ph, pl);
         }
-        const float* ch = Ch + (a0 + u) * nr;
-        const float* cl = Cl + (a0 + u) * nr;
+        sum.add(ph, pl, Cs, a0 + u);
+      }
+      if (kAhead) {
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-          if (r < nr) df_fma(sh[r], sl[r], ph, pl, ch[r], cl[r]);
+        for (int u = 0; u < kBatch; ++u) pv[u] = nv[u];
+      } else {
+        rows(pv, a0 + kBatch);
       }
     }
+    sum.get(sh, sl);
 #pragma unroll
     for (int r = 0; r < NR; ++r)
       if (r < nr) {
-        const double y = (double)sh[r] + (double)sl[r];
+        const double y = df_join<false>(sh[r], sl[r]);
         Y[(long)r * N + g] = y;
         // the accumulator pair is the output in double-float form already
         // (it and y = sh + sl agree to 2^-53 relative)
         if (kTwinOut) Yt[(long)r * N + g] = make_float2(sh[r], sl[r]);
-        sacc[r] += y * y;
+        if (partial) sacc[r] += y * y;
       }
   }
   if (!partial) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    double v = sacc[r];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][r] = v;
-  }
+  packed_sums<NR, 1>(sacc, lane);
+  if (lane % (32 / NR) == 0) red[warp][lane / (32 / NR)] = sacc[0];
   __syncthreads();
   if (threadIdx.x < nr) {
     double s = 0;
@@ -658,9 +844,8 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
   const long chunk = chunk_for(N, kStreamBlocks, kT);
   const int blocks = (int)((N + chunk - 1) / chunk);
   if (dfloat) {
-    const size_t smem = sizeof(float) * 2 * (size_t)(na > 0 ? na : 1) * nr;
 #define PG_COMBINE_DF3(NRV, TI, TO)                                                                                \
-  PG_CUDA_TRY(launch_dependent(k_combine_df<NRV, TI, TO>, dim3(blocks), dim3(kT), smem, st, N, chunk, Pt ? Pt : P, na, \
+  PG_CUDA_TRY(launch_dependent(k_combine_df<NRV, TI, TO>, dim3(blocks), dim3(kT), coef_bytes<NRV>(na), st, N, chunk, Pt ? Pt : P, na, \
                                C, ca, cr, cscale, X, alpha, inv_sqrt ? 1 : 0, Y, nr, reinterpret_cast<float2*>(Yt),  \
                                sq ? rs.partial.p : nullptr, sq, rs.counter.p, skip))
 #define PG_COMBINE_DF(NRV)                                             \
@@ -694,47 +879,32 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
   return PG_OK;  // with sq, the kernel's last block has reduced the norms
 }
 
-// FP32 -> FP64 with integer operations (exact for normal numbers and zero;
-// FP32 subnormals flush to a signed zero; Inf and NaN are kept): keeps the
-// conversion off the FP64 pipe, which retires about two operations per SM
-// per clock on this part.
-__device__ __forceinline__ double f32_to_f64_int(float v) {
-  const uint32_t u = __float_as_uint(v);
-  const uint32_t sign = u & 0x80000000u, e = (u >> 23) & 0xffu, mt = u & 0x7fffffu;
-  uint32_t hi = sign | ((e + 896u) << 20) | (mt >> 3);
-  uint32_t lo = mt << 29;
-  hi = e == 0 ? sign : hi;
-  lo = e == 0 ? 0u : lo;
-  hi = e == 255 ? (sign | 0x7ff00000u | (mt >> 3) | (mt ? 0x80000u : 0u)) : hi;
-  lo = e == 255 ? 0u : lo;
-  return __hiloint2double((int)hi, (int)lo);
-}
-
 // The Ritz step of the mixed form in one pass: U_r = B v_r and
 // W_r = Z v_r - lambda_r U_r in double-float from the twins of the m rows of
 // B and Z (v_r = column r of V, leading dimension ldv), written as FP64, and
 // |U_r|^2, |W_r|^2 (squares summed in FP32 per thread, in FP64 across threads)
-// reduced by the last block into out[r] and out[nr + r].  Two FP64 additions
-// per output and point (the pairs to FP64); the rest runs on the FP32 pipe.
+// reduced by the last block into out[r] and out[nr + r].  On the FP32 pipe (24
+// operations per output, row and point) next to the read of 16 bytes per row
+// and point; the FP64 pipe only adds the norms.  4 roots over 262144 points,
+// 8 / 30 / 60 rows: 27 / 61 / 102 us with FP64 additions per point, a read per
+// coefficient and rows read as they are needed, now 23 / 47 / 80 (64 registers
+// and four blocks per SM: 20 / 47 / 80, but 50 instead of 41 over 110592
+// points and 60 rows, whose blocks all fit with three).
 template <int NR>
 __global__ void __launch_bounds__(kT, NR <= 4 ? 3 : 2) k_ritz_df(long N, long chunk, const double* Bt, const double* Zt,
                                                                int m, const double* __restrict__ V, int ldv,
                                                                const double* __restrict__ lam, double* U, double* W,
                                                                int nr, double* __restrict__ partial, double* out,
                                                                unsigned* counter) {
+  constexpr bool kAhead = NR != 16;  // registers: 16 outputs spill
+  constexpr int kRows = kBatch / 2;
   pdl_wait();
   pdl_release();
-  extern __shared__ float smf[];
-  float* Ch = smf;  // m x nr
-  float* Cl = smf + m * nr;
+  extern __shared__ __align__(16) float smf[];
+  float* Cs = smf;  // as in k_combine_df
   __shared__ float nlh[NR], nll[NR];
   __shared__ double red[kT / 32][2 * NR];
-  for (int e = threadIdx.x; e < m * nr; e += kT) {
-    float h, l;
-    df_split(V[(long)(e / nr) + (long)(e % nr) * ldv], h, l);
-    Ch[e] = h;
-    Cl[e] = l;
-  }
+  load_coefs<NR>(Cs, m, nr, [&](int a, int r) { return V[(long)a + (long)r * ldv]; });
   if (threadIdx.x < nr) {
     float h, l;
     df_split(-lam[threadIdx.x], h, l);
@@ -751,35 +921,44 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 3 : 2) k_ritz_df(long N, long ch
     float uh[NR], ul[NR], zh[NR], zl[NR];
 #pragma unroll
     for (int r = 0; r < NR; ++r) uh[r] = ul[r] = zh[r] = zl[r] = 0.f;
-    for (int a0 = 0; a0 < m; a0 += kBatch / 2) {
-      double pb[kBatch / 2], pz[kBatch / 2];
+    DfSums<NR> su2(uh, ul), sz2(zh, zl);
+    // the next kRows rows of each are on their way while these are multiplied
+    const double *rb = Bt + g, *rz = Zt + g;
+    double pb[kRows], pz[kRows], nb[kRows], nz[kRows];
+    auto rows = [&](double (&b)[kRows], double (&z)[kRows], int a0) {
 #pragma unroll
-      for (int u = 0; u < kBatch / 2; ++u) {
-        pb[u] = a0 + u < m ? Bt[(long)(a0 + u) * N + g] : 0.0;
-        pz[u] = a0 + u < m ? Zt[(long)(a0 + u) * N + g] : 0.0;
+      for (int u = 0; u < kRows; ++u) {
+        b[u] = a0 + u < m ? rb[(long)(a0 + u) * N] : 0.0;
+        z[u] = a0 + u < m ? rz[(long)(a0 + u) * N] : 0.0;
       }
+    };
+    rows(pb, pz, 0);
+    for (int a0 = 0; a0 < m; a0 += kRows) {
+      if (kAhead) rows(nb, nz, a0 + kRows);
 #pragma unroll
-      for (int u = 0; u < kBatch / 2; ++u) {
+      for (int u = 0; u < kRows; ++u) {
         if (a0 + u >= m) break;
         // the 8 bytes are a float2 (hi, lo): hi in the low word
         const float bh = __int_as_float(__double2loint(pb[u])), bl = __int_as_float(__double2hiint(pb[u]));
         const float qh = __int_as_float(__double2loint(pz[u])), ql = __int_as_float(__double2hiint(pz[u]));
-        const float* ch = Ch + (a0 + u) * nr;
-        const float* cl = Cl + (a0 + u) * nr;
+        su2.add(bh, bl, Cs, a0 + u);
+        sz2.add(qh, ql, Cs, a0 + u);
+      }
+      if (kAhead) {
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-          if (r < nr) {
-            df_fma(uh[r], ul[r], bh, bl, ch[r], cl[r]);
-            df_fma(zh[r], zl[r], qh, ql, ch[r], cl[r]);
-          }
+        for (int u = 0; u < kRows; ++u) pb[u] = nb[u], pz[u] = nz[u];
+      } else {
+        rows(pb, pz, a0 + kRows);
       }
     }
+    su2.get(uh, ul);
+    sz2.get(zh, zl);
 #pragma unroll
     for (int r = 0; r < NR; ++r)
       if (r < nr) {
         df_fma(zh[r], zl[r], nlh[r], nll[r], uh[r], ul[r]);  // W = Z v - lambda U
-        const double u = f32_to_f64_int(uh[r]) + f32_to_f64_int(ul[r]);
-        const double w = f32_to_f64_int(zh[r]) + f32_to_f64_int(zl[r]);
+        const double u = df_join<true>(uh[r], ul[r]);
+        const double w = df_join<true>(zh[r], zl[r]);
         U[(long)r * N + g] = u;
         W[(long)r * N + g] = w;
         // the pair's sum in FP32 (after the cancellation in W its low part
@@ -790,22 +969,18 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 3 : 2) k_ritz_df(long N, long ch
       }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // sums of 16 lanes in FP32 (2^-22 relative at most), the last step and
+  // everything after it in FP64: few operations on the FP64 pipe
+  float sq[2 * NR];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    // sums of 16 lanes in FP32 (2^-22 relative at most), the last step and
-    // everything after it in FP64: few operations on the FP64 pipe
-    float af = su[r], bf = sw[r];
-    for (int o = 16; o > 1; o >>= 1) {
-      af += __shfl_down_sync(0xffffffffu, af, o);
-      bf += __shfl_down_sync(0xffffffffu, bf, o);
-    }
-    double a = f32_to_f64_int(af), b = f32_to_f64_int(bf);
-    a += __shfl_down_sync(0xffffffffu, a, 1);
-    b += __shfl_down_sync(0xffffffffu, b, 1);
-    if (lane == 0) {
-      red[warp][r] = a;
-      red[warp][NR + r] = b;
-    }
+  for (int r = 0; r < NR; ++r) sq[r] = su[r], sq[NR + r] = sw[r];
+  packed_sums<2 * NR, 2>(sq, lane);
+  constexpr int kRegs = NR == 16 ? 2 : 1;  // values per lane pair
+#pragma unroll
+  for (int i = 0; i < kRegs; ++i) {
+    double a = f32_to_f64_int(sq[i]);
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    if (lane % (kRegs * 16 / NR) == 0) red[warp][lane * NR / 16 + i] = a;
   }
   __syncthreads();
   if (threadIdx.x < 2 * nr) {
@@ -824,9 +999,8 @@ pg_status ritz_df(long N, const double* Bt, const double* Zt, int m, const doubl
   PG_TRY(rs.ensure(st));
   const long chunk = chunk_for(N, kStreamBlocks, kT);
   const int blocks = (int)((N + chunk - 1) / chunk);
-  const size_t smem = sizeof(float) * 2 * (size_t)m * nr;
 #define PG_RITZ_DF(NRV)                                                                                           \
-  PG_CUDA_TRY(launch_dependent(k_ritz_df<NRV>, dim3(blocks), dim3(kT), smem, st, N, chunk, Bt, Zt, m, V, ldv, lam, U, \
+  PG_CUDA_TRY(launch_dependent(k_ritz_df<NRV>, dim3(blocks), dim3(kT), coef_bytes<NRV>(m), st, N, chunk, Bt, Zt, m, V, ldv, lam, U, \
                                W, nr, rs.partial.p, sq, rs.counter.p))
   if (nr <= 1) PG_RITZ_DF(1);
   else if (nr <= 2) PG_RITZ_DF(2);
