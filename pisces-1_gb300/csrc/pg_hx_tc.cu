@@ -32,6 +32,7 @@ constexpr int kHalfThreads = 256;  // several K chunks: two CTAs per SM
 constexpr int kTileM = 128;
 constexpr int kMaxN = 256;  // n_axis limit: the MMA N extent (rows of the axis matrix, padded to 16)
 constexpr int kBatch = 16;  // global loads a thread keeps in flight while filling A
+constexpr int kHalfBatch = 24;  // with two CTAs per SM: a whole K chunk (at most 48 values) of a warp's two row groups
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -131,7 +132,10 @@ __device__ __forceinline__ void epilogue_x16(const float (&d)[16], float* stg, i
   // and 16 rounds of them do not fit the 128 registers of the launch
 #pragma unroll
   for (int h = 0; h < 16; h += 8) {
-    double prev[8];
+    // the loads first, without an operation between them: with the product
+    // beside its loads each round waited for its own two (160^3 x 16: 1.68 ms
+    // for the three passes, 1.34 so)
+    double prev[8], pot[8];
     float val[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -141,16 +145,16 @@ __device__ __forceinline__ void epilogue_x16(const float (&d)[16], float* stg, i
       const long gs = (long)__shfl_sync(0xffffffffu, (long long)gshift_own, r);
       const long c = c0w + r;
       const long a = (long)nx * c + i;
-      prev[u] = 0.0;
-      if (c < ncols && i < n) {
-        if (mode == 2) prev[u] = v[a - gs] * X[a];
-        else if (mode == 1) prev[u] = Y[a];
-      }
+      const bool in = c < ncols && i < n;
+      prev[u] = in && mode != 0 ? (mode == 2 ? X : Y)[a] : 0.0;
+      pot[u] = in && mode == 2 ? v[a - gs] : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const long c = c0w + 2 * (h + u) + half;
-      if (c < ncols && i < n) Y[(long)nx * c + i] = prev[u] + f32_to_f64_exact(val[u]);
+      const double k = f32_to_f64_exact(val[u]);
+      if (c < ncols && i < n)
+        Y[(long)nx * c + i] = __dadd_rn(mode == 2 ? __dmul_rn(pot[u], prev[u]) : prev[u], k);
     }
   }
   __syncwarp();  // the block is rewritten by the warp's next chunk
@@ -170,7 +174,7 @@ __device__ __forceinline__ long col_base(long c, int nx, int ny, long N) {
   return (c - vv * plane) + N * vv;
 }
 
-// Fill the A operand of one tile: columns c0 .. c0+127 at K values k0 ..
+// Fills the A operand of one tile: columns c0 .. c0+127 at K values k0 ..
 // k0+kc-1, split into TF32 hi/lo halves in the K-major core-matrix layout.
 // Lane L takes row m = 8 g + (L >> 2) and K index 4 q + (L & 3) of core
 // matrix (g, q), so one warp store fills one 8 x 4 core matrix: 128
@@ -180,33 +184,39 @@ __device__ __forceinline__ long col_base(long c, int nx, int ny, long N) {
 // wi of 16 / RG owns the row groups g = wi, wi + 16 / RG, ..., so each lane's
 // column bases are computed once per tile; kBatch loads per thread are in
 // flight before they are split and stored.
-template <int AXIS, int RG>
-__device__ __forceinline__ void fill_a(int wi, int lane, const double* __restrict__ X, long c0, long ncols, int k0,
-                                       int kc, int n, long stride, int nx, int ny, long N, unsigned char* sAh,
-                                       unsigned char* sAl) {
-  static_assert(kBatch % RG == 0, "a load batch covers whole row-group rounds");
-  constexpr int kWarps = (kTileM / 8) / RG;  // warps sharing the fill
-  const int kq = kc >> 2;                    // core matrices along K
+template <int AXIS, int RG, int B>
+struct FillA {
+  static_assert(B % RG == 0, "a load batch covers whole row-group rounds");
+  static constexpr int kWarps = (kTileM / 8) / RG;  // warps sharing the fill
   long base[RG];
   bool cv[RG];
+  const double* __restrict__ X;
+  int wi, lane;
+  __device__ __forceinline__ FillA(int wi_, int lane_, const double* __restrict__ X_, long c0, long ncols, int nx,
+                                   int ny, long N)
+      : X(X_), wi(wi_), lane(lane_) {
 #pragma unroll
-  for (int r = 0; r < RG; ++r) {
-    const long c = c0 + 8 * (wi + r * kWarps) + (lane >> 2);
-    cv[r] = c < ncols;
-    base[r] = cv[r] ? (AXIS == 0 ? (long)nx * c : col_base<AXIS>(c, nx, ny, N)) : 0;
+    for (int r = 0; r < RG; ++r) {
+      const long c = c0 + 8 * (wi + r * kWarps) + (lane >> 2);
+      cv[r] = c < ncols;
+      base[r] = cv[r] ? (AXIS == 0 ? (long)nx * c : col_base<AXIS>(c, nx, ny, N)) : 0;
+    }
   }
-  const int kl = lane & 3;
-  for (int t0 = 0; t0 < RG * kq; t0 += kBatch) {
-    const int q0 = t0 / RG;
-    double xv[kBatch];
+  // the batch's values of row-group rounds t0 .. t0 + B - 1
+  __device__ __forceinline__ void load(double (&xv)[B], int t0, int k0, int kq, int n, long stride) const {
+    const int q0 = t0 / RG, kl = lane & 3;
 #pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
+    for (int u = 0; u < B; ++u) {
       const int q = q0 + u / RG, r = u % RG;
       const int kk = k0 + 4 * q + kl;
       xv[u] = (q < kq && kk < n && cv[r]) ? X[base[r] + (long)kk * stride] : 0.0;
     }
+  }
+  __device__ __forceinline__ void store(const double (&xv)[B], int t0, int kq, unsigned char* sAh,
+                                        unsigned char* sAl) const {
+    const int q0 = t0 / RG;
 #pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
+    for (int u = 0; u < B; ++u) {
       const int q = q0 + u / RG, r = u % RG;
       if (q < kq) {
         float h, l;
@@ -216,6 +226,18 @@ __device__ __forceinline__ void fill_a(int wi, int lane, const double* __restric
         *(float*)(sAl + off) = l;
       }
     }
+  }
+};
+template <int AXIS, int RG>
+__device__ __forceinline__ void fill_a(int wi, int lane, const double* __restrict__ X, long c0, long ncols, int k0,
+                                       int kc, int n, long stride, int nx, int ny, long N, unsigned char* sAh,
+                                       unsigned char* sAl) {
+  const FillA<AXIS, RG, kBatch> f(wi, lane, X, c0, ncols, nx, ny, N);
+  const int kq = kc >> 2;  // core matrices along K
+  for (int t0 = 0; t0 < RG * kq; t0 += kBatch) {
+    double xv[kBatch];
+    f.load(xv, t0, k0, kq, n, stride);
+    f.store(xv, t0, kq, sAh, sAl);
   }
 }
 
@@ -258,6 +280,7 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
   // A tile and the B chunk are staged, multiplied into the same accumulator,
   // and the shared memory is reused once those MMAs have completed.
   extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr bool kAhead = TH == kHalfThreads;
   const int n = am.n;
   const uint32_t b_bytes = (uint32_t)npad * kc * 4;  // one K chunk of one half of B
   const uint32_t a_bytes = (uint32_t)kTileM * kc * 4;
@@ -329,12 +352,19 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
     const double* __restrict__ v = jobs.j[jb].v;
     const long ncols = jobs.j[jb].ncols;
     const long c0 = (tile - jobs.j[jb].tile0) * kTileM;
+    // two CTAs per SM: a chunk is one batch, loaded while the chunk before it
+    // is multiplied
+    constexpr int RG = kThreads / TH;
+    const FillA<AXIS, RG, kAhead ? kHalfBatch : RG> ahead(warp, lane, X, c0, ncols, nx, ny, N);
+    double xv[kAhead ? kHalfBatch : RG];
+    if (kAhead) ahead.load(xv, 0, 0, kc >> 2, n, am.stride);
     for (int ch = 0; ch < nch; ++ch) {
       const int k0 = ch * kc;
       if (nch > 1 && !first && tid == 0) load_b(ch);  // the previous chunk's MMAs have completed
       first = false;
       // ---- A operand: 128 columns x kc, split into TF32 hi/lo
-      fill_a<AXIS, kThreads / TH>(warp, lane, X, c0, ncols, k0, kc, n, am.stride, nx, ny, N, sAh, sAl);
+      if (kAhead) ahead.store(xv, 0, kc >> 2, sAh, sAl);
+      else fill_a<AXIS, RG>(warp, lane, X, c0, ncols, k0, kc, n, am.stride, nx, ny, N, sAh, sAl);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       bool bok = true;
@@ -369,6 +399,7 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
             smem_u32(&mbar)));
       }
+      if (kAhead && ch + 1 < nch) ahead.load(xv, 0, k0 + kc, kc >> 2, n, am.stride);
       const bool waited = mbar_wait(smem_u32(&mbar), phase);
       phase ^= 1u;
       if (!__syncthreads_and(waited ? 1 : 0)) {
@@ -697,9 +728,11 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
   // one persistent CTA of kThreads per SM, or the tuned count
   const long cap = ctas > 0 && ctas < g_num_sms ? ctas : g_num_sms;
   // several K chunks and more tiles than SMs: two CTAs of half the threads per
-  // SM (160^3 x 16: 2.25 -> 1.67 ms; with one tile per SM or fewer the wide
+  // SM, which load a chunk while the one before is multiplied (160^3 x 16:
+  // 2.25 -> 1.18 ms together with the x epilogue's loads apart from their
+  // product, 1.34 without the loads ahead; with one tile per SM or fewer the wide
   // CTA is faster, 128x64x40 x 3: 55 us against 60)
-  const bool half = nch > 1 && tiles > cap;
+  const bool half = nch > 1 && tiles > cap && kc <= 2 * kHalfBatch;
   const int grid = (int)std::min<long>(tiles, half ? 2 * cap : cap);
   int* err = g->tc_err.p;
   const size_t a_region = (size_t)2 * kTileM * kc * 4, b_region = (size_t)2 * npad * kc * 4;
