@@ -7,9 +7,18 @@
 //   (T - sigma)^-1 = (Q (x) Q (x) Q) D^-1 (Q (x) Q (x) Q)^T,
 //   D(i,j,k) = dx_i + dy_j + dz_k - sigma, |D| kept at least `floor`.
 // Three kinds of work items per vector, each two chained contractions:
-//   XF, plane k of R:     W1 = Q^T P Q      (x, then y forward)
+//   XF, planes of R:      W1 = Q^T P Q      (x, then y forward)
 //   ZS, 128 grid lines:   W2 = Q D^-1 Q^T L  (z forward, the diagonal, z backward)
-//   XB, plane k of W2:    R  = Q P Q^T      (x, then y backward)
+//   XB, planes of W2:     R  = Q P Q^T      (x, then y backward)
+// An XF or XB item is one plane, or, for n <= 64 (32), two (four), where the
+// launch has more planes than SMs: their rows lie one after the other in the
+// B operand of the first MMA, and the eigenbasis is stacked in A, so that
+// every block of 64 (32) TMEM lanes holds a copy of all the planes' products
+// and takes its own plane's columns on to the second MMA.  With a plane to an
+// item half of the lanes and of the epilogue's warps do nothing, and an item
+// of two planes takes little longer: 64^3 x 4 41.9 -> 38.8 us, x 16 134 -> 111,
+// 32^3 x 32 144 -> 102 (with fewer planes than SMs, 64^3 x 1, one plane is
+// better, 37.5 against 38.6).
 // A ZS item of a vector starts once every XF plane of the vector is in W1, an
 // XB item once every ZS tile of the vector is in W2 (per-vector completion
 // counters, bounded waits); the ticket order (XF(s), ZS(s - L), XB(s - 2L) for
@@ -32,6 +41,12 @@
 // (a power of two) and writes FP64.  The factor 2^-4 keeps the intermediate below 2^15:
 // an orthonormal transform grows no entry by more than sqrt(n) < 16, and in a
 // ZS item 2^-ef bounds 1 / |D| <= 1 / floor.
+//
+// Bound by the latency of the three phases, about 9 us each on 64^3: copies
+// landing 1, exponents 1, conversion 2, two MMAs 2, intermediate 1, output 1,
+// release and acquire 2.  (The output took 3.4 with an address product, an
+// exponent and a case distinction per value: 64^3 x 1 37.5 -> 32.9 us, 96^3 x 8
+// 158 -> 133.)
 //
 // Every wait is bounded; a timeout sets the grid's error word and the kernel
 // drains its copies and MMAs and returns.
@@ -57,6 +72,8 @@ struct KinGeom {
   int kx, ky, kz;     // K extents padded to 16 (also the padded N extents)
   int npy, npz;
   int nzt;            // ZS items per vector
+  int pp, nzi;        // planes per XF or XB item (1, 2 or 4), and those items per vector
+  uint32_t plane_stg; // staging bytes of one plane
   int lag;            // steps between a vector's XF, ZS and XB items
   int tau;            // the eigenbasis images hold Q 2^tau
   int ef;             // 1 / |D| <= 2^ef
@@ -88,10 +105,10 @@ struct KinArgs {
 struct KinCounters {
   unsigned ticket;
   unsigned finished;
-  unsigned done_xf[kKinMaxVec];  // XF planes in W1, per vector
-  unsigned done_zs[kKinMaxVec];  // ZS tiles in W2, per vector
-  unsigned exp_w1[kKinMaxVec];   // largest FP64 exponent (biased) in W1, per vector
-  unsigned exp_w2[kKinMaxVec];   // the same in W2
+  // per vector: items done and the largest FP64 exponent (biased) written,
+  // side by side so that a waiter reads both at once
+  uint2 w1[kKinMaxVec];  // XF items
+  uint2 w2[kKinMaxVec];  // ZS items
 };
 
 }  // namespace pg
@@ -103,15 +120,16 @@ using pg::KinCounters;
 using pg::KinGeom;
 
 constexpr int kXF = 0, kZS = 1, kXB = 2;
+constexpr int kMaxPlanes = 4;  // of one item
 
 struct KItem {
   int kind;  // kXF, kZS, kXB; -1: none
   int u;     // vector
-  int idx;   // plane or tile
+  int idx;   // plane group or tile
 };
 
-// Ticket -> item: steps s = 0, 1, ... hold XF(s) (nz planes), ZS(s - L) (nzt
-// tiles) and XB(s - 2L) (nz planes), each where the vector exists.
+// Ticket -> item: steps s = 0, 1, ... hold XF(s) (nz plane groups), ZS(s - L)
+// (nzt tiles) and XB(s - 2L) (nz plane groups), each where the vector exists.
 __device__ __forceinline__ KItem kdecode(unsigned t, int nvec, int nz, int nzt, int L) {
   for (int s = 0; s < nvec + 2 * L; ++s) {
     if (s < nvec) {
@@ -143,19 +161,21 @@ __device__ __forceinline__ bool kstage(const KinGeom& G, const KinArgs& A, const
   if (it.kind < 0) return true;
   int ok = 1;
   if (lane == 0 && it.kind != kXF) {
-    const volatile unsigned* c = it.kind == kZS ? &cnt->done_xf[it.u] : &cnt->done_zs[it.u];
-    const unsigned need = it.kind == kZS ? (unsigned)G.nz : (unsigned)G.nzt;
+    const uint2* c = it.kind == kZS ? &cnt->w1[it.u] : &cnt->w2[it.u];
+    const unsigned need = it.kind == kZS ? (unsigned)G.nzi : (unsigned)G.nzt;
     const unsigned long long t0 = globaltimer_ns();
-    while (*c < need) {
+    unsigned long long d;
+    while (true) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(c) : "memory");
+      if ((unsigned)d >= need) break;
       if (*abort || globaltimer_ns() - t0 > 2000000000ull) {
         ok = 0;
         break;
       }
-      __nanosleep(64);
+      __nanosleep(32);
     }
     // the item's scale comes from the largest exponent of the whole input vector
-    __threadfence();
-    *exp_out = (int)*(it.kind == kZS ? (volatile unsigned*)&cnt->exp_w1[it.u] : (volatile unsigned*)&cnt->exp_w2[it.u]);
+    *exp_out = (int)(d >> 32);
   }
   ok = __shfl_sync(0xffffffffu, ok, 0);
   if (!ok) return false;
@@ -165,7 +185,8 @@ __device__ __forceinline__ bool kstage(const KinGeom& G, const KinArgs& A, const
     fence_proxy_async_global();
   }
   const bool xy = it.kind != kZS;
-  const int nbox = xy ? (G.nx + 15) / 16 : kTile / 16;
+  const int nbox1 = (G.nx + 15) / 16, z0 = it.idx * G.pp;  // an item's planes z0 ..
+  const int nbox = xy ? nbox1 * (G.nz - z0 < G.pp ? G.nz - z0 : G.pp) : kTile / 16;
   const uint32_t box_bytes = 128u * (uint32_t)(xy ? G.ny : G.nz);
   if (lane == 0) {
     uint64_t state;
@@ -178,13 +199,15 @@ __device__ __forceinline__ bool kstage(const KinGeom& G, const KinArgs& A, const
   const uint32_t dst0 = smem_u32(smem + G.stg);
   if (xy) {
     const void* map = it.kind == kXF ? &A.r_xy : &A.w2_xy;
-    const int zc = it.u * G.nz + it.idx;
-    for (int b = lane; b < nbox; b += 32)
+    const int zc = it.u * G.nz + z0;
+    for (int b = lane; b < nbox; b += 32) {
+      const int h = b / nbox1;
       asm volatile(
           "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-          "[%5];" ::"r"(dst0 + (uint32_t)b * G.reg_xy),
-          "l"(map), "r"(16 * b), "r"(0), "r"(zc), "r"(bar)
+          "[%5];" ::"r"(dst0 + (uint32_t)h * G.plane_stg + (uint32_t)(b - h * nbox1) * G.reg_xy),
+          "l"(map), "r"(16 * (b - h * nbox1)), "r"(0), "r"(zc + h), "r"(bar)
           : "memory");
+    }
   } else {
     const void* map = &A.w1_z;
     const int p0 = it.idx * kTile;
@@ -197,6 +220,20 @@ __device__ __forceinline__ bool kstage(const KinGeom& G, const KinArgs& A, const
           : "memory");
   }
   return true;
+}
+
+// A conversion task (pg_tc16.cuh) of an item; an xy item's row counts over its
+// planes' padded rows.  h: its plane within the item.
+__device__ __forceinline__ Task ktask(const KinGeom& G, int ck, int planes, const TaskIter& ti, int& h) {
+  h = 0;
+  if (ck) return task_z(G, ti.row, ti.major);
+  int j = ti.row;
+  while (j >= G.npy) j -= G.npy, ++h;
+  Task k = task_xy(G, j, ti.major);
+  if (h >= planes) k.row = -1;
+  else k.src += (uint32_t)h * G.plane_stg;
+  k.dst += (uint32_t)(h * (G.npy >> 3)) * (uint32_t)(G.kx >> 3) * 128u;
+  return k;
 }
 
 // Sixteen FP32 values (one TMEM row segment) -> two 16-byte rows of FP16 high
@@ -229,8 +266,8 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       mbar_acc_empty[kMaxAcc], mbar_stg;
   __shared__ uint32_t tmem_base;
   __shared__ unsigned ring[kRing];
-  __shared__ int sig[kRing];  // item scale exponents, by ticket slot
-  __shared__ int s_emax[kProdWarps];
+  __shared__ int sig[kRing][kMaxPlanes];  // scale exponents of the item's planes, by ticket slot
+  __shared__ int s_emax[kMaxPlanes][kProdWarps];
   __shared__ int s_vexp[kRing];  // ZS and XB items: largest exponent of the input vector, by ticket slot
   __shared__ float s_d[3][kTile];  // eigenvalues per axis, zero past n
   __shared__ int s_abort, s_prod_ok, s_epi_ok, s_last, s_stg_issued;
@@ -253,19 +290,21 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    // the eigenbasis images (the grid's constant data) while the kernel ahead finishes
+    // the eigenbasis images (the grid's constant data) while the kernel ahead
+    // finishes; one under the other for the planes of an item
     const int nimg = G.q_sym ? 2 : 4;
+    const uint32_t q_row = (uint32_t)(G.kx >> 3) * 16u;  // bytes of a row
     uint64_t state;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 %0, [%1], %2;"
                  : "=l"(state)
-                 : "r"(smem_u32(&mbar_q)), "r"((uint32_t)nimg * G.q_bytes)
+                 : "r"(smem_u32(&mbar_q)), "r"((uint32_t)(nimg * G.pp) * G.q_bytes)
                  : "memory");
     const unsigned short* src[4] = {qf_hi, qf_lo, qb_hi, qb_lo};
     const uint32_t dst[4] = {G.qf_hi, G.qf_lo, G.qb_hi, G.qb_lo};
-    for (int m = 0; m < nimg; ++m)
+    for (int m = 0; m < nimg * G.pp; ++m)
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       smem_u32(smem + dst[m])),
-                   "l"(src[m]), "r"(G.q_bytes), "r"(smem_u32(&mbar_q))
+                       smem_u32(smem + dst[m / G.pp]) + (uint32_t)(m % G.pp) * (uint32_t)(kTile / G.pp) * q_row),
+                   "l"(src[m / G.pp]), "r"(G.q_bytes), "r"(smem_u32(&mbar_q))
                    : "memory");
   }
   if (warp == 0) {
@@ -273,17 +312,18 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
                  "r"(G.acc_cols << G.acc_shift));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  // so are the eigenvalues
+  for (int e = tid; e < 3 * kTile; e += kThreadsAll) {
+    const int a = e / kTile, i = e % kTile;
+    const int n = a == 0 ? G.nx : (a == 1 ? G.ny : G.nz);
+    s_d[a][i] = i < n ? (float)A.d[a][i] : 0.f;
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   pg::pdl_wait();
   pg::pdl_release();
   const uint32_t tmem = tmem_base;
-  for (int e = tid; e < 3 * kTile; e += kThreadsAll) {
-    const int a = e / kTile, i = e % kTile;
-    const int n = a == 0 ? G.nx : (a == 1 ? G.ny : G.nz);
-    s_d[a][i] = i < n ? (float)A.d[a][i] : 0.f;
-  }
   if (tid == 0) ring[0] = atomicAdd(&cnt->ticket, 1u);
   __syncthreads();
 
@@ -293,7 +333,7 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
     const uint32_t bar_stg = smem_u32(&mbar_stg);
     const unsigned char* stg = smem + G.stg;
     if (warp == 0) {
-      const KItem it0 = kdecode(ring[0], nvec, G.nz, G.nzt, G.lag);
+      const KItem it0 = kdecode(ring[0], nvec, G.nzi, G.nzt, G.lag);
       const bool ok = kstage(G, A, it0, cnt, smem, bar_stg, lane, abort, &s_vexp[0]);
       if (lane == 0) {
         if (!ok) *abort = 1;
@@ -301,7 +341,7 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       }
     }
     for (int i = 0;; ++i) {
-      const KItem it = kdecode(ring[i % kRing], nvec, G.nz, G.nzt, G.lag);
+      const KItem it = kdecode(ring[i % kRing], nvec, G.nzi, G.nzt, G.lag);
       if (ptid == 0) ring[(i + 1) % kRing] = atomicAdd(&cnt->ticket, 1u);
       if (it.kind < 0) {
         // no more work: hand the issuer its stop item once the image is free
@@ -321,11 +361,47 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       named_sync(1, kProdWarps * 32);
       if (!s_prod_ok) break;
       const int ck = it.kind == kZS ? 1 : 0;  // conversion tasks: z tile or plane
-      const int ntask = ck == 0 ? (G.kx >> 3) * G.npy : 16 * G.kz;
-      if (it.kind == kXF) {  // the item's scale: its largest exponent over the producers
-        int em = max_exponent(stg, ntask, ck, G, ptid);
-        em = (int)__reduce_max_sync(0xffffffffu, (unsigned)em);
-        if (lane == 0) s_emax[warp] = em;
+      const int rows = ck == 0 ? G.pp * G.npy : G.kz;
+      const int ntask = ck == 0 ? (G.kx >> 3) * rows : 16 * G.kz;
+      const int planes = G.nz - it.idx * G.pp < G.pp ? G.nz - it.idx * G.pp : G.pp;
+      if (it.kind == kXF) {  // a plane's scale: its largest exponent over the producers
+        uint32_t em[kMaxPlanes] = {0, 0, 0, 0};
+        TaskIter ti(ptid, rows);
+        auto scan = [&](const double (&v)[8], int h) {
+          uint32_t m = 0;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t e = (uint32_t)__double2hiint(v[q]) & 0x7fffffffu;
+            m = e > m ? e : m;
+          }
+          m >>= 20;
+#pragma unroll
+          for (int p = 0; p < kMaxPlanes; ++p) em[p] = h == p && m > em[p] ? m : em[p];
+        };
+        int t = ptid, h0, h1;
+        for (; t + kProdWarps * 32 < ntask; t += 2 * kProdWarps * 32) {
+          const Task k0 = ktask(G, 0, planes, ti, h0);
+          ti.next();
+          const Task k1 = ktask(G, 0, planes, ti, h1);
+          ti.next();
+          double v0[8], v1[8];
+          load8(stg, k0, v0);
+          load8(stg, k1, v1);
+          scan(v0, h0);
+          scan(v1, h1);
+        }
+        if (t < ntask) {
+          const Task k0 = ktask(G, 0, planes, ti, h0);
+          double v0[8];
+          load8(stg, k0, v0);
+          scan(v0, h0);
+        }
+#pragma unroll
+        for (int p = 0; p < kMaxPlanes; ++p)
+          if (p < G.pp) {
+            const unsigned m = __reduce_max_sync(0xffffffffu, em[p]);
+            if (lane == 0) s_emax[p][warp] = (int)m;
+          }
       }
       // the image is free once the previous item's second MMA is done
       if (ptid == 0) {
@@ -335,46 +411,53 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       }
       named_sync(1, kProdWarps * 32);
       if (!s_prod_ok) break;
-      int emax = 0;
-      if (it.kind == kXF) {
+      int sp[kMaxPlanes];
 #pragma unroll
-        for (int w = 0; w < kProdWarps; ++w) emax = s_emax[w] > emax ? s_emax[w] : emax;
-      } else {
-        emax = s_vexp[i % kRing];
+      for (int p = 0; p < kMaxPlanes; ++p) {
+        int emax = 0;
+        if (it.kind == kXF) {
+          if (p < G.pp) {
+#pragma unroll
+            for (int w = 0; w < kProdWarps; ++w) emax = s_emax[p][w] > emax ? s_emax[p][w] : emax;
+          }
+        } else {
+          emax = s_vexp[i % kRing];
+        }
+        // largest |x| < 2^(emax - 1022): scaled below 2^15; the factors of both
+        // epilogues, 2^-(s + tau - 4 [- ef]), stay normal FP32 numbers
+        int s = (emax == 0 || emax == 0x7ff) ? 0 : 1037 - emax;
+        const int s_lo = -123 - G.tau + G.ef, s_hi = 126 - G.tau;
+        s = s > s_hi ? s_hi : (s < s_lo ? s_lo : s);
+        if (ptid == 0) sig[i % kRing][p] = s;
+        sp[p] = s - 896;
       }
-      // largest |x| < 2^(emax - 1022): scaled below 2^15; the factors of both
-      // epilogues, 2^-(s + tau - 4 [- ef]), stay normal FP32 numbers
-      int s = (emax == 0 || emax == 0x7ff) ? 0 : 1037 - emax;
-      const int s_lo = -123 - G.tau + G.ef, s_hi = 126 - G.tau;
-      s = s > s_hi ? s_hi : (s < s_lo ? s_lo : s);
-      if (ptid == 0) sig[i % kRing] = s;
+      auto sb = [&](int h) { return h == 0 ? sp[0] : (h == 1 ? sp[1] : (h == 2 ? sp[2] : sp[3])); };
       unsigned char* ohi = smem + G.op_hi;
       unsigned char* olo = smem + G.op_lo;
-      TaskIter ti(ptid, ck == 0 ? G.npy : G.kz);
-      const int sb = s - 896;
-      int t = ptid;
+      TaskIter ti(ptid, rows);
+      int t = ptid, h0, h1;
       for (; t + kProdWarps * 32 < ntask; t += 2 * kProdWarps * 32) {
-        const Task k0 = task_of(G, ck, ti);
+        const Task k0 = ktask(G, ck, planes, ti, h0);
         ti.next();
-        const Task k1 = task_of(G, ck, ti);
+        const Task k1 = ktask(G, ck, planes, ti, h1);
         ti.next();
         double v0[8], v1[8];
         load8(stg, k0, v0);
         load8(stg, k1, v1);
-        uint4 h0, l0, h1, l1;
-        split8(v0, sb, h0, l0);
-        split8(v1, sb, h1, l1);
-        *reinterpret_cast<uint4*>(ohi + k0.dst) = h0;
-        *reinterpret_cast<uint4*>(olo + k0.dst) = l0;
-        *reinterpret_cast<uint4*>(ohi + k1.dst) = h1;
-        *reinterpret_cast<uint4*>(olo + k1.dst) = l1;
+        uint4 hi0, lo0, hi1, lo1;
+        split8(v0, sb(h0), hi0, lo0);
+        split8(v1, sb(h1), hi1, lo1);
+        *reinterpret_cast<uint4*>(ohi + k0.dst) = hi0;
+        *reinterpret_cast<uint4*>(olo + k0.dst) = lo0;
+        *reinterpret_cast<uint4*>(ohi + k1.dst) = hi1;
+        *reinterpret_cast<uint4*>(olo + k1.dst) = lo1;
       }
       if (t < ntask) {
-        const Task k = task_of(G, ck, ti);
+        const Task k = ktask(G, ck, planes, ti, h0);
         double v[8];
         load8(stg, k, v);
         uint4 h, l;
-        split8(v, sb, h, l);
+        split8(v, sb(h0), h, l);
         *reinterpret_cast<uint4*>(ohi + k.dst) = h;
         *reinterpret_cast<uint4*>(olo + k.dst) = l;
       }
@@ -382,7 +465,7 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       named_sync(1, kProdWarps * 32);
       mbar_arrive(smem_u32(&mbar_full));
       if (warp == 0) {
-        const KItem nx_it = kdecode(ring[(i + 1) % kRing], nvec, G.nz, G.nzt, G.lag);
+        const KItem nx_it = kdecode(ring[(i + 1) % kRing], nvec, G.nzi, G.nzt, G.lag);
         const bool ok = kstage(G, A, nx_it, cnt, smem, bar_stg, lane, abort, &s_vexp[(i + 1) % kRing]);
         if (lane == 0) {
           if (!ok) *abort = 1;
@@ -394,12 +477,13 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
     // ------------------------------------------------------------- epilogue
     const int quarter = warp & 3, part = (warp - kProdWarps) >> 2;  // warps of one lane quarter share its columns
     const bool leader = warp == kProdWarps && lane == 0;
-    const int r = 32 * quarter + lane;  // TMEM lane: x index (planes) or line of the tile
+    const int r = 32 * quarter + lane;  // TMEM lane: line of the tile, or x index xr of the item's plane xh
+    const int xh = 32 * quarter / (kTile / G.pp), xr = r - xh * (kTile / G.pp);
     unsigned char* mhi = smem + G.mid_hi;
     unsigned char* mlo = smem + G.mid_lo;
     for (int i = 0;; ++i) {
       const int b = i & ((1 << G.acc_shift) - 1);
-      const KItem it = kdecode(ring[i % kRing], nvec, G.nz, G.nzt, G.lag);
+      const KItem it = kdecode(ring[i % kRing], nvec, G.nzi, G.nzt, G.lag);
       if (leader) {
         const int ok = mbar_wait_or_abort(smem_u32(&mbar_acc_full[b]), 0u, abort);
         if (!ok) *abort = 1;
@@ -409,15 +493,18 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       if (!s_epi_ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (it.kind < 0) break;
-      const int s = sig[i % kRing];
       const bool zs = it.kind == kZS;
+      const int s = sig[i % kRing][zs ? 0 : xh];
+      const int plane = it.idx * G.pp + xh;
+      const bool xy_valid = xr < G.nx && plane < G.nz;
       const uint32_t acc = tmem + (uint32_t)b * G.acc_cols + ((uint32_t)(32 * quarter) << 16);
       const int ncol = zs ? G.npz : G.npy;  // columns of both results
       const int kq = (zs ? G.kz : G.ky) >> 3;  // core matrices along K of the second A image
       // ---- first result -> the second MMA's A image (K-major, row r)
       {
         const long p = zs ? (long)it.idx * kTile + r : 0;
-        const bool valid = zs ? p < nxny : r < G.nx;
+        const bool valid = zs ? p < nxny : xy_valid;
+        const uint32_t first = acc + (uint32_t)(zs ? 0 : xh * G.npy);  // the plane's columns
         float dxy = 0.f, sg = 0.f;
         if (zs && valid) {
           const int ii = (int)(p % G.nx), jj = (int)(p / G.nx);
@@ -428,7 +515,7 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
         const uint32_t row = (uint32_t)(r >> 3) * (uint32_t)kq * 128u + (uint32_t)(r & 7) * 16u;
         for (int c = part; c < (ncol >> 4); c += kEpiParts) {
           float d[16];
-          tmem_ld16(acc + (uint32_t)(16 * c), d);
+          tmem_ld16(first + (uint32_t)(16 * c), d);
 #pragma unroll
           for (int q = 0; q < 16; ++q) {
             float a = valid ? d[q] * f : 0.f;
@@ -459,51 +546,47 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       // (W1 and W2: the scale of the next phase's items)
       {
         const float unscale = exp2i(-(s + G.tau - 4 - (zs ? G.ef : 0)));
-        uint32_t em = 0;
-        auto track = [&em](float v) {
-          const uint32_t e = (__float_as_uint(v) >> 23) & 0xffu;
-          const uint32_t e64 = e == 0 ? 0u : (e == 255 ? 0x7ffu : e + 896u);
-          em = e64 > em ? e64 : em;
-        };
-        if (zs) {
-          const long p = (long)it.idx * kTile + r;
-          double* out = A.w2 + (long)it.u * nxny * G.nz;
-          for (int c = part; c < (G.npz >> 4); c += kEpiParts) {
-            float d[16];
-            tmem_ld16(acc + (uint32_t)(16 * c), d);
-            if (p < nxny) {
+        const long p = (long)it.idx * kTile + r;
+        const bool valid = zs ? p < nxny : xy_valid;
+        double* out = (zs ? A.w2 : (it.kind == kXF ? A.w1 : A.r)) + (long)it.u * nxny * G.nz +
+                      (zs ? p : nxny * plane + xr);
+        const long stride = zs ? nxny : G.nx;
+        const int nout = zs ? G.nz : G.ny;
+        uint32_t big = 0;  // largest |value| as bits
+        for (int c = part; c < (ncol >> 4); c += kEpiParts) {
+          float d[16];
+          tmem_ld16(acc + (uint32_t)(16 * c), d);
+          if (!valid) continue;
+          double* o = out + stride * (16 * c);
+          const int left = nout - 16 * c;
+          uint32_t mx = 0, mn = 0xffffffffu;
 #pragma unroll
-              for (int q = 0; q < 16; ++q) {
-                const int k = 16 * c + q;
-                if (k < G.nz) {
-                  const float v = d[q] * unscale;
-                  track(v);
-                  out[p + nxny * k] = f32_to_f64(v);
-                }
-              }
+          for (int q = 0; q < 16; ++q) {
+            d[q] *= unscale;
+            const uint32_t m = __float_as_uint(d[q]) & 0x7fffffffu;
+            if (q < left) {
+              mx = m > mx ? m : mx;
+              mn = m < mn ? m : mn;
             }
           }
-        } else {
-          double* out = (it.kind == kXF ? A.w1 : A.r) + (long)it.u * nxny * G.nz + nxny * it.idx;
-          for (int c = part; c < (G.npy >> 4); c += kEpiParts) {
-            float d[16];
-            tmem_ld16(acc + (uint32_t)(16 * c), d);
-            if (r < G.nx) {
+          big = mx > big ? mx : big;
+          if (left >= 16 && mn >= 0x800000u && mx < 0x7f800000u) {  // normal numbers only
 #pragma unroll
-              for (int q = 0; q < 16; ++q) {
-                const int j = 16 * c + q;
-                if (j < G.ny) {
-                  const float v = d[q] * unscale;
-                  track(v);
-                  out[r + (long)G.nx * j] = f32_to_f64(v);
-                }
-              }
+            for (int q = 0; q < 16; ++q, o += stride) {
+              const uint32_t u = __float_as_uint(d[q]);
+              *o = __hiloint2double((int)((((u & 0x7fffffffu) >> 3) + (896u << 20)) | (u & 0x80000000u)), (int)(u << 29));
             }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 16; ++q, o += stride)
+              if (q < left) *o = f32_to_f64(d[q]);
           }
         }
+        uint32_t em = big >> 23;
+        em = em == 0 ? 0u : (em == 255 ? 0x7ffu : em + 896u);
         if (it.kind != kXB) {
           em = __reduce_max_sync(0xffffffffu, em);
-          if (lane == 0 && em > 0) atomicMax(zs ? &cnt->exp_w2[it.u] : &cnt->exp_w1[it.u], em);
+          if (lane == 0 && em > 0) atomicMax(zs ? &cnt->w2[it.u].y : &cnt->w1[it.u].y, em);
         }
       }
       // W1 and W2 are read next by other CTAs' tensor copies: every writer
@@ -516,7 +599,7 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       if (leader) {
         if (it.kind != kXB) {
           __threadfence();
-          atomicAdd(it.kind == kXF ? &cnt->done_xf[it.u] : &cnt->done_zs[it.u], 1u);
+          atomicAdd(it.kind == kXF ? &cnt->w1[it.u].x : &cnt->w2[it.u].x, 1u);
         }
         mbar_arrive(smem_u32(&mbar_acc_empty[b]));
       }
@@ -524,7 +607,8 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
   } else if (lane == 0) {
     // --------------------------------------------------------------- issuer
     // kind::f16, FP16 A and B, FP32 D; bit 15: A MN-major
-    const uint32_t id_xy = (1u << 4) | ((uint32_t)(G.npy >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+    const uint32_t id_x = (1u << 4) | ((uint32_t)(G.pp * G.npy >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+    const uint32_t id_y = (1u << 4) | ((uint32_t)(G.npy >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
     const uint32_t id_z1 = (1u << 4) | (1u << 15) | ((uint32_t)(G.npz >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
     const uint32_t id_z2 = (1u << 4) | ((uint32_t)(G.npz >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
     const uint32_t sb = smem_u32(smem);
@@ -555,7 +639,7 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
         ok = mbar_wait_or_abort(smem_u32(&mbar_acc_empty[b]), (uint32_t)(((i - nacc) >> G.acc_shift) & 1), abort);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const KItem it = kdecode(ring[i % kRing], nvec, G.nz, G.nzt, G.lag);
+      const KItem it = kdecode(ring[i % kRing], nvec, G.nzi, G.nzt, G.lag);
       if (it.kind < 0) {
         mbar_arrive(smem_u32(&mbar_acc_full[b]));
         mbar_arrive(smem_u32(&mbar_acc_full[b]));
@@ -566,11 +650,11 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
       // first MMA
       if (it.kind != kZS) {
         const uint64_t ah = fw ? d_qfh : d_qbh, al = fw ? d_qfl : d_qbl;
-        for (int kk = 0; kk < G.kx / 16; ++kk) {  // x: A = Q (rows i', K = i), B = plane rows j
+        for (int kk = 0; kk < G.kx / 16; ++kk) {  // x: A = Q (rows i', K = i, per plane), B = the planes' rows j
           const uint64_t o = (uint64_t)kk * 16;
-          mma_f16(acc, al + o, d_pbh + o, id_xy, kk > 0 ? 1u : 0u);
-          mma_f16(acc, ah + o, d_pbl + o, id_xy, 1u);
-          mma_f16(acc, ah + o, d_pbh + o, id_xy, 1u);
+          mma_f16(acc, al + o, d_pbh + o, id_x, kk > 0 ? 1u : 0u);
+          mma_f16(acc, ah + o, d_pbl + o, id_x, 1u);
+          mma_f16(acc, ah + o, d_pbh + o, id_x, 1u);
         }
       } else {
         for (int kk = 0; kk < G.kz / 16; ++kk) {  // z: A = 128 lines (M = point, K = plane), B = Q^T
@@ -598,9 +682,9 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
         const uint64_t bh = fw ? d_qfyh : d_qbyh, bl = fw ? d_qfyl : d_qbyl;
         for (int kk = 0; kk < G.ky / 16; ++kk) {  // y: A = first result (rows i', K = j), B = Q (rows j', K = j)
           const uint64_t o = (uint64_t)kk * 16;
-          mma_f16(acc, d_mxl + o, bh + o, id_xy, kk > 0 ? 1u : 0u);
-          mma_f16(acc, d_mxh + o, bl + o, id_xy, 1u);
-          mma_f16(acc, d_mxh + o, bh + o, id_xy, 1u);
+          mma_f16(acc, d_mxl + o, bh + o, id_y, kk > 0 ? 1u : 0u);
+          mma_f16(acc, d_mxh + o, bl + o, id_y, 1u);
+          mma_f16(acc, d_mxh + o, bh + o, id_y, 1u);
         }
       } else {
         for (int kk = 0; kk < G.kz / 16; ++kk) {  // z back: A = scaled result (rows point, K = k'), B = Q
@@ -641,10 +725,8 @@ __global__ void __launch_bounds__(kThreadsAll, 1)
   __syncthreads();
   if (s_last) {
     for (int u = tid; u < nvec; u += kThreadsAll) {
-      cnt->done_xf[u] = 0;
-      cnt->done_zs[u] = 0;
-      cnt->exp_w1[u] = 0;
-      cnt->exp_w2[u] = 0;
+      cnt->w1[u] = make_uint2(0, 0);
+      cnt->w2[u] = make_uint2(0, 0);
     }
     if (tid == 0) {
       cnt->ticket = 0;
@@ -710,6 +792,7 @@ KinPlan plan_kin(const pg_grid* g) {
   G.npz = tc_npad(nz);
   G.nzt = (int)(((long)nx * ny + kTile - 1) / kTile);
   G.lag = 1;
+  const int pp = nx <= 32 ? 4 : (nx <= 64 ? 2 : 1);  // planes of an item, at most (kin_f16 sets pp and nzi)
   G.tau = g->q16_scale;
   G.q_sym = g->q16_sym ? 1 : 0;
   const uint32_t npx = (uint32_t)tc_npad(nx);
@@ -730,9 +813,9 @@ KinPlan plan_kin(const pg_grid* g) {
     G.qb_lo = cur;
     cur += q_slot;
   }
-  // the operand image: a plane (npy x kx, plus the overread of a 128-row
-  // A read), a z tile (128 x kz), or the second A image (128 x k)
-  const uint32_t plane = (uint32_t)G.npy * (uint32_t)G.kx * 2u + kOverread;
+  // the operand image: planes (npy x kx each, and one alone plus the overread
+  // of a 128-row A read), a z tile (128 x kz), or the second A image (128 x k)
+  const uint32_t plane = (uint32_t)(pp * G.npy) * (uint32_t)G.kx * 2u + (pp == 1 ? kOverread : 0u);
   const uint32_t ztile = (uint32_t)kTile * (uint32_t)std::max(G.ky, G.kz) * 2u;
   const uint32_t op = (std::max(plane, ztile) + 127u) / 128u * 128u;
   G.op_hi = cur;
@@ -741,7 +824,8 @@ KinPlan plan_kin(const pg_grid* g) {
   cur += op;
   G.reg_xy = (uint32_t)(128 * ny + 1023) / 1024u * 1024u;
   G.reg_z = (uint32_t)(128 * nz + 1023) / 1024u * 1024u;
-  const uint32_t stg_bytes = std::max((uint32_t)((nx + 15) / 16) * G.reg_xy, (uint32_t)(kTile / 16) * G.reg_z);
+  G.plane_stg = (uint32_t)((nx + 15) / 16) * G.reg_xy;
+  const uint32_t stg_bytes = std::max((uint32_t)pp * G.plane_stg, (uint32_t)(kTile / 16) * G.reg_z);
   // the second A image (128 rows): in a region of its own if that fits, so
   // that the producers convert the next item while the second MMA runs
   const uint32_t mid = (uint32_t)kTile * (uint32_t)std::max(G.ky, G.kz) * 2u;
@@ -761,7 +845,7 @@ KinPlan plan_kin(const pg_grid* g) {
   P.smem = cur;
   if ((long)P.smem > (long)g_kin_max_dyn) return no("images and staging exceed shared memory");
   uint32_t cols = 32;
-  while (cols < (uint32_t)std::max(G.npy, G.npz)) cols <<= 1;
+  while (cols < (uint32_t)std::max(pp * G.npy, G.npz)) cols <<= 1;
   G.acc_cols = cols;
   G.acc_shift = cols * 4 <= 512 ? 2 : 1;
   P.ok = true;
@@ -853,7 +937,13 @@ pg_status kin_f16(const pg_grid* g, double* R, double* w1, double* w2, int k, co
     // in flight that ZS and XB items seldom wait (measured at 48-96 points,
     // 2-8 vectors); with one or two vectors the order matters little
     P.G.lag = nb >= 3 ? 3 : 1;
-    const long items = (long)nb * (2 * P.G.nz + P.G.nzt);
+    // several planes to an item once there are more planes than SMs; fewer
+    // planes go to an SM each
+    P.G.pp = 1;
+    const int most = P.G.nx <= 32 ? 4 : (P.G.nx <= 64 ? 2 : 1);
+    while (P.G.pp < most && (long)nb * ((P.G.nz + P.G.pp - 1) / P.G.pp) > g_kin_sms) P.G.pp *= 2;
+    P.G.nzi = (P.G.nz + P.G.pp - 1) / P.G.pp;
+    const long items = (long)nb * (2 * P.G.nzi + P.G.nzt);
     const int grid = (int)std::min<long>(items, g_kin_sms);
     const unsigned short* qbh = g->q16_sym ? g->q16f_hi.p : g->q16b_hi.p;
     const unsigned short* qbl = g->q16_sym ? g->q16f_lo.p : g->q16b_lo.p;
