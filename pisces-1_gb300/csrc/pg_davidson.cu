@@ -96,20 +96,20 @@ int blocks_for(long N) {
 
 // ritz_r = U_r / |U_r|;  res_r = W_r - lambda_r ritz_r   (src/Davidson.cpp:240-260),
 // with per-block partial sums of |res_r|^2, reduced by the last block into
-// rsq (|res_r|^2, then 1/|res_r|).  uinv[r] = 1/|U_r| (written by the
-// combine that formed U).
+// hsq[nr + r]; hsq[r] = |U_r|^2 (page-locked host memory: the norms need no
+// copy).  usq: |U_r|^2, then 1/|U_r| (written by the combine that formed U).
 template <int NR>
 __global__ void __launch_bounds__(kT) k_ritz_residual(long N, long chunk, int nr, double* __restrict__ U,
-                                                      double* __restrict__ W, const double* __restrict__ uinv,
+                                                      double* __restrict__ W, const double* __restrict__ usq,
                                                       const double* __restrict__ lam, double* __restrict__ partial,
-                                                      double* rsq, unsigned* counter) {
+                                                      double* hsq, unsigned* counter) {
   pdl_wait();
   pdl_release();
   __shared__ double red[kT / 32][NR];
   double inv[NR], nl[NR], acc[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
-    inv[r] = r < nr ? uinv[r] : 0.0;
+    inv[r] = r < nr ? usq[nr + r] : 0.0;
     nl[r] = r < nr ? -lam[r] : 0.0;
     acc[r] = 0.0;
   }
@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(kT) k_ritz_residual(long N, long chunk, int nr
     for (int w = 0; w < kT / 32; ++w) t += red[w][threadIdx.x];
     partial[(long)blockIdx.x * nr + threadIdx.x] = t;
   }
-  reduce_in_last_block(partial, nr, rsq, 1, counter);
+  if (blockIdx.x == 0 && threadIdx.x < nr) hsq[threadIdx.x] = usq[threadIdx.x];
+  reduce_in_last_block(partial, nr, hsq + nr, 0, counter);
 }
 
 // Davidson correction (lambda - diag H)^-1 r with the 1e-12 floor
@@ -300,9 +301,7 @@ namespace pg {
 namespace {
 
 // Device scalars of one Davidson handle (offsets into pg_davidson::dsq).
-constexpr int kUsq = 0;     // |U_r|^2 and 1/|U_r| (2 x 16); mixed form: |U_r|^2 and |W_r|^2 (k_ritz_df)
-constexpr int kLam = 32;    // Ritz values (16)
-constexpr int kRsq = 64;    // |r_r|^2 and 1/|r_r| (2 x 16)
+constexpr int kUsq = 0;     // |U_r|^2 and 1/|U_r| (2 x 16, FP64 form)
 constexpr int kOnes = 96;   // 1.0 (16), the "keep X" coefficients of combine
 constexpr int kDots = 112;  // Jacobi-Davidson dot products (2)
 constexpr int kSigma = 128; // shifts of the kinetic preconditioner (2 x 16)
@@ -310,12 +309,11 @@ constexpr int kScalars = 256;
 
 // Regions of pg_davidson::hpin (doubles)
 constexpr int kPinCols = 0;                    // new S columns, m x nc <= 128 x 128
-constexpr int kPinHsq = kPinCols + 128 * 128;  // |U_r|^2 ... |r_r|^2 (kRsq + 16)
-constexpr int kPinV = kPinHsq + 96;            // Ritz coefficients, maxsub x nroots <= 128 x 16
-constexpr int kPinLam = kPinV + 128 * 16;      // Ritz values (16)
-constexpr int kPinSig = kPinLam + 16;          // preconditioner shifts (2 x 16)
+constexpr int kPinHsq = kPinCols + 128 * 128;  // |U_r|^2, then |r_r|^2 (2 x 16)
+constexpr int kPinLam = kPinHsq + 96;          // Ritz values (16)
+constexpr int kPinV = kPinLam + 16;            // Ritz coefficients, maxsub x nroots <= 128 x 16
+constexpr int kPinSig = kPinV + 128 * 16;      // preconditioner shifts (2 x 16)
 constexpr int kPinTotal = kPinSig + 32;
-static_assert(kRsq + 16 <= 96, "hsq region");
 
 pg_status ensure_scratch(pg_davidson* d, int ndim, int maxsub, int nroots, cudaStream_t st) {
   // grow-only scratch: a reused handle allocates only while its problems grow
@@ -342,94 +340,6 @@ pg_status ensure_scratch(pg_davidson* d, int ndim, int maxsub, int nroots, cudaS
   d->maxsub = maxsub;
   d->nroots = nroots;
   return PG_OK;
-}
-
-// Coefficients of one block Gram-Schmidt pass with the Pythagorean Gram (the
-// BCGS-PIP form): the corrections R (k vectors) sit right after the nb basis
-// vectors of B, and G holds the Gram products of [B R] against R,
-// G[a*k + j] = [B R]_a . R_j, so the first nb rows are C = B^T R and the last
-// k rows are R^T R.  With B orthonormal, (R - B C)^T (R - B C) = R^T R - C^T C,
-// whose Cholesky factor L gives U = L^-T; the pass is then one combine over
-// [B R] with coef[a*k + j] = -(C U)[a][j] for a < nb and U[a-nb][j] below.
-// A pivot is floored at 1e-24 of that vector's R^T R diagonal: where the
-// subtraction cancels (R almost inside span(B)) the pass yields scaled
-// rounding noise, mostly orthogonal to B, which the second pass (no
-// cancellation left) projects and normalises.  One block; k <= 16, nb <= 128.
-//
-// skip_out (first pass): 1 when every squared pivot L_jj^2 keeps at least
-// kPipKeep of that correction's squared norm R_j^T R_j, else 0.  Pivot j is
-// what remains of R_j after removing span(B) and the corrections before it;
-// with ratios that large the pass's rounding leaves the block orthonormal to
-// about u / kPipKeep (u: the unit roundoff of the products, 2^-53 in FP64,
-// about 2^-48 in double-float), and the second pass, which would change the
-// vectors only by that much, is skipped.  skip_in (second pass): return at
-// once when set.
-constexpr double kPipKeep = 1e-3;
-__global__ void __launch_bounds__(256) k_pip_coef(const double* __restrict__ G, int nb, int k,
-                                                  double* __restrict__ coef, int* __restrict__ skip_out,
-                                                  const int* __restrict__ skip_in) {
-  pdl_wait();
-  pdl_release();
-  if (skip_in && *skip_in) return;
-  __shared__ double Cs[128][kMaxCombine];
-  __shared__ double L[kMaxCombine][kMaxCombine + 1];
-  __shared__ double U[kMaxCombine][kMaxCombine + 1];
-  __shared__ int Keep[kMaxCombine];
-  const int tid = threadIdx.x;
-  for (int e = tid; e < nb * k; e += blockDim.x) Cs[e / k][e % k] = G[e];
-  __syncthreads();
-  if (tid < k * k) {  // R^T R - C^T C, each entry summed in basis order
-    const int i = tid / k, j = tid % k;
-    double s = G[(long)(nb + i) * k + j];
-    for (int a = 0; a < nb; ++a) s -= Cs[a][i] * Cs[a][j];
-    L[i][j] = s;
-  }
-  __syncthreads();
-  if (tid < 32) {
-    const int lane = tid;
-    for (int j = 0; j < k; ++j) {
-      if (lane == 0) {
-        double s = L[j][j];
-        for (int p = 0; p < j; ++p) s -= L[j][p] * L[j][p];
-        const double floor = 1e-24 * G[(long)(nb + j) * k + j];
-        const double piv = s > floor ? s : (floor > 1e-300 ? floor : 1e-300);
-        L[j][j] = sqrt(piv);
-        Keep[j] = piv >= kPipKeep * G[(long)(nb + j) * k + j];
-      }
-      __syncwarp();
-      if (lane > j && lane < k) {
-        double t = L[lane][j];
-        for (int p = 0; p < j; ++p) t -= L[lane][p] * L[j][p];
-        L[lane][j] = t / L[j][j];
-      }
-      __syncwarp();
-    }
-    if (skip_out && lane == 0) {
-      int all = 1;
-      for (int j = 0; j < k; ++j) all &= Keep[j];
-      *skip_out = all;
-    }
-    if (lane < k) {  // U = L^-T, column c on lane c (upper triangular)
-      const int c = lane;
-      for (int i = k - 1; i >= 0; --i) {
-        double s = i == c ? 1.0 : 0.0;
-        for (int p = i + 1; p < k; ++p) s -= L[p][i] * U[p][c];
-        U[i][c] = i > c ? 0.0 : s / L[i][i];
-      }
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < (nb + k) * k; e += blockDim.x) {
-    const int a = e / k, j = e % k;
-    double s;
-    if (a < nb) {
-      s = 0.0;
-      for (int i = 0; i <= j; ++i) s -= Cs[a][i] * U[i][j];
-    } else {
-      s = U[a - nb][j];
-    }
-    coef[e] = s;
-  }
 }
 
 // C = L^-T for the Cholesky factor of the k x k Gram matrix G (row-major,
@@ -554,7 +464,7 @@ namespace {
 // Orthonormalise the k vectors R (contiguous, R[j*N]) against the first nbas
 // columns of B and among themselves, into B[nbas .. nbas+k) (out must be
 // B + nbas*N; R is copied there first when it lives elsewhere).  Two passes of
-// block Gram-Schmidt with the Pythagorean Gram (k_pip_coef): one Gram over
+// block Gram-Schmidt with the Pythagorean Gram (pip_coef): one Gram over
 // [B R] against R, one coefficient kernel, one combine over [B R] in place.
 // The second pass repairs what the first leaves (rounding, or the cancellation
 // of a correction that lies almost inside span(B)).  Same spans as the
@@ -572,13 +482,11 @@ pg_status block_orthonormalise(pg_davidson* d, long N, double* R, int k, double*
   if (Bt) PG_TRY(split_twin(N * k, R, Rt, st, R != out ? out : nullptr));
   else if (R != out) PG_CUDA_TRY(cudaMemcpyAsync(out, R, sizeof(double) * N * k, cudaMemcpyDeviceToDevice, st));
   // the second pass runs only where the first one's pivots ask for it
-  // (k_pip_coef); the decision stays on the device
+  // (pip_coef); the decision stays on the device
   for (int pass = 0; pass < 2; ++pass) {
     const int* skip = pass == 1 ? d->pip_skip.p : nullptr;
-    PG_TRY(gram(N, B, nbas + k, out, k, d->dgram.p, d->rs, st, d->dfloat, Bt, Rt, skip));
-    PG_CUDA_TRY(launch_dependent(k_pip_coef, dim3(1), dim3(256), 0, st, d->dgram.p, nbas, k, d->dcoef.p,
-                                 pass == 0 ? d->pip_skip.p : nullptr, skip));
-    PG_TRY(check_launch("k_pip_coef"));
+    const PipPass pip{nbas, k, d->dcoef.p, pass == 0 ? d->pip_skip.p : nullptr};
+    PG_TRY(gram(N, B, nbas + k, out, k, d->dgram.p, d->rs, st, d->dfloat, Bt, Rt, skip, &pip));
     PG_TRY(combine(N, B, nbas + k, d->dcoef.p, k, 1, 1.0, nullptr, nullptr, false, out, k, nullptr, d->rs, st,
                    d->dfloat, Bt, Rt, skip));
   }
@@ -668,13 +576,12 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
       }
       for (int cb = 0; cb < nc; cb += per) {
         const int k = std::min(per, nc - cb);
-        PG_TRY(gram(N, Z, m, B + (long)(c0 + cb) * N, k, d->dcoef.p + (size_t)cb * m, d->rs, st, d->dfloat,
+        // straight into page-locked memory: no copy
+        PG_TRY(gram(N, Z, m, B + (long)(c0 + cb) * N, k, d->hpin.p + kPinCols + (size_t)cb * m, d->rs, st, d->dfloat,
                     d->dfloat ? d->zt.p : nullptr, d->dfloat ? d->bt.p + (long)(c0 + cb) * N : nullptr));
       }
       const double* cols = d->hpin.p + kPinCols;
       const auto w0 = std::chrono::steady_clock::now();
-      PG_CUDA_TRY(cudaMemcpyAsync(d->hpin.p + kPinCols, d->dcoef.p, sizeof(double) * m * nc, cudaMemcpyDeviceToHost,
-                                  st));
       PG_CUDA_TRY(cudaStreamSynchronize(st));
       d->t_wait += std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count();
       // gram output is [a*nb + b] per chunk: a = Z column i, b = new B column
@@ -703,26 +610,25 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
     }
     // Ritz vectors u = B v (renormalised) and residuals Z v - lambda u
     // (src/Davidson.cpp:240-269), all roots in one pass
-    double* dV = d->dcoef.p;
-    double* dlam = d->dsq.p + kLam;
+    double* dlam = d->dcoef.p;  // Ritz values and coefficients in one copy
+    double* dV = dlam + 16;
     double* usq = d->dsq.p + kUsq;
-    double* rsq = d->dsq.p + kRsq;
+    double* hsq = d->hpin.p + kPinHsq;  // the norms, written by the kernels
     memcpy(d->hpin.p + kPinV, d->V.data(), sizeof(double) * ms * nroots);
     memcpy(d->hpin.p + kPinLam, d->sse.data(), sizeof(double) * nroots);
-    PG_CUDA_TRY(cudaMemcpyAsync(dV, d->hpin.p + kPinV, sizeof(double) * ms * nroots, cudaMemcpyHostToDevice, st));
-    PG_CUDA_TRY(cudaMemcpyAsync(dlam, d->hpin.p + kPinLam, sizeof(double) * nroots, cudaMemcpyHostToDevice, st));
+    PG_CUDA_TRY(cudaMemcpyAsync(dlam, d->hpin.p + kPinLam, sizeof(double) * (16 + (size_t)ms * nroots),
+                                cudaMemcpyHostToDevice, st));
     if (d->dfloat) {
       // mixed form: both products, the residual and the norms in one pass
       // over the twins of B and Z (U is not renormalised: |U| = 1 to ~1e-14)
-      PG_TRY(ritz_df(N, d->bt.p, d->zt.p, m, dV, ms, dlam, ritz, res, nroots, usq, d->rs, st));
+      PG_TRY(ritz_df(N, d->bt.p, d->zt.p, m, dV, ms, dlam, ritz, res, nroots, hsq, d->rs, st));
     } else {
-      PG_TRY(combine(N, B, m, dV, 1, ms, 1.0, nullptr, nullptr, false, ritz, nroots, usq, d->rs, st));
-      PG_TRY(combine(N, Z, m, dV, 1, ms, 1.0, nullptr, nullptr, false, res, nroots, nullptr, d->rs, st));
+      PG_TRY(combine_pair(N, B, Z, m, dV, 1, ms, ritz, res, nroots, usq, d->rs, st));
       const long chunk = (N + kRedBlocks - 1) / kRedBlocks;
       const int nblk = (int)((N + chunk - 1) / chunk);
 #define PG_RITZ(NRV) \
   PG_CUDA_TRY(launch_dependent(k_ritz_residual<NRV>, dim3(nblk), dim3(kT), 0, st, N, chunk, nroots, ritz, res, \
-                               usq + nroots, dlam, d->rs.partial.p, rsq, d->rs.counter.p))
+                               usq, dlam, d->rs.partial.p, hsq, d->rs.counter.p))
       if (nroots <= 1) PG_RITZ(1);
       else if (nroots <= 2) PG_RITZ(2);
       else if (nroots <= 4) PG_RITZ(4);
@@ -731,14 +637,8 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
 #undef PG_RITZ
       PG_TRY(check_launch("k_ritz_residual"));
     }
-    // |r_r|^2 and |U_r|^2 in one read (rsq and usq both live in dsq; the
-    // mixed form's pass leaves |W_r|^2 right after |U_r|^2)
-    static_assert(kUsq == 0 && kRsq > kUsq, "dsq layout");
     const auto w1 = std::chrono::steady_clock::now();
-    PG_CUDA_TRY(cudaMemcpyAsync(d->hpin.p + kPinHsq, d->dsq.p, sizeof(double) * (kRsq + nroots),
-                                cudaMemcpyDeviceToHost, st));
-    const double* hr = d->hpin.p + kPinHsq + (d->dfloat ? kUsq + nroots : kRsq);
-    const double* hu = d->hpin.p + kPinHsq + kUsq;
+    const double *hu = hsq, *hr = hsq + nroots;  // |U_r|^2 and |r_r|^2
     PG_CUDA_TRY(cudaStreamSynchronize(st));
     d->t_wait += std::chrono::duration<double>(std::chrono::steady_clock::now() - w1).count();
     for (int r = 0; r < nroots; ++r) {

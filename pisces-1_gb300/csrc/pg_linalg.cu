@@ -27,12 +27,8 @@ long chunk_for(long N, int blocks, int align) {
 // out[o] = sum_b partial[b*no + o] over nb partial rows; one warp per output,
 // lanes stride over the rows, then a fixed shuffle tree.  inv_sqrt_out: also
 // store 1/sqrt(out[o]) at out[no + o] (used to normalise vectors on device).
-__global__ void __launch_bounds__(kT) k_reduce_partials(const double* __restrict__ partial, int nb, int no,
-                                                        double* __restrict__ out, int sqrt_mode,
-                                                        const int* __restrict__ skip) {
-  pdl_wait();
-  pdl_release();
-  if (skip && *skip) return;
+__device__ __forceinline__ void reduce_rows(const double* __restrict__ partial, int nb, int no, double* out,
+                                            int sqrt_mode) {
   const int warp = (blockIdx.x * kT + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= no) return;
@@ -53,6 +49,119 @@ __global__ void __launch_bounds__(kT) k_reduce_partials(const double* __restrict
     out[warp] = s;
     if (sqrt_mode) out[no + warp] = 1.0 / sqrt(s);
   }
+}
+__global__ void __launch_bounds__(kT) k_reduce_partials(const double* __restrict__ partial, int nb, int no,
+                                                        double* __restrict__ out, int sqrt_mode,
+                                                        const int* __restrict__ skip) {
+  pdl_wait();
+  pdl_release();
+  if (skip && *skip) return;
+  reduce_rows(partial, nb, no, out, sqrt_mode);
+}
+
+// Coefficients of one block Gram-Schmidt pass with the Pythagorean Gram (the
+// BCGS-PIP form): the corrections R (k vectors) sit right after the nb basis
+// vectors of B, and G holds the Gram products of [B R] against R,
+// G[a*k + j] = [B R]_a . R_j, so the first nb rows are C = B^T R and the last
+// k rows are R^T R.  With B orthonormal, (R - B C)^T (R - B C) = R^T R - C^T C,
+// whose Cholesky factor L gives U = L^-T; the pass is then one combine over
+// [B R] with coef[a*k + j] = -(C U)[a][j] for a < nb and U[a-nb][j] below.
+// A pivot is floored at 1e-24 of that vector's R^T R diagonal: where the
+// subtraction cancels (R almost inside span(B)) the pass yields scaled
+// rounding noise, mostly orthogonal to B, which the second pass (no
+// cancellation left) projects and normalises.  k <= 16, nb <= 128.
+//
+// skip_out (first pass): 1 when every squared pivot L_jj^2 keeps at least
+// kPipKeep of that correction's squared norm R_j^T R_j, else 0.  Pivot j is
+// what remains of R_j after removing span(B) and the corrections before it;
+// with ratios that large the pass's rounding leaves the block orthonormal to
+// about u / kPipKeep (u: the unit roundoff of the products, 2^-53 in FP64,
+// about 2^-48 in double-float), and the second pass, which would change the
+// vectors only by that much, is skipped.
+constexpr double kPipKeep = 1e-3;
+__device__ __forceinline__ void pip_coef(const double* G, int nb, int k, double* __restrict__ coef,
+                                         int* __restrict__ skip_out) {
+  __shared__ double Cs[128][kMaxCombine];
+  __shared__ double L[kMaxCombine][kMaxCombine + 1];
+  __shared__ double U[kMaxCombine][kMaxCombine + 1];
+  __shared__ int Keep[kMaxCombine];
+  __shared__ double Rd[kMaxCombine];  // R_j^T R_j
+  const int tid = threadIdx.x;
+  for (int e = tid; e < nb * k; e += blockDim.x) Cs[e / k][e % k] = __ldcg(G + e);
+  __syncthreads();
+  if (tid < k * k) {  // R^T R - C^T C, each entry summed in basis order
+    const int i = tid / k, j = tid % k;
+    double s = __ldcg(G + (long)(nb + i) * k + j);
+    if (i == j) Rd[j] = s;
+    for (int a = 0; a < nb; ++a) s -= Cs[a][i] * Cs[a][j];
+    L[i][j] = s;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    const int lane = tid;
+    for (int j = 0; j < k; ++j) {
+      if (lane == 0) {
+        double s = L[j][j];
+        for (int p = 0; p < j; ++p) s -= L[j][p] * L[j][p];
+        const double floor = 1e-24 * Rd[j];
+        const double piv = s > floor ? s : (floor > 1e-300 ? floor : 1e-300);
+        L[j][j] = sqrt(piv);
+        Keep[j] = piv >= kPipKeep * Rd[j];
+      }
+      __syncwarp();
+      if (lane > j && lane < k) {
+        double t = L[lane][j];
+        for (int p = 0; p < j; ++p) t -= L[lane][p] * L[j][p];
+        L[lane][j] = t / L[j][j];
+      }
+      __syncwarp();
+    }
+    if (skip_out && lane == 0) {
+      int all = 1;
+      for (int j = 0; j < k; ++j) all &= Keep[j];
+      *skip_out = all;
+    }
+    if (lane < k) {  // U = L^-T, column c on lane c (upper triangular)
+      const int c = lane;
+      for (int i = k - 1; i >= 0; --i) {
+        double s = i == c ? 1.0 : 0.0;
+        for (int p = i + 1; p < k; ++p) s -= L[p][i] * U[p][c];
+        U[i][c] = i > c ? 0.0 : s / L[i][i];
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < (nb + k) * k; e += blockDim.x) {
+    const int a = e / k, j = e % k;
+    double s;
+    if (a < nb) {
+      s = 0.0;
+      for (int i = 0; i <= j; ++i) s -= Cs[a][i] * U[i][j];
+    } else {
+      s = U[a - nb][j];
+    }
+    coef[e] = s;
+  }
+}
+
+// k_reduce_partials followed by pip_coef in the block that finishes last: one
+// launch between a pass's Gram product and its combine.
+__global__ void __launch_bounds__(kT) k_reduce_pip(const double* __restrict__ partial, int nb, int no, double* out,
+                                                   const int* __restrict__ skip, const PipPass pass,
+                                                   unsigned* counter) {
+  pdl_wait();
+  pdl_release();
+  if (skip && *skip) return;
+  reduce_rows(partial, nb, no, out, 0);
+  __shared__ int s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *counter = 0u;
+  pip_coef(out, pass.nb, pass.k, pass.coef, pass.skip_out);
 }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -140,17 +249,22 @@ __global__ void __launch_bounds__(kT, 2) k_gram(long N, long chunk, const double
 }
 
 template <int NR>
-__global__ void __launch_bounds__(kT) k_combine(long N, long chunk, const double* P, int na,
+__global__ void __launch_bounds__(kT) k_combine(long N, long chunk, const double* P, const double* P2, int na,
                                                 const double* __restrict__ C, int ca, int cr, double cscale,
                                                 const double* X,
-                                                const double* __restrict__ alpha, int inv_sqrt, double* Y, int nr,
-                                                double* __restrict__ partial, double* sq_out, unsigned* counter,
+                                                const double* __restrict__ alpha, int inv_sqrt, double* Y, double* Y2,
+                                                int nr, double* __restrict__ partial, double* sq_out, unsigned* counter,
                                                 const int* __restrict__ skip) {
   // no early release: blocks of the next kernel that take the free places of
   // some SMs would leave it uneven (back to back 96 x 4 over 110592 points,
   // on the FP64 pipe: 79 us, 100 with a release here)
   pdl_wait();
   if (skip && *skip) return;
+  if (blockIdx.y) {  // the second product of combine_pair
+    P = P2;
+    Y = Y2;
+    partial = nullptr;
+  }
   extern __shared__ double sm[];
   double* Cs = sm;                 // na x nr
   __shared__ double al[NR];
@@ -735,8 +849,13 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long
 
 // out[o] = sum of partial[b*no + o] over the nb rows, in a fixed order (k_reduce_partials)
 pg_status reduce(const double* partial, int nb, int no, double* out, bool sqrt_mode, cudaStream_t st,
-                 const int* skip = nullptr) {
+                 const int* skip = nullptr, const PipPass* pass = nullptr, unsigned* counter = nullptr) {
   const int blocks = (no * 32 + kT - 1) / kT;
+  if (pass) {
+    PG_CUDA_TRY(launch_dependent(k_reduce_pip, dim3(blocks), dim3(kT), 0, st, partial, nb, no, out, skip, *pass,
+                                 counter));
+    return check_launch("k_reduce_pip");
+  }
   PG_CUDA_TRY(launch_dependent(k_reduce_partials, dim3(blocks), dim3(kT), 0, st, partial, nb, no, out,
                                sqrt_mode ? 1 : 0, skip));
   return check_launch("k_reduce_partials");
@@ -805,7 +924,7 @@ static pg_status launch_gram(long N, long chunk, int blocks, const double* P, in
 }
 
 pg_status gram(long N, const double* P, int na, const double* Q, int nb, double* out, RedScratch& rs,
-               cudaStream_t st, bool dfloat, const double* Pt, const double* Qt, const int* skip) {
+               cudaStream_t st, bool dfloat, const double* Pt, const double* Qt, const int* skip, const PipPass* pass) {
   PG_ARG(na > 0 && nb > 0 && na * nb <= kMaxGramOut && na + nb <= 144, "gram: %d x %d outputs exceed the limits",
          na, nb);
   PG_TRY(rs.ensure(st));
@@ -827,11 +946,41 @@ pg_status gram(long N, const double* P, int na, const double* Q, int nb, double*
       PG_CUDA_TRY(launch_dependent(k_gram_df<false>, dim3(dblocks), dim3(kT), gg.smem, st, N, dchunk, Ps, na, Qs,
                                    nb, gg.tp, gg.m, gg.S, gg.ablk, gg.nblk, sp, sq, rs.partial.p, skip));
     PG_TRY(check_launch("k_gram_df"));
-    return reduce(rs.partial.p, dblocks, na * nb, out, false, st, skip);
+    return reduce(rs.partial.p, dblocks, na * nb, out, false, st, skip, pass, rs.counter.p);
   } else {
     PG_TRY(launch_gram(N, chunk, blocks, P, na, Q, nb, rs.partial.p, skip, st));
   }
-  return reduce(rs.partial.p, blocks, na * nb, out, false, st, skip);
+  return reduce(rs.partial.p, blocks, na * nb, out, false, st, skip, pass, rs.counter.p);
+}
+
+// k_combine over blocks of chunk points; with P2 also Y2 from P2 (its blocks beside the others)
+static pg_status launch_combine(long N, long chunk, int blocks, const double* P, const double* P2, int na,
+                                const double* C, int ca, int cr, double cscale, const double* X, const double* alpha,
+                                bool inv_sqrt, double* Y, double* Y2, int nr, double* sq, RedScratch& rs,
+                                cudaStream_t st, const int* skip) {
+  const size_t smem = sizeof(double) * (size_t)(na > 0 ? na : 1) * nr;
+#define PG_COMBINE(NRV)                                                                                             \
+  PG_CUDA_TRY(launch_dependent(k_combine<NRV>, dim3(blocks, P2 ? 2 : 1), dim3(kT), smem, st, N, chunk, P, P2, na, C, \
+                               ca, cr, cscale, X, alpha, inv_sqrt ? 1 : 0, Y, Y2, nr, sq ? rs.partial.p : nullptr, sq, \
+                               rs.counter.p, skip))
+  if (nr <= 1) PG_COMBINE(1);
+  else if (nr <= 2) PG_COMBINE(2);
+  else if (nr <= 4) PG_COMBINE(4);
+  else if (nr <= 8) PG_COMBINE(8);
+  else PG_COMBINE(16);
+#undef PG_COMBINE
+  return check_launch("k_combine");
+}
+
+pg_status combine_pair(long N, const double* P, const double* P2, int na, const double* C, int ca, int cr, double* Y,
+                       double* Y2, int nr, double* sq, RedScratch& rs, cudaStream_t st) {
+  PG_ARG(P && P2 && Y && Y2 && nr > 0 && nr <= kMaxCombine && na > 0 && na * nr <= 128 * kMaxCombine,
+         "combine_pair: bad sizes na=%d nr=%d", na, nr);
+  PG_TRY(rs.ensure(st));
+  const long chunk = chunk_for(N, kStreamBlocks, kT);
+  const int blocks = (int)((N + chunk - 1) / chunk);
+  return launch_combine(N, chunk, blocks, P, P2, na, C, ca, cr, 1.0, nullptr, nullptr, false, Y, Y2, nr, sq, rs, st,
+                        nullptr);
 }
 
 pg_status combine(long N, const double* P, int na, const double* C, int ca, int cr, double cscale, const double* X,
@@ -864,17 +1013,8 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
 #undef PG_COMBINE_DF3
     PG_TRY(check_launch("k_combine_df"));
   } else {
-    const size_t smem = sizeof(double) * (size_t)(na > 0 ? na : 1) * nr;
-#define PG_COMBINE(NRV)                                                                                           \
-  PG_CUDA_TRY(launch_dependent(k_combine<NRV>, dim3(blocks), dim3(kT), smem, st, N, chunk, P, na, C, ca, cr, cscale, X, \
-                               alpha, inv_sqrt ? 1 : 0, Y, nr, sq ? rs.partial.p : nullptr, sq, rs.counter.p, skip))
-    if (nr <= 1) PG_COMBINE(1);
-    else if (nr <= 2) PG_COMBINE(2);
-    else if (nr <= 4) PG_COMBINE(4);
-    else if (nr <= 8) PG_COMBINE(8);
-    else PG_COMBINE(16);
-#undef PG_COMBINE
-    PG_TRY(check_launch("k_combine"));
+    PG_TRY(launch_combine(N, chunk, blocks, P, nullptr, na, C, ca, cr, cscale, X, alpha, inv_sqrt, Y, nullptr, nr, sq,
+                          rs, st, skip));
   }
   return PG_OK;  // with sq, the kernel's last block has reduced the norms
 }

@@ -70,9 +70,22 @@ __device__ __forceinline__ void reduce_in_last_block(const double* partial, int 
 // skip (optional, device): when *skip is nonzero at the time the launches
 // run, they return at once and out is left as it was (a decision taken by an
 // earlier kernel on the same stream, without a device-to-host read).
+// pass (optional): P holds [B R] and Q = R, out is followed by the pass's
+// coefficients (PipPass), in the launch that reduces the partial sums.
+// out may be page-locked host memory (read after a synchronisation).
+struct PipPass {
+  int nb;         // basis vectors before R
+  int k;          // vectors of R
+  double* coef;   // (nb + k) x k
+  int* skip_out;  // first pass: 1 when the second is not needed
+};
 pg_status gram(long N, const double* P, int na, const double* Q, int nb, double* out, RedScratch& rs, cudaStream_t st,
                bool dfloat = false, const double* Pt = nullptr, const double* Qt = nullptr,
-               const int* skip = nullptr);
+               const int* skip = nullptr, const PipPass* pass = nullptr);
+
+// Y = P C with the norms sq, as combine, and Y2 = P2 C, FP64, in one launch.
+pg_status combine_pair(long N, const double* P, const double* P2, int na, const double* C, int ca, int cr, double* Y,
+                       double* Y2, int nr, double* sq, RedScratch& rs, cudaStream_t st);
 
 // Y[r*N + g] = alpha_r * X[r*N + g] + cscale * sum_a P[a*N + g] * C[a*ca + r*cr]   (r < nr <= kMaxCombine)
 // alpha_r: 0 if alpha is null; alpha[r] if inv_sqrt is false; 1/sqrt(alpha[r]) if true.
