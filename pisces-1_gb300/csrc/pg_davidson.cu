@@ -179,10 +179,13 @@ __global__ void k_jd_prep(long N, double* __restrict__ r, double* __restrict__ j
 // y_v(i,j,k) /= (dx_i + dy_j + dz_k - sigma_v), the denominator kept at
 // least `floor` in magnitude.  fast: the scale factor in FP32 (it only sets
 // the convergence rate; the mixed form uses it to stay off the FP64 pipe).
+struct Shifts {
+  double s[16];
+};
 template <int NR>
 __global__ void __launch_bounds__(kT) k_kin_scale(int nx, int ny, int nz, const double* __restrict__ dx,
                                                   const double* __restrict__ dy, const double* __restrict__ dz,
-                                                  const double* __restrict__ sigma, double floor,
+                                                  const Shifts sigma, double floor,
                                                   double* __restrict__ Y, int nvec, int fast) {
   // 32-bit index arithmetic (the grid has fewer than 2^31 points)
   const unsigned N = (unsigned)nx * ny * nz;
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(kT) k_kin_scale(int nx, int ny, int nz, const 
 #pragma unroll
       for (int v = 0; v < NR; ++v)
         if (v < nvec) {
-          float den = dk - (float)sigma[v];
+          float den = dk - (float)sigma.s[v];
           if (fabsf(den) < (float)floor) den = den < 0 ? -(float)floor : (float)floor;
           Y[(size_t)v * N + g] = y[v] * (double)(1.0f / den);
         }
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kT) k_kin_scale(int nx, int ny, int nz, const 
 #pragma unroll
       for (int v = 0; v < NR; ++v)
         if (v < nvec) {
-          double den = dk - sigma[v];
+          double den = dk - sigma.s[v];
           if (fabs(den) < floor) den = den < 0 ? -floor : floor;
           Y[(size_t)v * N + g] = y[v] / den;
         }
@@ -260,14 +263,12 @@ extern "C" pg_status pg_kinetic_precondition(const pg_grid* g, double* R, int k,
   if (k == 0) return PG_OK;
   PG_ARG(R && sigma, "pg_kinetic_precondition: null R or sigma");
   cudaStream_t st = pg::as_stream(stream);
-  // W1, W2 (each a multiple of 256 bytes) and sigma
+  // W1, W2 (each a multiple of 256 bytes); sigma goes with the launches
   const size_t wb = (sizeof(double) * k * (size_t)g->N + 255) / 256 * 256;
   pg::ScratchLease scratch(g, st);
   unsigned char* w = nullptr;
-  PG_TRY(scratch.get(2 * wb + sizeof(double) * k, &w));
-  double* sg = reinterpret_cast<double*>(w + 2 * wb);
-  PG_CUDA_TRY(cudaMemcpyAsync(sg, sigma, sizeof(double) * k, cudaMemcpyHostToDevice, st));
-  PG_TRY(pg::kinetic_precondition(g, R, k, sg, reinterpret_cast<double*>(w), reinterpret_cast<double*>(w + wb),
+  PG_TRY(scratch.get(2 * wb, &w));
+  PG_TRY(pg::kinetic_precondition(g, R, k, sigma, reinterpret_cast<double*>(w), reinterpret_cast<double*>(w + wb),
                                   precision, st));
   // waits for the stream: the scratch is the next call's
   return pg::check_tc_error(g, st);
@@ -304,7 +305,6 @@ namespace {
 constexpr int kUsq = 0;     // |U_r|^2 and 1/|U_r| (2 x 16, FP64 form)
 constexpr int kOnes = 96;   // 1.0 (16), the "keep X" coefficients of combine
 constexpr int kDots = 112;  // Jacobi-Davidson dot products (2)
-constexpr int kSigma = 128; // shifts of the kinetic preconditioner (2 x 16)
 constexpr int kScalars = 256;
 
 // Regions of pg_davidson::hpin (doubles)
@@ -312,8 +312,7 @@ constexpr int kPinCols = 0;                    // new S columns, m x nc <= 128 x
 constexpr int kPinHsq = kPinCols + 128 * 128;  // |U_r|^2, then |r_r|^2 (2 x 16)
 constexpr int kPinLam = kPinHsq + 96;          // Ritz values (16)
 constexpr int kPinV = kPinLam + 16;            // Ritz coefficients, maxsub x nroots <= 128 x 16
-constexpr int kPinSig = kPinV + 128 * 16;      // preconditioner shifts (2 x 16)
-constexpr int kPinTotal = kPinSig + 32;
+constexpr int kPinTotal = kPinV + 128 * 16;
 
 pg_status ensure_scratch(pg_davidson* d, int ndim, int maxsub, int nroots, cudaStream_t st) {
   // grow-only scratch: a reused handle allocates only while its problems grow
@@ -412,11 +411,11 @@ __global__ void k_olsen_coef(const double* __restrict__ G, int k, double* __rest
   }
 }
 
-pg_status kinetic_precondition(pg_davidson* d, double* R, int k, const double* sigma_dev, cudaStream_t st) {
+pg_status kinetic_precondition(pg_davidson* d, double* R, int k, const double* sigma, cudaStream_t st) {
   const long N = d->pc_grid->N;
   PG_TRY(d->pc_w1.ensure((size_t)k * N));
   PG_TRY(d->pc_w2.ensure((size_t)k * N));
-  return pg::kinetic_precondition(d->pc_grid, R, k, sigma_dev, d->pc_w1.p, d->pc_w2.p, d->pc_precision, st,
+  return pg::kinetic_precondition(d->pc_grid, R, k, sigma, d->pc_w1.p, d->pc_w2.p, d->pc_precision, st,
                                   d->nroots > 1);
 }
 
@@ -428,22 +427,24 @@ pg_status kinetic_precondition(pg_davidson* d, double* R, int k, const double* s
 // (Q^T), a diagonal scale and three backward contractions (Q).  The mixed
 // form runs them as one FP16-split tensor-core kernel where the grid allows
 // (k_kin_f16), else as six axis passes and a scale kernel.
-pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double* sigma_dev, double* w1, double* w2,
+pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double* sigma, double* w1, double* w2,
                                int pr, cudaStream_t st, bool in_order) {
   const long N = g->N;
   // the smallest kinetic level, a scale for the denominator floor
   double dmin = 0;
   for (int a = 0; a < 3; ++a) dmin += 0.5 * (M_PI / g->L[a]) * (M_PI / g->L[a]);
   if (pr == PG_MIXED && g->pc_kernel != 1 && kin_f16_ok(g) && (((uintptr_t)R | (uintptr_t)w1 | (uintptr_t)w2) & 15u) == 0)
-    return kin_f16(g, R, w1, w2, k, sigma_dev, 0.1 * dmin, st);
+    return kin_f16(g, R, w1, w2, k, sigma, 0.1 * dmin, st);
   PG_TRY(axis_apply(g, 2, g->q_sl[2], g->q_dev[2].p, g->q_hi[2].p, g->q_lo[2].p, R, w1, k, 0, pr, st, in_order));
   PG_TRY(axis_apply(g, 1, g->q_sl[1], g->q_dev[1].p, g->q_hi[1].p, g->q_lo[1].p, w1, w2, k, 0, pr, st, in_order));
   PG_TRY(axis_apply(g, 0, g->q_sl[0], g->q_dev[0].p, g->q_hi[0].p, g->q_lo[0].p, w2, w1, k, 0, pr, st, in_order));
   for (int v0 = 0; v0 < k; v0 += 16) {  // at most 16 vectors per launch
     const int kk = std::min(16, k - v0);
+    Shifts sh{};
+    std::copy(sigma + v0, sigma + v0 + kk, sh.s);
 #define PG_KIN_SCALE(NRV)                                                                                     \
   k_kin_scale<NRV><<<blocks_for(N), kT, 0, st>>>(g->n[0], g->n[1], g->n[2], g->d_dev[0].p, g->d_dev[1].p,      \
-                                                 g->d_dev[2].p, sigma_dev + v0, 0.1 * dmin, w1 + (long)v0 * N, \
+                                                 g->d_dev[2].p, sh, 0.1 * dmin, w1 + (long)v0 * N, \
                                                  kk, pr == PG_MIXED ? 1 : 0)
     if (kk <= 1) PG_KIN_SCALE(1);
     else if (kk <= 2) PG_KIN_SCALE(2);
@@ -788,11 +789,9 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
     d->nnewB = (int)sel.size();
     if (corrflag == 3 && d->nnewB > 0 && !d->pc_olsen) {
       // exact-kinetic correction M r_j, M = (T - lambda_j)^-1
-      double* sig = d->hpin.p + kPinSig;
+      double sig[kMaxCombine];
       for (int j = 0; j < d->nnewB; ++j) sig[j] = d->sse[sel[j]];
-      double* dsig = d->dsq.p + kSigma;
-      PG_CUDA_TRY(cudaMemcpyAsync(dsig, sig, sizeof(double) * d->nnewB, cudaMemcpyHostToDevice, st));
-      PG_TRY(kinetic_precondition(d, res, d->nnewB, dsig, st));
+      PG_TRY(kinetic_precondition(d, res, d->nnewB, sig, st));
     } else if (corrflag == 3 && d->nnewB > 0) {
       // Olsen correction with M = (T - lambda_j)^-1 applied exactly:
       // c_j = -M r_j + (u_j.M r_j / u_j.M u_j) M u_j, orthogonal to u_j.  With
@@ -808,11 +807,9 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
         PG_CUDA_TRY(cudaMemcpyAsync(RU + (long)(k + j) * N, u, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
       }
       PG_CUDA_TRY(cudaMemcpyAsync(Uc, RU + (long)k * N, sizeof(double) * N * k, cudaMemcpyDeviceToDevice, st));
-      double* sig = d->hpin.p + kPinSig;
+      double sig[2 * kMaxCombine];
       for (int j = 0; j < k; ++j) sig[j] = sig[k + j] = d->sse[sel[j]];
-      double* dsig = d->dsq.p + kSigma;
-      PG_CUDA_TRY(cudaMemcpyAsync(dsig, sig, sizeof(double) * 2 * k, cudaMemcpyHostToDevice, st));
-      PG_TRY(kinetic_precondition(d, RU, 2 * k, dsig, st));  // RU = [M R, M U]
+      PG_TRY(kinetic_precondition(d, RU, 2 * k, sig, st));  // RU = [M R, M U]
       PG_TRY(gram(N, Uc, k, RU, 2 * k, d->dgram.p, d->rs, st, d->dfloat));
       k_olsen_coef<<<1, 256, 0, st>>>(d->dgram.p, k, d->dcoef.p);
       PG_TRY(check_launch("k_olsen_coef"));

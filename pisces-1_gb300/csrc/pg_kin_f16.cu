@@ -98,7 +98,7 @@ struct KinArgs {
   double* r;
   double* w1;
   double* w2;
-  const double* sigma;  // per vector
+  double sigma[kKinMaxVec];  // per vector
   const double* d[3];   // eigenvalues per axis
 };
 
@@ -899,7 +899,8 @@ void kin_f16_plan_text(const pg_grid* g, char* buf, int len) {
 }
 
 // R <- (T - sigma_v)^-1 R for the k vectors of R (contiguous, 16-byte
-// aligned), with W1 and W2 k vectors of scratch each; sigma on the device.
+// aligned), with W1 and W2 k vectors of scratch each; sigma on the host (it goes with the
+// launch).
 pg_status kin_f16(const pg_grid* g, double* R, double* w1, double* w2, int k, const double* sigma, double floor,
                   cudaStream_t st) {
   PG_ARG(k >= 0 && R && w1 && w2 && sigma && floor > 0.0, "FP16 preconditioner: bad arguments");
@@ -930,7 +931,7 @@ pg_status kin_f16(const pg_grid* g, double* R, double* w1, double* w2, int k, co
     A.r = R + (long)v0 * N;
     A.w1 = w1;
     A.w2 = w2;
-    A.sigma = sigma + v0;
+    std::copy(sigma + v0, sigma + v0 + nb, A.sigma);
     for (int a = 0; a < 3; ++a) A.d[a] = g->d_dev[a].p;
     P.G.nvec = nb;
     // steps between a vector's phases: three keep enough independent planes
