@@ -269,20 +269,22 @@ using pg::TcJobs;
 
 template <int AXIS, int TH>
 __global__ void __launch_bounds__(TH, kThreads / TH)
-    k_hx_tc(int nx, int ny, int nz, AxisMap am, int npad, int kc, int nch, uint32_t tmem_cols,
+    k_hx_tc(int nx, int ny, int nz, AxisMap am, int npad, int kb, int kc, int nch, uint32_t tmem_cols,
             const float* __restrict__ t_hi, const float* __restrict__ t_lo, const __grid_constant__ TcJobs jobs,
             int mode, uint32_t stage_off, int* __restrict__ err) {
   // mode 0: Y = D;  1: Y += D;  2: Y = V X + D   (D = the axis contraction)
   // stage_off (AXIS 0): byte offset of the 16 warps' epilogue blocks in the
   // dynamic shared memory (it may overlap the A tile, free by then), or
   // kNoStage
-  // K is processed in nch chunks of kc (one chunk for n <= 112): per chunk the
-  // A tile and the B chunk are staged, multiplied into the same accumulator,
-  // and the shared memory is reused once those MMAs have completed.
+  // K is processed in nch chunks of kc: per chunk the A tile and the B chunk
+  // are staged, multiplied into the same accumulator, and the shared memory is
+  // reused once those MMAs have completed.  kb > kc: B is one image of kb
+  // values and stays (one chunk, or A alone in chunks).
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr bool kAhead = TH == kHalfThreads;
   const int n = am.n;
-  const uint32_t b_bytes = (uint32_t)npad * kc * 4;  // one K chunk of one half of B
+  const bool stays = nch == 1 || kb > kc;  // B
+  const uint32_t b_bytes = (uint32_t)npad * kb * 4;  // one K chunk of one half of B
   const uint32_t a_bytes = (uint32_t)kTileM * kc * 4;
   unsigned char* sBh = smem;
   unsigned char* sBl = smem + b_bytes;
@@ -306,11 +308,11 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
                  : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      smem_u32(sBh)),
-                 "l"(t_hi + (size_t)ch * npad * kc), "r"(b_bytes), "r"(smem_u32(&mbar_b))
+                 "l"(t_hi + (size_t)ch * npad * kb), "r"(b_bytes), "r"(smem_u32(&mbar_b))
                  : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      smem_u32(sBl)),
-                 "l"(t_lo + (size_t)ch * npad * kc), "r"(b_bytes), "r"(smem_u32(&mbar_b))
+                 "l"(t_lo + (size_t)ch * npad * kb), "r"(b_bytes), "r"(smem_u32(&mbar_b))
                  : "memory");
   };
   if (tid == 0) {
@@ -335,13 +337,13 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
   const uint32_t tmem = tmem_base;
   const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(npad >> 3) << 17) |
                          ((uint32_t)(kTileM >> 4) << 24);
-  const uint32_t lbo = 128, sbo = (uint32_t)(kc >> 2) * 128;
+  const uint32_t lbo = 128, sbo = (uint32_t)(kc >> 2) * 128, sbo_b = (uint32_t)(kb >> 2) * 128;
   const int warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3;      // TMEM lanes 32*quarter .. +31
   const int group = warp >> 2;       // which 16-column chunks this warp reads (every kThreads/128-th)
   uint32_t phase = 0, b_phase = 0;
   bool ok = true;
-  bool b_ready = false;   // single chunk: B resident
+  bool b_ready = false;   // B is here to stay
   bool first = true;      // the first chunk's B load was issued above
 
   for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
     if (kAhead) ahead.load(xv, 0, 0, kc >> 2, n, am.stride);
     for (int ch = 0; ch < nch; ++ch) {
       const int k0 = ch * kc;
-      if (nch > 1 && !first && tid == 0) load_b(ch);  // the previous chunk's MMAs have completed
+      if (!stays && !first && tid == 0) load_b(ch);  // the previous chunk's MMAs have completed
       first = false;
       // ---- A operand: 128 columns x kc, split into TF32 hi/lo
       if (kAhead) ahead.store(xv, 0, kc >> 2, sAh, sAl);
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       bool bok = true;
-      if (nch > 1 || !b_ready) {  // this chunk's B images have landed
+      if (!stays || !b_ready) {  // this chunk's B images have landed
         bok = mbar_wait(smem_u32(&mbar_b), b_phase);
         b_phase ^= 1u;
         b_ready = true;
@@ -379,11 +381,13 @@ __global__ void __launch_bounds__(TH, kThreads / TH)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (tid == 0) {
-        const uint32_t ah = smem_u32(sAh), al = smem_u32(sAl), bh = smem_u32(sBh), bl = smem_u32(sBl);
-        for (int kk = 0; kk < kc / 8; ++kk) {
+        const uint32_t b0 = kb > kc ? (uint32_t)k0 * 32u : 0u;  // this chunk's place in B
+        const uint32_t ah = smem_u32(sAh), al = smem_u32(sAl), bh = smem_u32(sBh) + b0, bl = smem_u32(sBl) + b0;
+        const int steps = (kb > kc && kb - k0 < kc ? kb - k0 : kc) / 8;
+        for (int kk = 0; kk < steps; ++kk) {
           const uint32_t off = (uint32_t)kk * 256;  // 8 K-elements = two core matrices
           const uint64_t dah = smem_desc(ah + off, lbo, sbo), dal = smem_desc(al + off, lbo, sbo);
-          const uint64_t dbh = smem_desc(bh + off, lbo, sbo), dbl = smem_desc(bl + off, lbo, sbo);
+          const uint64_t dbh = smem_desc(bh + off, lbo, sbo_b), dbl = smem_desc(bl + off, lbo, sbo_b);
           const uint32_t acc = (ch > 0 || kk > 0) ? 1u : 0u;
           // small terms first, then the leading product
           asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -732,12 +736,28 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
   // 2.25 -> 1.18 ms together with the x epilogue's loads apart from their
   // product, 1.34 without the loads ahead; with one tile per SM or fewer the wide
   // CTA is faster, 128x64x40 x 3: 55 us against 60)
-  const bool half = nch > 1 && tiles > cap && kc <= 2 * kHalfBatch;
+  // One K chunk and one to two tiles per SM: the same with B resident and A in
+  // chunks of at most 48 values, where both fit 112 KB (n <= 96), so that all
+  // tiles are under way at once; the pipelined form would take two turns
+  // (three passes, us, pipelined / so: 64x64x72 x 5 65.0 / 54.8, 88x90x88 x 4
+  // 82.3 / 72.8, 48x52x50 x 10 56.0 / 51.2).  With more tiles its turns overlap
+  // and it is as fast or faster (88x90x88 x 7 120 / 143, 64x64x72 x 12 88 / 94).
+  int ka = kc, na = nch;
+  if (nch == 1 && form == 0 && ctas <= 0 && tiles > cap && tiles <= 2 * cap) {
+    const long left = 112 * 1024 - (long)2 * npad * kc * 4;
+    const int most = (int)std::min<long>(2 * kHalfBatch, left > 0 ? left / (2 * kTileM * 4) / 8 * 8 : 0);
+    if (most >= 24) {
+      na = (kpad + most - 1) / most;
+      ka = ((kpad + na - 1) / na + 7) / 8 * 8;
+    }
+  }
+  const bool resident = na > 1 && nch == 1;
+  const bool half = resident || (nch > 1 && tiles > cap && kc <= 2 * kHalfBatch);
   const int grid = (int)std::min<long>(tiles, half ? 2 * cap : cap);
   int* err = g->tc_err.p;
-  const size_t a_region = (size_t)2 * kTileM * kc * 4, b_region = (size_t)2 * npad * kc * 4;
+  const size_t a_region = (size_t)2 * kTileM * ka * 4, b_region = (size_t)2 * npad * kc * 4;
   // several tiles per CTA: the pipelined form overlaps them (form 0), or as tuned
-  const bool pipe = nch == 1 && (form == 2 || (form == 0 && tiles > cap));
+  const bool pipe = nch == 1 && !resident && (form == 2 || (form == 0 && tiles > cap));
   if (pipe) {
     // x-axis epilogue blocks of the eight consumer warps after the A tile
     const size_t stage = (size_t)(kPipeThreads - kProducers) / 32 * kStageWarpBytes;
@@ -764,20 +784,20 @@ pg_status tc_axis_jobs(const pg_grid* g, int a, const float* Ahi, const float* A
   const int th = half ? kHalfThreads : kThreads;
   const size_t stage = (size_t)th / 32 * kStageWarpBytes;
   uint32_t stage_off = kNoStage;
-  size_t smem_t = smem;
+  size_t smem_t = a_region + b_region;
   if (a == 0) {
     if (a_region >= stage) {
       stage_off = (uint32_t)b_region;
-    } else if (smem + stage <= (size_t)g_max_dyn) {
-      stage_off = (uint32_t)smem;
-      smem_t = smem + stage;
+    } else if (smem_t + stage <= (size_t)g_max_dyn) {
+      stage_off = (uint32_t)smem_t;
+      smem_t += stage;
     }
   }
   const auto k = half ? (a == 0   ? k_hx_tc<0, kHalfThreads>
                          : a == 1 ? k_hx_tc<1, kHalfThreads>
                                   : k_hx_tc<2, kHalfThreads>)
                       : (a == 0 ? k_hx_tc<0, kThreads> : a == 1 ? k_hx_tc<1, kThreads> : k_hx_tc<2, kThreads>);
-  PG_CUDA_TRY(launch_dependent(k, dim3(grid), dim3(th), smem_t, st, g->n[0], g->n[1], g->n[2], am, npad, kc, nch, cols,
+  PG_CUDA_TRY(launch_dependent(k, dim3(grid), dim3(th), smem_t, st, g->n[0], g->n[1], g->n[2], am, npad, kc, ka, na, cols,
                                Ahi, Alo, jobs, mode, stage_off, err));
   return check_launch("k_hx_tc");
 }
