@@ -590,14 +590,18 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   a.tmem_cols = 32;
   while (a.tmem_cols < (uint32_t)(kSliceAcc * S.nc)) a.tmem_cols <<= 1;
   if (!chunks) a.tmem_cols <<= 1;  // two sets
-  // Few lines: fewer per CTA (the digits and the read-out are shared among
-  // more SMs; the products cost the same), then the N chunks of a tile to CTAs
-  // of their own.
+  // Few lines: the N chunks of a tile go to CTAs of their own, then fewer lines
+  // to a CTA, as long as there is an SM for each.  In this order: a CTA's
+  // read-out takes as long for 32 lines as for 128 (TMEM lanes belong to one
+  // scheduler's warps), its digits do not (64^3 x 1: 44 us with the lines
+  // first, 34 so; 80^3 x 1 62 / 48, 160x60x60 x 1 91 / 63).
+  const long full = (nlines + kLines - 1) / kLines;
+  const int groups = (int)std::max<long>(1, std::min<long>(S.nnc, 152 / full));
+  a.nc_per = (S.nnc + groups - 1) / groups;
+  const int split = (S.nnc + a.nc_per - 1) / a.nc_per;
   a.lc = kLines;
-  while (a.lc > 32 && (nlines + a.lc / 2 - 1) / (a.lc / 2) <= 152) a.lc /= 2;
+  while (a.lc > 32 && (nlines + a.lc / 2 - 1) / (a.lc / 2) * split <= 152) a.lc /= 2;
   const long tiles = (nlines + a.lc - 1) / a.lc;
-  const int split = tiles * S.nnc <= 152 ? S.nnc : 1;
-  a.nc_per = (S.nnc + split - 1) / split;
   const dim3 grid((unsigned)tiles, (unsigned)split);
   // at most two K chunks (160 values) per launch, so that the sums of one
   // accumulator stay below 2^24; a longer axis adds up in Y

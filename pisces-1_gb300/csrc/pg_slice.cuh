@@ -97,13 +97,12 @@ __device__ __forceinline__ double slice_join(const float* acc, int e) {
   uint32_t l = ((uint32_t)lo & ((1u << (3 * kSliceP)) - 1u)) << (32 - 3 * kSliceP);
   uint32_t w2 = (uint32_t)((unsigned long long)hi >> 32) ^ sgn, w1 = (uint32_t)hi ^ sgn, w0 = l ^ sgn;
   int ex = e + 1023 + 63 + 3 * kSliceP;
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const bool up = w2 == 0;
-    ex -= up ? 32 : 0;
-    w2 = up ? w1 : w2;
-    w1 = up ? w0 : w1;
-    w0 = up ? 0u : w0;
+  if (w2 == 0) {  // small against the line's largest value
+    const bool two = w1 == 0;
+    ex -= two ? 64 : 32;
+    w2 = two ? w0 : w1;
+    w1 = two ? 0u : w0;
+    w0 = 0u;
   }
   const int lz = __clz((int)w2);
   ex -= lz;

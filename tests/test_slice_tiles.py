@@ -14,11 +14,12 @@ pytestmark = pytest.mark.gpu
 LD = np.longdouble
 
 
-# lines of the first axis: 10000 (128 a tile, 2 column chunks), 10224 (6
-# chunks), 19200 (3), 10000 (K chunks), 9728 (64 a tile) and 9792 (128), 4864
-# (32) and 4896 (64)
+# many lines: tiles of 128 on every axis, or of 64 and 32 on the short ones;
+# then fewer, where a tile's column chunks go to blocks of their own (64, 96
+# with two chunks to a block, 160 in K chunks too)
 @pytest.mark.parametrize("n,nvec", [((17, 100, 100), 1), ((96, 72, 71), 2), ((80, 80, 80), 3), ((97, 50, 200), 1),
-                                    ((33, 64, 152), 1), ((33, 64, 153), 1), ((50, 64, 76), 1), ((50, 48, 102), 1)])
+                                    ((33, 64, 152), 1), ((33, 64, 153), 1), ((50, 64, 76), 1), ((50, 48, 102), 1),
+                                    ((64, 64, 64), 1), ((96, 60, 80), 1), ((160, 48, 50), 1)])
 def test_hx_fp64_over_many_lines(pg, n, nvec):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(n[0] * 1000 + n[2])
