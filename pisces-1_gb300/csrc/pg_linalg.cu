@@ -787,8 +787,9 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long
   if (skip && *skip) return;
   extern __shared__ __align__(16) float smf[];
   float* Cs = smf;  // [row][pair]: (hi, hi, lo, lo); NR 1: [row] (hi, lo)
+  constexpr int NS = NR == 6 ? 8 : (NR > 8 ? 16 : NR);  // norms: a power of two
   __shared__ float alh[NR], all[NR];
-  __shared__ double red[kT / 32][NR];
+  __shared__ double red[kT / 32][NS];
   load_coefs<NR>(Cs, na, nr, [&](int a, int r) { return cscale * C[(long)a * ca + (long)r * cr]; });
   if (threadIdx.x < nr) {
     double a = 0;
@@ -799,9 +800,9 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long
     all[threadIdx.x] = l;
   }
   __syncthreads();
-  double sacc[NR];
+  double sacc[NS];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) sacc[r] = 0;
+  for (int r = 0; r < NS; ++r) sacc[r] = 0;
   const bool keep = X && alpha;
   const long g_begin = blockIdx.x * chunk;
   const long g_end = g_begin + chunk < N ? g_begin + chunk : N;
@@ -863,8 +864,8 @@ __global__ void __launch_bounds__(kT, NR <= 4 ? 4 : 2) k_combine_df(long N, long
   }
   if (!partial) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  packed_sums<NR, 1>(sacc, lane);
-  if (lane % (32 / NR) == 0) red[warp][lane / (32 / NR)] = sacc[0];
+  packed_sums<NS, 1>(sacc, lane);
+  if (lane % (32 / NS) == 0) red[warp][lane / (32 / NS)] = sacc[0];
   __syncthreads();
   if (threadIdx.x < nr) {
     double s = 0;
@@ -986,15 +987,33 @@ static pg_status launch_combine(long N, long chunk, int blocks, const double* P,
                                 bool inv_sqrt, double* Y, double* Y2, int nr, double* sq, RedScratch& rs,
                                 cudaStream_t st, const int* skip) {
   const size_t smem = sizeof(double) * (size_t)(na > 0 ? na : 1) * nr;
+  // one kernel per number of outputs: an operation left out by a predicate
+  // takes the FP64 pipe as long as any other (64 x 12 over 262144 points 570 us
+  // as 16 outputs, 397 as 12; 40 x 5 186 as 8, 94 as 5)
 #define PG_COMBINE(NRV)                                                                                             \
-  PG_CUDA_TRY(launch_dependent(k_combine<NRV>, dim3(blocks, P2 ? 2 : 1), dim3(kT), smem, st, N, chunk, P, P2, na, C, \
-                               ca, cr, cscale, X, alpha, inv_sqrt ? 1 : 0, Y, Y2, nr, sq ? rs.partial.p : nullptr, sq, \
-                               rs.counter.p, skip))
-  if (nr <= 1) PG_COMBINE(1);
-  else if (nr <= 2) PG_COMBINE(2);
-  else if (nr <= 4) PG_COMBINE(4);
-  else if (nr <= 8) PG_COMBINE(8);
-  else PG_COMBINE(16);
+  case NRV:                                                                                                         \
+    PG_CUDA_TRY(launch_dependent(k_combine<NRV>, dim3(blocks, P2 ? 2 : 1), dim3(kT), smem, st, N, chunk, P, P2, na, \
+                                 C, ca, cr, cscale, X, alpha, inv_sqrt ? 1 : 0, Y, Y2, nr,                          \
+                                 sq ? rs.partial.p : nullptr, sq, rs.counter.p, skip));                             \
+    break
+  switch (nr) {
+    PG_COMBINE(1);
+    PG_COMBINE(2);
+    PG_COMBINE(3);
+    PG_COMBINE(4);
+    PG_COMBINE(5);
+    PG_COMBINE(6);
+    PG_COMBINE(7);
+    PG_COMBINE(8);
+    PG_COMBINE(9);
+    PG_COMBINE(10);
+    PG_COMBINE(11);
+    PG_COMBINE(12);
+    PG_COMBINE(13);
+    PG_COMBINE(14);
+    PG_COMBINE(15);
+    PG_COMBINE(16);
+  }
 #undef PG_COMBINE
   return check_launch("k_combine");
 }
@@ -1034,7 +1053,10 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
     if (nr <= 1) PG_COMBINE_DF(1);
     else if (nr <= 2) PG_COMBINE_DF(2);
     else if (nr <= 4) PG_COMBINE_DF(4);
+    else if (nr <= 6) PG_COMBINE_DF(6);
     else if (nr <= 8) PG_COMBINE_DF(8);
+    else if (nr <= 10) PG_COMBINE_DF(10);
+    else if (nr <= 12) PG_COMBINE_DF(12);
     else PG_COMBINE_DF(16);
 #undef PG_COMBINE_DF
 #undef PG_COMBINE_DF3

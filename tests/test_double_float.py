@@ -68,3 +68,17 @@ def test_block_products_mixed_tiles(pg, rows, n):
     ref = np.stack([(C[:, r][:, None].astype(LD) * P.astype(LD)).sum(axis=0) for r in range(rows[1])])
     mag = np.stack([abs(C[:, r][:, None] * P).sum(axis=0) for r in range(rows[1])])
     assert np.all(abs(y.cpu().numpy().reshape(ref.shape) - ref) <= 150 * 2.0 ** -47 * mag)
+
+
+@pytest.mark.parametrize("nr", range(1, 17))
+@pytest.mark.parametrize("precision", [0, 1])
+def test_combine_columns_do_not_depend_on_their_number(pg, nr, precision):
+    """A column of a block combine has the bits of the same column on its own (each count of columns has a kernel)."""
+    torch = pytest.importorskip("torch")
+    gen = torch.Generator(device="cuda").manual_seed(nr)
+    P = torch.randn(19, 5003, dtype=torch.float64, device="cuda", generator=gen)
+    C = torch.randn(19, nr, dtype=torch.float64, device="cuda", generator=gen)
+    y = pg.block_combine(P, C, precision=precision).reshape(nr, -1)
+    for r in {0, nr // 2, nr - 1}:
+        one = pg.block_combine(P, C[:, r:r + 1].contiguous(), precision=precision).reshape(-1)
+        assert torch.equal(y[r], one)
