@@ -448,6 +448,7 @@ pg_status kinetic_precondition(const pg_grid* g, double* R, int k, const double*
                                                  kk, pr == PG_MIXED ? 1 : 0)
     if (kk <= 1) PG_KIN_SCALE(1);
     else if (kk <= 2) PG_KIN_SCALE(2);
+    else if (kk <= 3) PG_KIN_SCALE(3);
     else if (kk <= 4) PG_KIN_SCALE(4);
     else if (kk <= 8) PG_KIN_SCALE(8);
     else PG_KIN_SCALE(16);
@@ -632,6 +633,7 @@ extern "C" pg_status pg_davidson_rci(pg_davidson* d, int ndim, int maxsub, int n
                                usq, dlam, d->rs.partial.p, hsq, d->rs.counter.p))
       if (nroots <= 1) PG_RITZ(1);
       else if (nroots <= 2) PG_RITZ(2);
+      else if (nroots <= 3) PG_RITZ(3);
       else if (nroots <= 4) PG_RITZ(4);
       else if (nroots <= 8) PG_RITZ(8);
       else PG_RITZ(16);
