@@ -110,6 +110,7 @@ pg_status check_model(const char* who, const pg_sites* t, const pg_scpol_model* 
 // polarisable sites, Epc, A and A's digit images.
 struct ModelDev {
   const double *pos = nullptr, *epc = nullptr, *inva = nullptr;
+  std::vector<double> pos_host;
   pg::SliceMat mat;
   size_t img_bytes = 0;
   static size_t up(size_t b) { return (b + 255) / 256 * 256; }
@@ -124,10 +125,13 @@ struct ModelDev {
     img_bytes = pg::slice_rows_shape(n, finite ? big : INFINITY, &mat);
     return up(img_bytes) + 2 * up(sizeof(double) * n) + up(sizeof(double) * n * n);
   }
-  // the host arrays may be released once the call has waited for the stream
+  // The copies are queued: this struct and the caller's arrays are to outlive
+  // a wait for the stream (a copy from pageable memory may read its source
+  // until then), on error returns too.
   pg_status upload(const pg_sites* t, const pg_scpol_model* m, unsigned char* buf, cudaStream_t st) {
     const int n = 3 * m->npp;
-    std::vector<double> p(n);
+    std::vector<double>& p = pos_host;
+    p.resize(n);
     for (int i = 0; i < m->npp; ++i)
       for (int c = 0; c < 3; ++c) p[3 * i + c] = t->sites[3 * m->pol_site[i] + c];
     double* d = reinterpret_cast<double*>(buf + up(img_bytes));
@@ -142,6 +146,12 @@ struct ModelDev {
     PG_TRY(pg::slice_rows_matrix(inva, buf, &mat, st));
     return PG_OK;
   }
+};
+
+// Waits for the stream when a call ends, whichever way.
+struct WaitOnExit {
+  cudaStream_t st;
+  ~WaitOnExit() { cudaStreamSynchronize(st); }
 };
 
 long chunk_points(long N, int n) {
@@ -433,6 +443,7 @@ pg_status scpol_add_points(const pg_grid* g, const pg_sites* t, const pg_scpol_m
   PG_TRY(check_model("pg_potential_scpol_add", t, m));
   if (count == 0) return PG_OK;
   ModelDev md;
+  WaitOnExit done{st};
   const int n = 3 * m->npp;
   // E of a chunk is read back while it is still in L2
   const long chunk = std::min<long>(count, std::max<long>(152L * 128, (long)(kFieldBytes / (sizeof(double) * n)) / 128 * 128));
@@ -474,6 +485,7 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
   cudaStream_t st = pg::as_stream(stream);
   ModelDev md;
   pg::DevBuf<unsigned char> mbuf;
+  WaitOnExit done{st};
   PG_TRY(mbuf.alloc(md.bytes(m)));
   PG_TRY(md.upload(t, m, mbuf.p, st));
   const int ns = t->nsites, n = 3 * m->npp;

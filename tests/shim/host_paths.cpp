@@ -1,0 +1,91 @@
+// Host paths of the library on a CUDA runtime without a GPU (fake_cudart).
+// One case per run: its name is the argument, the exit status says whether it
+// holds.
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "fake_cudart.hpp"
+#include "pisces_gb300.h"
+
+namespace {
+
+#define REQUIRE(cond)                                                                    \
+  do {                                                                                   \
+    if (!(cond)) {                                                                       \
+      fprintf(stderr, "%s:%d: %s (%s)\n", __FILE__, __LINE__, #cond, pg_last_error());   \
+      return 1;                                                                          \
+    }                                                                                    \
+  } while (0)
+
+bool is(const std::string& kernel, const char* name) { return kernel.find(name) != std::string::npos; }
+
+pg_grid* grid(int nx, int ny, int nz) {
+  const int n[3] = {nx, ny, nz};
+  const double L[3] = {0.6 * (nx + 1), 0.6 * (ny + 1), 0.6 * (nz + 1)};
+  pg_grid* g = nullptr;
+  if (pg_grid_create(n, L, &g) != PG_OK) fprintf(stderr, "grid: %s\n", pg_last_error());
+  return g;
+}
+
+// A polarisation model on the first npp sites.
+struct Model {
+  std::vector<double> sites, inva, epc;
+  std::vector<int> pol;
+  pg_sites t{};
+  pg_scpol_model m{};
+  explicit Model(int npp) {
+    for (int i = 0; i < 3 * npp; ++i) sites.push_back(0.25 * i - 3.0), epc.push_back(0.01 * i);
+    inva.assign((size_t)9 * npp * npp, 0.125);
+    for (int i = 0; i < npp; ++i) pol.push_back(i);
+    t.nsites = npp;
+    t.sites = sites.data();
+    m.npp = npp;
+    m.pol_site = pol.data();
+    m.inva = inva.data();
+    m.epc = epc.data();
+    m.damp_type = 2;
+    m.damp = 2.0;
+  }
+};
+
+// The positions that the field kernel is given are the sites', also where the
+// runtime reads pageable host memory only when the stream gets to the copy.
+int scpol_upload() {
+  pg_grid* g = grid(6, 5, 4);
+  Model a(7);
+  std::vector<double> v(g ? pg_grid_npoints(g) : 1), psi(v.size());
+  const double* pos = nullptr;
+  std::vector<double> seen;
+  fake::state().on_launch = [&](const std::string& k, void** args) {
+    if (is(k, "k_scpol_field")) pos = *static_cast<const double**>(args[9]);
+  };
+  fake::state().on_wait = [&] {
+    if (pos && seen.empty()) seen.assign(pos, pos + 21);
+  };
+  fake::state().defer_copies = true;
+  REQUIRE(pg_potential_scpol_add(g, &a.t, &a.m, v.data(), nullptr, nullptr) == PG_OK);
+  REQUIRE(seen == a.sites);
+  pos = nullptr;
+  seen.clear();
+  std::vector<double> grad(21), tmu(21), mcm(441);
+  REQUIRE(pg_hf_gradient_grid(g, &a.t, &a.m, psi.data(), grad.data(), tmu.data(), mcm.data(), nullptr) == PG_OK);
+  REQUIRE(seen == a.sites);
+  pg_grid_destroy(g);
+  return 0;
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::map<std::string, std::function<int()>> cases = {
+      {"scpol_upload", scpol_upload},
+  };
+  const auto it = cases.find(argc > 1 ? argv[1] : "");
+  return it == cases.end() ? 2 : it->second();
+}
