@@ -105,8 +105,8 @@ struct KinArgs {
 struct KinCounters {
   unsigned ticket;
   unsigned finished;
-  // per vector: items done and the largest FP64 exponent (biased) written,
-  // side by side so that a waiter reads both at once
+  // per vector: items done (x) and the largest FP64 exponent (biased) written
+  // (y), in one sector
   uint2 w1[kKinMaxVec];  // XF items
   uint2 w2[kKinMaxVec];  // ZS items
 };
@@ -164,10 +164,14 @@ __device__ __forceinline__ bool kstage(const KinGeom& G, const KinArgs& A, const
     const uint2* c = it.kind == kZS ? &cnt->w1[it.u] : &cnt->w2[it.u];
     const unsigned need = it.kind == kZS ? (unsigned)G.nzi : (unsigned)G.nzt;
     const unsigned long long t0 = globaltimer_ns();
-    unsigned long long d;
+    // each half is read with the width it is written with: the acquire of the
+    // count orders the exponent's read, and the tensor copies of the vector,
+    // after everything its writers released (a wider read of both halves would
+    // only overlap the writers' accesses, which orders nothing)
+    unsigned d;
     while (true) {
-      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(c) : "memory");
-      if ((unsigned)d >= need) break;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(d) : "l"(&c->x) : "memory");
+      if (d >= need) break;
       if (*abort || globaltimer_ns() - t0 > 2000000000ull) {
         ok = 0;
         break;
@@ -175,7 +179,9 @@ __device__ __forceinline__ bool kstage(const KinGeom& G, const KinArgs& A, const
       __nanosleep(32);
     }
     // the item's scale comes from the largest exponent of the whole input vector
-    *exp_out = (int)(d >> 32);
+    unsigned e;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(&c->y) : "memory");
+    *exp_out = (int)e;
   }
   ok = __shfl_sync(0xffffffffu, ok, 0);
   if (!ok) return false;
