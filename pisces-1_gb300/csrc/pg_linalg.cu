@@ -248,8 +248,13 @@ __global__ void __launch_bounds__(kT, 2) k_gram(long N, long chunk, const double
   }
 }
 
+// Blocks per SM asked of the compiler: left to itself it gave 7 and 8 outputs
+// 99 registers (two blocks) and 15 outputs 170 (one), and one or two outputs,
+// bound by loads in flight, three blocks.  884736 points, us, before / so: 40 x 1
+// 84.5 / 69.2, 64 x 1 129 / 107, 120 x 1 232 / 194; 262144 points: 40 x 2
+// 44.6 / 39.9, 40 x 7 151 / 131, 40 x 8 171 / 149, 120 x 2 127 / 113.
 template <int NR>
-__global__ void __launch_bounds__(kT) k_combine(long N, long chunk, const double* P, const double* P2, int na,
+__global__ void __launch_bounds__(kT, NR <= 2 ? 4 : (NR <= 8 ? 3 : 2)) k_combine(long N, long chunk, const double* P, const double* P2, int na,
                                                 const double* __restrict__ C, int ca, int cr, double cscale,
                                                 const double* X,
                                                 const double* __restrict__ alpha, int inv_sqrt, double* Y, double* Y2,
