@@ -209,7 +209,7 @@ struct SliceMat {
   int nch = 1, kc = 16;          // K chunks and their width (a multiple of 16)
   int nnc = 1, nc = 16;          // N chunks and their rows (a multiple of 16)
   bool plain = false;            // entries outside the slices' range: FP64 multiply-adds for every line
-  size_t block_bytes() const { return (size_t)7 * nc * kc * 2; }
+  size_t block_bytes() const { return (size_t)10 * nc * kc * 2; }  // ten digits in FP16
 };
 
 }  // namespace pg
@@ -231,6 +231,7 @@ struct pg_grid {
   // digit images of the kinetic matrices and of the eigenbasis transforms
   // (forward Q^T, backward Q) for the FP64 axis contractions (pg_slice.cu)
   pg::SliceMat t_sl[3], q_sl[3], qb_sl[3];
+  bool t_sliced = false;           // T of every axis has exact images
   pg::DevBuf<unsigned char> sl_img;
   // TF32-rounded high part and the TF32-rounded remainder T - hi, each as
   // tensor-core operand images (tc_kmajor_off layout, one tc_npad x tc_kchunk

@@ -154,7 +154,9 @@ pg_status hx(const pg_grid* g, const double* v, const double* x, double* y, int 
   PG_ARG(x != y, "pg_hx: X and Y must not alias");
   if (precision == PG_MIXED) return hx_mixed(g, v, x, y, nvec, st, false, unit);
   PG_ARG(precision == PG_FP64, "pg_hx: unknown precision %d", precision);
-  if (in_order) {
+  // where the slices would round T's small entries further than the chain of
+  // multiply-adds rounds (a sine-DVR axis above about 750 points): the chain
+  if (in_order || !g->t_sliced) {
     by_vectors(nvec, [&](auto nv, int v0, int groups) {
       k_hx_fp64<nv.value><<<dim3((unsigned)((g->N + 255) / 256), (unsigned)groups), 256, 0, st>>>(
           g->n[0], g->n[1], g->n[2], g->t_dev[0].p, g->t_dev[1].p, g->t_dev[2].p, v, x + (long)v0 * g->N,

@@ -4,21 +4,23 @@
 //
 // Grid lines along the axis are the rows of the left operand: a CTA takes
 // 128 of them (fewer on small grids), converts their values to digit images
-// once (each line scaled by its own largest exponent), and multiplies them
-// with the matrix's digit images, which the bulk copy engine fetches from L2.  The tensor core's
-// accumulators (7 x nc columns of TMEM) are read back one line per lane.
+// once (each line scaled by its own largest exponent; above 64 points once
+// per 48 outputs), and multiplies them with the matrix's digit images, which
+// the bulk copy engine fetches from L2.  The tensor core's accumulators (10 x
+// nc columns of TMEM) are read back one line per lane.
 //
-// Bounds: per point and axis about 35 integer operations to make the digits,
-// 60 to join the accumulators and one or two FP64 operations (V X, the sum
+// Bounds: per point and axis about 40 integer operations to make the digits,
+// 95 to join the accumulators and one or two FP64 operations (V X, the sum
 // into Y), against n FP64 multiply-adds before; the FP64 pipe is about 60
-// times slower than the integer pipes here.  A tile of 128 lines of 64 points
-// spends 4000 cycles on loading, 6000 on digits and 13000 on the read-out;
-// the products run beside the read-out.
+// times slower than the integer pipes here.  No one part sets the time: of
+// 23.4 us for an axis of 64^3 x 4 (a tile per CTA) the products cost 1.4 us
+// beside the rest, the joins 2.6, the digits 2.0; the others are the latencies
+// of the lines' loads, of each N chunk's read-out and of its sum into Y.
 //
-// H X, FP64 multiply-adds / one accumulator set and K chunks of 64 (digits
-// made again for each 64 outputs) / as here, us: 32^3 33.5 / 30.7 / 20.8,
-// 64^3 x 4 371 / 52.8 / 54.4, 83x90x71 x 6 1814 / 245 / 173, 96^3 x 8 3428 /
-// 498 / 342, 160^3 x 16 (K chunks) 63060 / 5586 / 5543.
+// H X, us, FP64 multiply-adds / slices of seven 9-bit digits (whose operands
+// and sums were not exact, pg_slice.cuh) / as here: 32^3 34.0 / 19.9 / 23.0,
+// 64^3 x 4 371 / 53.0 / 70.2, 83x90x71 x 6 1816 / 173 / 341, 96^3 x 8 3435 / 341
+// / 617, 160^3 x 16 (K chunks, two launches an axis) 63100 / 5505 / 12315.
 #include <algorithm>
 #include <cmath>
 
@@ -31,9 +33,9 @@ constexpr int kLines = 128;  // MMA M
 constexpr int kST = 512;     // threads that fill and read out
 constexpr int kTransMost = (kST / 32) * 32 * 5 * 8;  // transpose buffer: 32 lines x 4 columns per warp
 
-// A line whose largest exponent lies outside [kExpLo, kExpHi] (subnormal or
-// huge values, infinities, NaN) is multiplied with FP64 multiply-adds instead.
-constexpr int kExpLo = 200, kExpHi = 1900;
+// A line whose largest exponent lies outside [exp_lo, exp_hi] (subnormal or
+// huge values, infinities, NaN, products that could leave the range of normal
+// numbers) is multiplied with FP64 multiply-adds instead.
 
 struct SliceArgs {
   long nlines;   // lines of all vectors
@@ -43,8 +45,9 @@ struct SliceArgs {
   int lc;        // lines per CTA: 128, or 64 or 32 where that still leaves one CTA per SM at most
   int h0, nch;   // K chunks [h0, h0 + nch) of this launch
   int plain;     // every line by FP64 multiply-adds
+  int exp_lo, exp_hi;
   int nc_per;    // N chunks per CTA (blockIdx.y takes the next ones)
-  int scale;     // exponent of accumulator 6: kSliceUnit - tau - 1075 - kSliceGuard
+  int scale;     // exponent of accumulator 9: kSliceUnit - tau - 1075 - kSliceGuard
   uint32_t block_bytes;  // one (K, N) block of the matrix image
   uint32_t off_b, off_t; // shared-memory offsets of the matrix blocks and the transpose buffer
   int tc;                // columns transposed at a time: 4, or 2 where shared memory is short
@@ -54,12 +57,12 @@ struct SliceArgs {
   long sa, sb;           // strides of A64 (output, input index)
 };
 
-// kChunks false: the whole axis in one K chunk (n <= 96).  The lines' digits
+// kChunks false: the whole axis in one K chunk (n <= 64).  The lines' digits
 // are made once; the matrix comes in chunks of nc columns, double buffered,
 // into two halves of tensor memory, so that a chunk's products run while the
 // one before is read out.
-// kChunks true: K chunks of at most 80, N chunks of 64; the digits are made
-// again for every N chunk.
+// kChunks true: K chunks of at most 48, N chunks of at most 48; the digits are
+// made again for every N chunk.
 // The products of the former are issued by a warp of its own (the 17th), which
 // waits for the matrix blocks and for the accumulators to be read: issued
 // by a thread that also reads out, two chunks of 64^3 took 5600 cycles before
@@ -183,7 +186,7 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     if (em) atomicMax(&s_emax[line], (int)em);
   };
   // a line's scale, once its maximum is complete; slow: by FP64 multiply-adds
-  auto is_slow = [&](int em) { return A.plain || (em != 0 && (em < kExpLo || em > kExpHi)); };
+  auto is_slow = [&](int em) { return A.plain || (em != 0 && (em < A.exp_lo || em > A.exp_hi)); };
   const uint32_t lbo = 128, sbo = (uint32_t)koct * 128u;
   const uint32_t a_slice = (uint32_t)kLines * (uint32_t)A.kc * 2u;
   // digits: one 16-byte row of a core matrix per slice and octet
@@ -198,8 +201,8 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
         uint32_t w[NS][4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const unsigned long long f0 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q], emax);
-          const unsigned long long f1 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q + 1], emax);
+          const pg::SliceInt f0 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q], emax);
+          const pg::SliceInt f1 = pg::slice_fixed(slow ? 0.0 : val[u][2 * q + 1], emax);
 #pragma unroll
           for (int i = 0; i < NS; ++i) w[i][q] = pg::slice_digit2(f0, f1, i);
         }
@@ -214,11 +217,10 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
   };
   // One thread: the products of the digits with matrix block b into
   // accumulator set b, once the block has landed.  Digit i of the lines meets
-  // digits 0 .. 6 - i of the matrix, which lie one under the other in shared
-  // memory as one operand of (7 - i) nc rows, in accumulators i .. 6, which
+  // digits 0 .. 9 - i of the matrix, which lie one under the other in shared
+  // memory as one operand of (10 - i) nc rows, in accumulators i .. 9, which
   // lie side by side: at most 256 columns an instruction (one product at a
-  // time read the lines' digits 28 times instead of 10, and took 7700 cycles
-  // a tile of 64 x 64; so, and with the descriptors counted up, 4600).
+  // time reads the lines' digits once for each).
   auto issue = [&](int b, uint32_t parity, bool first) {
     if (!mbar_wait(smem_u32(&bar_b[b]), parity)) {
       s_fail = 1;
@@ -467,7 +469,7 @@ __global__ void k_slice_matrix(const SliceBuild B) {
   const size_t block = (size_t)pg::kSliceN * nc * kc * 2;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
     const int i = e / n, k = e - i * n;
-    const unsigned long long f = pg::slice_fixed(B.A[m][B.trans ? k * n + i : e], B.emax[m]);
+    const pg::SliceInt f = pg::slice_fixed(B.A[m][B.trans ? k * n + i : e], B.emax[m]);
     const int c = i / nc, h = k / kc;
     unsigned char* p = B.img[m] + (size_t)(h * B.nnc[m] + c) * block + pg::tc16_kmajor_off(i - c * nc, k - h * kc, kc);
 #pragma unroll
@@ -491,21 +493,36 @@ cudaError_t launch_slice(const SliceArgs& a, dim3 grid, size_t smem, const unsig
 
 namespace pg {
 
-// Up to 96 points: one K chunk, N chunks of 32 (two sets of 7 accumulators in
+// Up to 64 points: one K chunk, N chunks of 16 (two sets of 10 accumulators in
 // 512 columns of tensor memory; the lines' digits and two blocks of the
-// matrix's in shared memory), or of 16 where shared memory asks for it (above
-// 80 points) and on short axes, whose small grids then spread over more CTAs.
-// The digits of 81 to 96 points made once instead of twice: 96^3 x 8 498 ->
-// 342 us; 32 points in two chunks on CTAs of their own: 30 -> 21 us a product.
-// Longer axes: K chunks of at most 80, N chunks of 64.
+// matrix's in shared memory).  Longer axes: K chunks and N chunks of at most
+// 48 (10 x 48 columns; 169 KB of shared memory), whose products with all K
+// chunks of a launch meet in one set of accumulators.
 static void slice_shape(int n, SliceMat* S) {
   S->n = n;
-  S->nch = n <= 96 ? 1 : (n + 79) / 80;
+  S->nch = n <= 64 ? 1 : (n + 47) / 48;
   S->kc = ((n + S->nch - 1) / S->nch + 15) / 16 * 16;
   const int npad = (n + 15) / 16 * 16;
-  const int most = S->nch > 1 ? 64 : (n > 80 || n <= 32 ? 16 : 32);
+  const int most = S->nch > 1 ? 48 : 16;
   S->nnc = (npad + most - 1) / most;
   S->nc = ((npad + S->nnc - 1) / S->nnc + 15) / 16 * 16;
+}
+
+// Whether a product from slices of this n x n matrix is as exact, value by
+// value, as a chain of n multiply-adds may be: entries that are not zero no
+// further than r bits below the largest, which the slices round by 2^(r - 26)
+// of an FP64 rounding (kSliceGuard bits are to spare), two such roundings (T
+// and the line) against n.  The sine DVR keeps to this up to about 750 points.
+static bool slice_exact(const std::vector<double>& t) {
+  double big = 0, small = INFINITY;
+  for (double x : t) {
+    if (!std::isfinite(x)) return false;
+    const double a = fabs(x);
+    big = std::max(big, a);
+    if (a > 0) small = std::min(small, a);
+  }
+  if (big == 0) return true;
+  return std::ilogb(big) - std::ilogb(small) <= kSliceGuard + std::ilogb(sqrt((double)t.size())) - 1;
 }
 
 // T, Q^T and Q of the three axes; the host copies give the largest entry
@@ -514,6 +531,7 @@ pg_status slice_grid(pg_grid* g) {
   SliceBuild B{};
   SliceMat* S[9];
   int share[9], count = 0;
+  g->t_sliced = slice_exact(g->t[0]) && slice_exact(g->t[1]) && slice_exact(g->t[2]);
   size_t off[9], total = 0;
   for (int m = 0; m < 9; ++m) {
     const int a = m % 3;
@@ -525,6 +543,7 @@ pg_status slice_grid(pg_grid* g) {
       if (g->n[b] == g->n[a] && g->t[b] == g->t[a]) share[m] = m - a + b;
     if (share[m] < 0 && m >= 6 && g->dvrtype != 3) share[m] = m - 3;  // the DST-I is symmetric
     while (share[m] >= 0 && share[share[m]] >= 0) share[m] = share[share[m]];
+    if (m < 3 && !g->t_sliced) continue;  // no images of T
     off[m] = total;
     if (share[m] < 0) total += ((size_t)S[m]->nch * S[m]->nnc * S[m]->block_bytes() + 255) / 256 * 256;
   }
@@ -537,6 +556,7 @@ pg_status slice_grid(pg_grid* g) {
     if (m < 3) {
       big = 0;
       for (double t : g->t[a]) big = std::max(big, fabs(t));
+      if (!g->t_sliced) continue;
     }
     int ex = 0;
     frexp(big, &ex);  // big < 2^ex, its biased exponent ex + 1022
@@ -578,6 +598,8 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   a.sa = trans ? 1 : S.n;
   a.sb = trans ? S.n : 1;
   a.scale = kSliceUnit - kSliceGuard - S.tau - 1075;
+  a.exp_lo = 200;
+  a.exp_hi = 1900;
   a.block_bytes = (uint32_t)S.block_bytes();
   const bool chunks = S.nch > 1;
   a.off_b = (uint32_t)(kSliceN * kLines * S.kc * 2);
@@ -603,7 +625,7 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   while (a.lc > 32 && (nlines + a.lc / 2 - 1) / (a.lc / 2) * split <= 152) a.lc /= 2;
   const long tiles = (nlines + a.lc - 1) / a.lc;
   const dim3 grid((unsigned)tiles, (unsigned)split);
-  // at most two K chunks (160 values) per launch, so that the sums of one
+  // at most kSliceK values (two K chunks) per launch, so that the sums of one
   // accumulator stay below 2^24; a longer axis adds up in Y
   int launches = 0;
   for (int h0 = 0; h0 < S.nch; h0 += 2, ++launches) {
@@ -612,10 +634,9 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
     a.mode = h0 == 0 || mode == 3 ? mode : 1;
     a.out0 = (long)launches * split * nlines;
     cudaError_t e;
-    if (chunks) e = launch_slice<3, true>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    if (chunks) e = launch_slice<2, true>(a, grid, smem, S.img, A64, v, x, y, err, st);
     else if (S.kc <= 32) e = launch_slice<1, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
-    else if (S.kc <= 64) e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
-    else e = launch_slice<3, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    else e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
     PG_CUDA_TRY(e);
     PG_TRY(check_launch("k_slice_axis"));
   }
