@@ -522,7 +522,8 @@ static bool slice_exact(const std::vector<double>& t) {
     if (a > 0) small = std::min(small, a);
   }
   if (big == 0) return true;
-  return std::ilogb(big) - std::ilogb(small) <= kSliceGuard + std::ilogb(sqrt((double)t.size())) - 1;
+  return big < 1e270 && small > 1e-270 &&
+         std::ilogb(big) - std::ilogb(small) <= kSliceGuard + std::ilogb(sqrt((double)t.size())) - 1;
 }
 
 // T, Q^T and Q of the three axes; the host copies give the largest entry
@@ -598,8 +599,9 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   a.sa = trans ? 1 : S.n;
   a.sb = trans ? S.n : 1;
   a.scale = kSliceUnit - kSliceGuard - S.tau - 1075;
-  a.exp_lo = 200;
-  a.exp_hi = 1900;
+  // lines whose products stay normal numbers with this matrix (slice_join)
+  a.exp_lo = std::max(2, -1022 - a.scale);
+  a.exp_hi = std::min(2046, 1023 - kSliceBits - a.scale);
   a.block_bytes = (uint32_t)S.block_bytes();
   const bool chunks = S.nch > 1;
   a.off_b = (uint32_t)(kSliceN * kLines * S.kc * 2);
@@ -661,7 +663,7 @@ int slice_row_count(int n) {
 
 size_t slice_rows_shape(int n, double big, SliceMat* S) {
   slice_shape(n, S);
-  S->plain = !std::isfinite(big) || big > 1e200 || (big != 0 && big < 1e-200);
+  S->plain = !std::isfinite(big) || (big != 0 && (big > 1e270 || big < 1e-270));
   int ex = 0;
   if (!S->plain) frexp(big, &ex);
   S->tau = kSliceN * kSliceP - 1 - ex;
