@@ -116,13 +116,18 @@ struct ModelDev {
   static size_t up(size_t b) { return (b + 255) / 256 * 256; }
   size_t bytes(const pg_scpol_model* m) {
     const int n = 3 * m->npp;
-    double big = 0;
+    std::vector<double> col(n, 0.0);  // the largest entry of each column
     bool finite = true;
     for (size_t e = 0; e < (size_t)n * n; ++e) {
       finite &= std::isfinite(m->inva[e]);
-      big = std::max(big, fabs(m->inva[e]));
+      col[e % n] = std::max(col[e % n], fabs(m->inva[e]));
     }
-    img_bytes = pg::slice_rows_shape(n, finite ? big : INFINITY, &mat);
+    double big = 0, low = INFINITY;
+    for (double c : col) {
+      big = std::max(big, c);
+      if (c > 0) low = std::min(low, c);
+    }
+    img_bytes = pg::slice_rows_shape(n, finite ? big : INFINITY, low, &mat);
     return up(img_bytes) + 2 * up(sizeof(double) * n) + up(sizeof(double) * n * n);
   }
   // The copies are queued: this struct and the caller's arrays are to outlive

@@ -661,9 +661,9 @@ int slice_row_count(int n) {
   return (S.nch + 1) / 2 * S.nnc;
 }
 
-size_t slice_rows_shape(int n, double big, SliceMat* S) {
+size_t slice_rows_shape(int n, double big, double low, SliceMat* S) {
   slice_shape(n, S);
-  S->plain = !std::isfinite(big) || (big != 0 && (big > 1e270 || big < 1e-270));
+  S->plain = !std::isfinite(big) || (big != 0 && (big > 1e270 || low < 1e-270 || low < std::ldexp(big, -20)));
   int ex = 0;
   if (!S->plain) frexp(big, &ex);
   S->tau = kSliceN * kSliceP - 1 - ex;

@@ -157,8 +157,11 @@ pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double
 // A64 and the images (slice_rows_matrix) on the device; err as tc_err.
 enum SliceRows { kRowStore = 0, kRowDot = 3 };
 int slice_row_count(int n);
-// shape and bytes of the images of an n x n matrix whose largest entry is big
-size_t slice_rows_shape(int n, double big, SliceMat* S);
+// Shape and bytes of the images of an n x n matrix whose largest entry is big
+// and whose columns that are not zero all reach low.  A column far below the
+// largest would keep few of its bits (one scale for the matrix): from 2^-20 on,
+// as for entries outside the slices' range, every line goes by multiply-adds.
+size_t slice_rows_shape(int n, double big, double low, SliceMat* S);
 pg_status slice_rows_matrix(const double* A64, unsigned char* img, SliceMat* S, cudaStream_t st);
 pg_status slice_rows(long nlines, const SliceMat& S, const double* A64, const double* x, double* y, SliceRows mode,
                      int* rows, int* err, cudaStream_t st);

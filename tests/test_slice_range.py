@@ -1,8 +1,9 @@
-"""The FP64 products from slices at the ends of FP64's range.
+"""The FP64 products from slices at the ends of FP64's range, and with matrices of very different columns.
 
 The slices of a line and of the matrix each have a scale of their own; the
 result's exponent is the sum of both, and it has to stay that of a normal
-number.  Lines and matrices for which it may not go through FP64 multiply-adds.
+number.  Lines and matrices for which it may not, and columns that one scale
+for the whole matrix would cut, go through FP64 multiply-adds.
 """
 import numpy as np
 import pytest
@@ -64,3 +65,22 @@ def test_row_dots_at_the_ends_of_the_range(pg, torch, clusters, a, e):
         assert np.all(v == ref)
     else:
         assert np.all(np.abs(v - ref) <= 60 * 2.0 ** -53 * abs(ref) + n * n * 2.0 ** -1022)
+
+
+@pytest.mark.parametrize("ratio", [2.0 ** -12, 2.0 ** -30, 2.0 ** -70, 2.0 ** -120])
+def test_columns_of_very_different_size(pg, torch, clusters, ratio):
+    """Half of the columns a factor smaller, and a field that meets only them: V is theirs alone.
+
+    V = -sum E_k A_kc E_c / 2 with E zero but in the small columns: one
+    rounding of each product sum, chains of 24 equal terms: 30 roundings."""
+    grid = pg.Grid((5, 6, 7), 12.0)
+    n, h = 24, 12
+    inva = np.full((n, n), 1.0 / 3.0)
+    inva[h:, h:] *= ratio
+    inva[:h, h:] *= ratio
+    epc = np.zeros(n)
+    epc[h:] = 0.7
+    v = grid.scpol_add(far_model(pg, clusters, n // 3, inva, epc),
+                       torch.zeros(grid.N, dtype=torch.float64, device="cuda")).cpu().numpy()
+    ref = -0.5 * (h * 0.7) ** 2 / 3.0 * ratio
+    assert np.all(np.abs(v - ref) <= 30 * 2.0 ** -53 * abs(ref)), float(np.abs(v / ref - 1).max() * 2 ** 53)
