@@ -268,16 +268,24 @@ pg_status pg_water_default_tables(int nw, const double* sites, const double* cha
 /* ------------------------------------------------------------------- H * X */
 
 /* Y = H X for nvec vectors: H = V + Tx (+) Ty (+) Tz.  precision PG_FP64:
- * FP64 throughout, the kinetic contractions from exact slices of both
- * operands on the tensor cores (each rounded once); the call returns once
- * its launches are queued, and pg_grid_check reports a completion wait that
- * timed out.  PG_MIXED: kinetic contractions as split FP16 or TF32
- * tensor-core products accumulated in FP32, V*X in FP64.  nvec = 0 does
+ * FP64 throughout, the kinetic contractions on the tensor cores from slices
+ * that hold T and X to 79 bits below their largest values, each rounded once
+ * (a value is within a few roundings of the magnitude of its own terms).
+ * pg_solve, the engine and pg_davidson's own products use chains of FP64
+ * multiply-adds instead where several states are asked for in FP64: a state
+ * that a restart leaves with a sign decided by rounding may come out with the
+ * other one in a caller's loop around pg_davidson_rci and pg_hx.
+ * PG_MIXED: kinetic contractions as split FP16 or TF32
+ * tensor-core products accumulated in FP32, V*X in FP64.  Waits for the stream
+ * and returns PG_DEVICE_TIMEOUT if a completion wait inside a kernel of this
+ * grid timed out (Y is then incomplete); in FP64 on a stream that is being
+ * captured it queues its launches and returns, and pg_grid_check reports after
+ * the graph has run.  nvec = 0 does
  * nothing and accepts null X and Y.  Replaces DVR::MatrixTimesVector applied
  * vector by vector (src/mtx.cpp:22-109, src/davdriver.cpp:67-78). */
 pg_status pg_hx(const pg_grid* g, const double* v_dev, const double* x_dev, double* y_dev, int nvec, int precision,
                 void* stream);
-/* pg_hx without the completion check of the mixed form: returns once the
+/* pg_hx without the completion check: returns once the
  * launches are queued (no host wait).  A tensor-core completion wait that
  * timed out is recorded in the grid's status word and reported by the next
  * pg_grid_check. */

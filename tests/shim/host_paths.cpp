@@ -80,11 +80,49 @@ int scpol_upload() {
   return 0;
 }
 
+// A completion wait that times out inside a kernel: the call that queued it
+// says so, in FP64 as in the mixed form; the queue-only form leaves it to the
+// check, which clears it.
+int hx_status() {
+  pg_grid* g = grid(66, 20, 20);
+  const long N = g ? pg_grid_npoints(g) : 1;
+  std::vector<double> v(N), x(N), y(N);
+  bool fail = true;
+  fake::state().on_launch = [&](const std::string& k, void** args) {
+    if (fail && is(k, "k_slice_axis")) **static_cast<int**>(args[6]) = 1;
+  };
+  REQUIRE(pg_hx(g, v.data(), x.data(), y.data(), 1, PG_FP64, nullptr) == PG_DEVICE_TIMEOUT);
+  REQUIRE(pg_grid_check(g, nullptr) == PG_DEVICE_TIMEOUT);
+  REQUIRE(pg_grid_check(g, nullptr) == PG_OK);
+  const int waits = fake::state().waits;
+  REQUIRE(pg_hx_async(g, v.data(), x.data(), y.data(), 1, PG_FP64, nullptr) == PG_OK);
+  REQUIRE(fake::state().waits == waits);
+  REQUIRE(pg_grid_check(g, nullptr) == PG_DEVICE_TIMEOUT);
+  fail = false;
+  REQUIRE(pg_hx(g, v.data(), x.data(), y.data(), 1, PG_FP64, nullptr) == PG_OK);
+  pg_grid_destroy(g);
+  return 0;
+}
+
+// On a stream that is being captured the FP64 form only queues.
+int hx_captured() {
+  pg_grid* g = grid(66, 20, 20);
+  const long N = g ? pg_grid_npoints(g) : 1;
+  std::vector<double> v(N), x(N), y(N);
+  fake::state().capturing = true;
+  REQUIRE(pg_hx(g, v.data(), x.data(), y.data(), 1, PG_FP64, nullptr) == PG_OK);
+  fake::state().capturing = false;
+  pg_grid_destroy(g);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::map<std::string, std::function<int()>> cases = {
       {"scpol_upload", scpol_upload},
+      {"hx_status", hx_status},
+      {"hx_captured", hx_captured},
   };
   const auto it = cases.find(argc > 1 ? argv[1] : "");
   return it == cases.end() ? 2 : it->second();
