@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdio>
 #include <map>
 #include <memory>
@@ -60,6 +61,20 @@ inline pg_status check_launch(const char* what) {
     return PG_CUDA;
   }
   return PG_OK;
+}
+
+// Runs set() once for every device it is called on: a kernel's attributes
+// belong to the device that was current when they were set.
+template <class Set>
+inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, const Set& set) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = set();
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 // Device buffer owned by RAII (cudaMalloc/cudaFree).

@@ -927,17 +927,17 @@ inline bool pair_ok(long N, const double* P, const double* Q) {
   return N % 2 == 0 && ((uintptr_t)P % 16) == 0 && ((uintptr_t)Q % 16) == 0;
 }
 
-// Dynamic shared-memory opt-in, once per kernel.
+// Dynamic shared-memory opt-in, once per kernel and device.
 static pg_status opt_in_smem() {
-  static const cudaError_t init = [] {  // thread-safe static initialisation
+  static std::atomic<unsigned long long> done{0};
+  PG_CUDA_TRY(once_per_device(done, [] {
     cudaError_t e = cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_gram_df<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_gram_df<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);
     return e;
-  }();
-  PG_CUDA_TRY(init);
+  }));
   return PG_OK;
 }
 

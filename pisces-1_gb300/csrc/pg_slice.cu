@@ -483,8 +483,10 @@ constexpr int kSmemMost = 226 * 1024;
 template <int NU, bool kChunks>
 cudaError_t launch_slice(const SliceArgs& a, dim3 grid, size_t smem, const unsigned char* img, const double* A64,
                          const double* v, const double* x, double* y, int* err, cudaStream_t st) {
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_slice_axis<NU, kChunks>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+  static std::atomic<unsigned long long> done{0};
+  const cudaError_t attr = pg::once_per_device(done, [] {
+    return cudaFuncSetAttribute(k_slice_axis<NU, kChunks>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+  });
   if (attr != cudaSuccess) return attr;
   return pg::launch_dependent(k_slice_axis<NU, kChunks>, grid, dim3(kST + (kChunks ? 0 : 32)), smem, st, a, img, A64, v, x, y, err);
 }

@@ -15,7 +15,7 @@ struct Copy {
 };
 std::recursive_mutex m;
 std::map<cudaStream_t, std::vector<Copy>> pending;
-std::map<void*, size_t> device_blocks;
+std::map<void*, std::pair<size_t, int>> device_blocks;
 std::map<const void*, size_t> pinned_sizes;
 std::map<const void*, std::string>& names() {
   static std::map<const void*, std::string> n;
@@ -55,6 +55,18 @@ namespace fake {
 State& state() {
   static State s;
   return s;
+}
+int device_of(const void* p) {
+  for (auto& b : device_blocks)
+    if ((const char*)p >= (const char*)b.first && (const char*)p < (const char*)b.first + b.second.first)
+      return b.second.second;
+  return -1;
+}
+size_t kept_on(int device) {
+  size_t n = 0;
+  for (auto& b : device_blocks)
+    if (b.second.second == device) n += b.second.first;
+  return n;
 }
 }  // namespace fake
 
@@ -106,13 +118,13 @@ cudaError_t cudaMalloc(void** p, size_t n) {
   }
   *p = aligned_alloc(256, (n + 255) / 256 * 256);
   memset(*p, 0, (n + 255) / 256 * 256);
-  device_blocks[*p] = n;
+  device_blocks[*p] = {n, s.device};
   s.in_use += n;
   return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {
   std::lock_guard<std::recursive_mutex> l(m);
-  fake::state().in_use -= device_blocks[p];
+  fake::state().in_use -= device_blocks[p].first;
   device_blocks.erase(p);
   free(p);
   return cudaSuccess;

@@ -33,5 +33,7 @@ struct State {
 };
 
 State& state();
+int device_of(const void* p);  // the device whose allocation holds p, or -1
+size_t kept_on(int device);    // device bytes allocated on it
 
 }  // namespace fake

@@ -10,6 +10,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda_runtime_api.h>
+
 #include "fake_cudart.hpp"
 #include "pisces_gb300.h"
 
@@ -116,6 +118,25 @@ int hx_captured() {
   return 0;
 }
 
+// Kernels that need more shared memory than the default get it on every device
+// they run on.
+int second_device() {
+  for (int dev = 0; dev < 3; ++dev) {
+    REQUIRE(cudaSetDevice(dev) == cudaSuccess);
+    pg_grid* g = grid(66, 20, 20);
+    const long N = g ? pg_grid_npoints(g) : 1;
+    std::vector<double> v(N), x(N * 44), y(N * 44), out(40 * 4);
+    const double sigma = -0.1;
+    REQUIRE(pg_hx(g, v.data(), x.data(), y.data(), 1, PG_FP64, nullptr) == PG_OK);
+    REQUIRE(pg_kinetic_precondition(g, x.data(), 1, &sigma, PG_FP64, nullptr) == PG_OK);
+    for (int precision : {PG_FP64, PG_MIXED})
+      REQUIRE(pg_block_gram(N, x.data(), 40, y.data(), 4, out.data(), precision, nullptr) == PG_OK);
+    REQUIRE(fake::state().refused.empty());
+    pg_grid_destroy(g);
+  }
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -123,6 +144,7 @@ int main(int argc, char** argv) {
       {"scpol_upload", scpol_upload},
       {"hx_status", hx_status},
       {"hx_captured", hx_captured},
+      {"second_device", second_device},
   };
   const auto it = cases.find(argc > 1 ? argv[1] : "");
   return it == cases.end() ? 2 : it->second();
