@@ -227,6 +227,34 @@ __global__ void k_potential_spherical(int nx, int ny, int nz, const double* __re
   }
 }
 
+// Device memory for the tables of one call, which waits for its stream before
+// it returns: kept with the thread for the next call on the same device, up to
+// kTablesMost; a larger buffer lasts for the call.
+constexpr size_t kTablesMost = 32u << 20;
+class CallTables {
+ public:
+  pg_status get(size_t bytes, unsigned char** p) {
+    static thread_local struct {
+      int device = -1;
+      pg::DevBuf<unsigned char> buf;
+    } kept;
+    pg::DevBuf<unsigned char>* b = &own_;
+    if (bytes <= kTablesMost) {
+      int dev = 0;
+      PG_CUDA_TRY(cudaGetDevice(&dev));
+      if (dev != kept.device) kept.buf.release();
+      kept.device = dev;
+      b = &kept.buf;
+    }
+    PG_TRY(b->ensure(bytes));
+    *p = b->p;
+    return PG_OK;
+  }
+
+ private:
+  pg::DevBuf<unsigned char> own_;
+};
+
 int grid_stride_blocks(long N) {
   long b = (N + 255) / 256;
   return (int)(b < 152L * 16 ? (b > 0 ? b : 1) : 152L * 16);
@@ -310,25 +338,25 @@ extern "C" pg_status pg_potential_eval(const pg_grid* g, const pg_sites* t, doub
                   bits(t->charge_damp), bits(t->dipole_damp), bits(t->pol_damp)};
   cudaStream_t st = pg::as_stream(stream);
   const int per = g->n[0] + g->n[1] + g->n[2];
-  // per-thread, grow-only device copies (the call waits for its stream before
-  // returning, so the next call may overwrite them)
-  static thread_local pg::DevBuf<double> drec;
-  static thread_local pg::DevBuf<AxisEntry> daxes;
   // points per thread: four where that leaves every SM several blocks, fewer
   // on small grids (blocks of 64 threads spread evenly over the SMs: 64^3 in
   // 1.45 ms, with 128 threads 1.65)
   const long cols = (long)g->n[0] * g->n[1];
   const int R = g->N >= 200000 ? 4 : (g->N >= 80000 ? 2 : 1);
   const dim3 grid((unsigned)((cols + kPT - 1) / kPT), (unsigned)((g->n[2] + R - 1) / R));
-  PG_TRY(drec.ensure(rec.size()));
-  PG_TRY(daxes.ensure((size_t)ns * per));
-  PG_CUDA_TRY(cudaMemcpyAsync(drec.p, rec.data(), rec.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  CallTables tables;
+  unsigned char* tab = nullptr;
+  const size_t rec_bytes = rec.size() * sizeof(double);  // a multiple of 128
+  PG_TRY(tables.get(rec_bytes + (size_t)ns * per * sizeof(AxisEntry), &tab));
+  double* drec = reinterpret_cast<double*>(tab);
+  AxisEntry* daxes = reinterpret_cast<AxisEntry*>(tab + rec_bytes);
+  PG_CUDA_TRY(cudaMemcpyAsync(drec, rec.data(), rec_bytes, cudaMemcpyHostToDevice, st));
   const long entries = (long)ns * per;
   k_site_axes<<<(unsigned)std::min<long>((entries + 255) / 256, 152L * 16), 256, 0, st>>>(
-      g->n[0], g->n[1], g->n[2], g->x_dev[0].p, g->x_dev[1].p, g->x_dev[2].p, drec.p, ns, daxes.p);
+      g->n[0], g->n[1], g->n[2], g->x_dev[0].p, g->x_dev[1].p, g->x_dev[2].p, drec, ns, daxes);
   PG_TRY(pg::check_launch("k_site_axes"));
   const auto k = R == 4 ? k_potential_dpp<4> : (R == 2 ? k_potential_dpp<2> : k_potential_dpp<1>);
-  k<<<grid, kPT, 0, st>>>(g->n[0], g->n[1], g->n[2], drec.p, ns, daxes.p, D, v, parts);
+  k<<<grid, kPT, 0, st>>>(g->n[0], g->n[1], g->n[2], drec, ns, daxes, D, v, parts);
   PG_TRY(pg::check_launch("k_potential_dpp"));
   PG_CUDA_TRY(cudaStreamSynchronize(st));
   return PG_OK;
@@ -344,12 +372,14 @@ extern "C" pg_status pg_potential_ions_add(const pg_grid* g, int nions, const do
     for (int c = 0; c < 3; ++c) ion[4 * s + c] = pos[3 * s + c];
     ion[4 * s + 3] = q[s];
   }
-  static thread_local pg::DevBuf<double> d;  // per-thread, grow-only; idle again on return
-  PG_TRY(d.ensure(ion.size()));
+  CallTables tables;
+  unsigned char* tab = nullptr;
+  PG_TRY(tables.get(ion.size() * sizeof(double), &tab));
+  double* d = reinterpret_cast<double*>(tab);
   cudaStream_t st = pg::as_stream(stream);
-  PG_CUDA_TRY(cudaMemcpyAsync(d.p, ion.data(), ion.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  PG_CUDA_TRY(cudaMemcpyAsync(d, ion.data(), ion.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   k_potential_ions<<<grid_stride_blocks(g->N), 256, 0, st>>>(g->n[0], g->n[1], g->n[2], g->x_dev[0].p,
-                                                             g->x_dev[1].p, g->x_dev[2].p, d.p, nions,
+                                                             g->x_dev[1].p, g->x_dev[2].p, d, nions,
                                                              1.0 / r_cation, 1.0 / r_anion, v);
   PG_TRY(pg::check_launch("k_potential_ions"));
   PG_CUDA_TRY(cudaStreamSynchronize(st));

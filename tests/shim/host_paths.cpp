@@ -137,6 +137,40 @@ int second_device() {
   return 0;
 }
 
+// The tables of a V(r) call lie on the device that the call runs on, and what
+// a thread keeps of them between calls is bounded.
+int potential_tables() {
+  std::vector<double> sites(3 * 60000, 0.5), q(60000, -0.1);
+  std::vector<int> at(60000);
+  for (int i = 0; i < 60000; ++i) at[i] = i;
+  std::vector<const void*> seen;
+  fake::state().on_launch = [&](const std::string& k, void** args) {
+    if (is(k, "k_potential_dpp")) seen = {*static_cast<void**>(args[3]), *static_cast<void**>(args[5])};
+    if (is(k, "k_potential_ions")) seen = {*static_cast<void**>(args[6])};
+  };
+  for (int dev : {0, 1, 0}) {
+    REQUIRE(cudaSetDevice(dev) == cudaSuccess);
+    pg_grid* g = grid(20, 12, 10);
+    std::vector<double> v(g ? pg_grid_npoints(g) : 1);
+    pg_sites t{};
+    t.sites = sites.data();
+    t.charges = q.data();
+    t.charge_site = at.data();
+    t.charge_damp = 1.7;
+    for (int ns : {5, 60000, 7}) {
+      t.nsites = t.ncharges = ns;
+      const size_t before = fake::kept_on(dev);
+      REQUIRE(pg_potential_eval(g, &t, v.data(), nullptr, nullptr) == PG_OK);
+      for (const void* p : seen) REQUIRE(fake::device_of(p) == dev || ns == 60000);
+      REQUIRE(seen.size() == 2 && fake::kept_on(dev) <= before + (32u << 20));
+    }
+    REQUIRE(pg_potential_ions_add(g, 3, sites.data(), q.data(), 1.0, 1.0, v.data(), nullptr) == PG_OK);
+    for (const void* p : seen) REQUIRE(fake::device_of(p) == dev);
+    pg_grid_destroy(g);
+  }
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -145,6 +179,7 @@ int main(int argc, char** argv) {
       {"hx_status", hx_status},
       {"hx_captured", hx_captured},
       {"second_device", second_device},
+      {"potential_tables", potential_tables},
   };
   const auto it = cases.find(argc > 1 ? argv[1] : "");
   return it == cases.end() ? 2 : it->second();
