@@ -43,7 +43,7 @@ constexpr int kPT = 64;         // threads per block: small blocks spread evenly
 
 // record fields
 enum { R_X, R_Y, R_Z, R_Q, R_MX, R_MY, R_MZ, R_ALPHA, R_Z0, R_C0, R_Z1, R_C1, R_FLAGS };
-enum { F_CHARGE = 1, F_DIPOLE = 2, F_POL = 4, F_ZPOS = 32 };  // bits 3..4: number of Slater terms; Slater exponents >= 0
+enum { F_CHARGE = 1, F_DIPOLE = 2, F_POL = 4, F_ZPOS = 32 };  // bits 3..4: number of Slater terms; Slater exponents without a sign
 
 constexpr double kStoCut = 50.0;  // z R beyond which a Slater core term is dropped
 constexpr uint64_t kStoCutBits = 0x4049000000000000ull;  // its FP64 bits
@@ -318,7 +318,7 @@ extern "C" pg_status pg_potential_eval(const pg_grid* g, const pg_sites* t, doub
   // order reproduces that order only if every list is sorted by site.
   for (int s = 0; s < ns; ++s) {
     double* R = &rec[(size_t)s * kRec];
-    const bool zpos = R[R_Z0] >= 0 && R[R_Z1] >= 0;
+    const bool zpos = !std::signbit(R[R_Z0]) && !std::signbit(R[R_Z1]);  // -0 R is not above 0 as an integer
     R[R_FLAGS] = (double)(flags[s] | ((nsto[s] > 2 ? 2 : nsto[s]) << 3) | (zpos ? F_ZPOS : 0));
   }
 
