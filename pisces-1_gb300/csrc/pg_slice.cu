@@ -585,6 +585,17 @@ pg_status slice_grid(pg_grid* g) {
 
 namespace {
 
+// SMs of the current device.
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 152;
+  if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 152;
+  if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // Launches the contraction of nlines lines (stride inner); mode 3 writes
 // *rows rows of nlines partial dots.
 pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, const double* A64, bool trans,
@@ -622,11 +633,12 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   // scheduler's warps), its digits do not (64^3 x 1: 44 us with the lines
   // first, 34 so; 80^3 x 1 62 / 48, 160x60x60 x 1 91 / 63).
   const long full = (nlines + kLines - 1) / kLines;
-  const int groups = (int)std::max<long>(1, std::min<long>(S.nnc, 152 / full));
+  const int sms = sm_count();
+  const int groups = (int)std::max<long>(1, std::min<long>(S.nnc, sms / full));
   a.nc_per = (S.nnc + groups - 1) / groups;
   const int split = (S.nnc + a.nc_per - 1) / a.nc_per;
   a.lc = kLines;
-  while (a.lc > 32 && (nlines + a.lc / 2 - 1) / (a.lc / 2) * split <= 152) a.lc /= 2;
+  while (a.lc > 32 && (nlines + a.lc / 2 - 1) / (a.lc / 2) * split <= sms) a.lc /= 2;
   const long tiles = (nlines + a.lc - 1) / a.lc;
   const dim3 grid((unsigned)tiles, (unsigned)split);
   // at most kSliceK values (two K chunks) per launch, so that the sums of one

@@ -33,7 +33,7 @@ void flush(cudaStream_t st) {
   pending[st].clear();
 }
 
-cudaError_t launch(const void* f, size_t smem, void** args) {
+cudaError_t launch(const void* f, dim3 grid, size_t smem, void** args) {
   std::lock_guard<std::recursive_mutex> l(m);
   fake::State& s = fake::state();
   const std::string& name = names()[f];
@@ -45,6 +45,7 @@ cudaError_t launch(const void* f, size_t smem, void** args) {
     }
   }
   s.launches[name] += 1;
+  s.grids[name] = {grid.x, grid.y};
   if (s.on_launch) s.on_launch(name, args);
   return cudaSuccess;
 }
@@ -103,11 +104,11 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void* st) {
   *(cudaStream_t*)st = config.st;
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void** args, size_t smem, cudaStream_t) {
-  return launch((const void*)k, smem, args);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3, void** args, size_t smem, cudaStream_t) {
+  return launch((const void*)k, grid, smem, args);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
-  return launch(f, c->dynamicSmemBytes, args);
+  return launch(f, c->gridDim, c->dynamicSmemBytes, args);
 }
 cudaError_t cudaMalloc(void** p, size_t n) {
   std::lock_guard<std::recursive_mutex> l(m);
@@ -197,7 +198,7 @@ cudaError_t cudaSetDevice(int d) {
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-  *v = a == cudaDevAttrMultiProcessorCount ? 152 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448 : 0;
+  *v = a == cudaDevAttrMultiProcessorCount ? fake::state().sms : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448 : 0;
   return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {

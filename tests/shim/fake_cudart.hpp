@@ -15,6 +15,8 @@ namespace fake {
 
 struct State {
   int device = 0;
+  int sms = 152;
+  std::map<std::string, std::pair<unsigned, unsigned>> grids;  // of each kernel's last launch
   // copies from pageable memory run when their stream is waited for, as they
   // may where the device reads pageable memory directly
   bool defer_copies = false;

@@ -171,6 +171,24 @@ int potential_tables() {
   return 0;
 }
 
+// The tiles of an axis are spread over the SMs that the device has.
+int slice_grids() {
+  std::pair<unsigned, unsigned> want[2] = {{13, 2}, {4, 1}};  // 400 lines of 66 points, two column chunks
+  for (int dev : {0, 1}) {
+    REQUIRE(cudaSetDevice(dev) == cudaSuccess);
+    fake::state().sms = dev == 0 ? 152 : 6;
+    pg_grid* g = grid(66, 20, 20);
+    std::vector<double> v(g ? pg_grid_npoints(g) : 1), x(v), y(v);
+    REQUIRE(pg_hx(g, v.data(), x.data(), y.data(), 1, PG_FP64, nullptr) == PG_OK);
+    bool seen = false;
+    for (auto& k : fake::state().grids)
+      if (is(k.first, "k_slice_axisILi2ELb1E")) seen = k.second == want[dev];
+    REQUIRE(seen);
+    pg_grid_destroy(g);
+  }
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -180,6 +198,7 @@ int main(int argc, char** argv) {
       {"hx_captured", hx_captured},
       {"second_device", second_device},
       {"potential_tables", potential_tables},
+      {"slice_grids", slice_grids},
   };
   const auto it = cases.find(argc > 1 ? argv[1] : "");
   return it == cases.end() ? 2 : it->second();
