@@ -51,6 +51,13 @@ long pg_kernel_launches(void);
 /* Number of device allocations (cudaMalloc) this library has made since it
  * was loaded, successful or not. */
 long pg_device_allocations(void);
+/* Device memory kept between calls: a grid keeps the scratch of its own calls
+ * (pg_kinetic_precondition, pg_potential_scpol_add; at most 256 MiB) and the
+ * buffers of pg_solve (at most 1 GiB), together at most 2 GiB over all grids of
+ * the process.  It is given back when the grid is destroyed, when an allocation
+ * of this library would fail otherwise, and by pg_release_buffers, which frees
+ * what grids without a call in progress keep and returns the bytes. */
+long pg_release_buffers(void);
 
 /* ------------------------------------------------------------------ kinetic */
 
@@ -365,12 +372,13 @@ pg_status pg_davidson_set_preconditioner(pg_davidson* d, const pg_grid* g, int p
 /* The kinetic preconditioner on its own: R <- (T - sigma_j)^-1 R for the k
  * contiguous vectors R (device, N each, 16-byte aligned for the FP16 kernel),
  * sigma[k] on the host; |T - sigma_j| is kept at least a tenth of the lowest
- * kinetic level.  PG_FP64: six FP64 axis passes and a diagonal scale; PG_MIXED:
+ * kinetic level.  PG_FP64: six FP64 axis passes (as pg_hx) and a diagonal scale; PG_MIXED:
  * where every axis has the same n <= 96 (n even), one FP16-split tensor-core
  * kernel (k_kin_f16: per vector, xy forward transforms of the planes, z
  * forward transform + diagonal + z backward transform of 128-line tiles, xy
- * backward transforms), else six split-TF32 axis passes.  Allocates 2 k N
- * doubles of scratch and synchronises the stream.  No reference counterpart
+ * backward transforms), else six split-TF32 axis passes.  Takes 2 k N doubles
+ * of scratch (kept with the grid, pg_release_buffers) and synchronises the
+ * stream.  No reference counterpart
  * (corrflag 3 is this library's own). */
 pg_status pg_kinetic_precondition(const pg_grid* g, double* R, int k, const double* sigma, int precision,
                                   void* stream);

@@ -104,6 +104,7 @@ SYMBOLS = {
     "pg_version": (C.c_int, []),
     "pg_kernel_launches": (C.c_long, []),
     "pg_device_allocations": (C.c_long, []),
+    "pg_release_buffers": (C.c_long, []),
     "pg_sine_dvr": (C.c_int, [C.c_int, C.c_double, C.c_double, C.c_double, _dp, _dp, C.c_int]),
     "pg_grid_create": (C.c_int, [_ip, _dp, C.POINTER(_vp)]),
     "pg_grid_create_dvr": (C.c_int, [_ip, _dp, C.c_int, C.POINTER(_vp)]),

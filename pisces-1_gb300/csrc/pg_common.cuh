@@ -77,7 +77,12 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, const 
   return e;
 }
 
-// Device buffer owned by RAII (cudaMalloc/cudaFree).
+// Frees the buffers that idle grids keep between calls (pg_keep.cu); the bytes
+// given back.
+size_t release_kept();
+
+// Device buffer owned by RAII (cudaMalloc/cudaFree).  An allocation that fails
+// is tried again once without the kept buffers.
 template <class T>
 struct DevBuf {
   T* p = nullptr;
@@ -90,7 +95,12 @@ struct DevBuf {
     release();
     if (count == 0) return PG_OK;
     count_device_alloc();
-    if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) {
+    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      if (release_kept() > 0) e = cudaMalloc(&p, count * sizeof(T));
+    }
+    if (e != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
       set_error("cudaMalloc of %zu bytes failed", count * sizeof(T));
@@ -301,8 +311,9 @@ struct pg_grid {
   mutable std::map<std::pair<const void*, int>, TensorMapPair> tmaps;
   // device scratch of calls that wait for their stream before they return,
   // and the buffers of pg_solve, kept between calls (pg_keep.cu); freed with
-  // the grid
-  mutable std::mutex scratch_m, solve_m;
+  // the grid, by release_kept, or where an allocation fails.  A buffer is its
+  // holder's alone while its flag is set.
+  mutable std::atomic<bool> scratch_busy{false}, solve_busy{false};
   mutable pg::DevBuf<unsigned char> scratch;
   mutable std::shared_ptr<pg::SolveWorkspace> solve_ws;
   mutable size_t solve_kept = 0;
@@ -323,7 +334,7 @@ class ScratchLease {
  private:
   const pg_grid* g_;
   cudaStream_t st_;
-  std::unique_lock<std::mutex> lock_;
+  bool held_ = false;  // the grid's buffer
   DevBuf<unsigned char> own_;
 };
 
@@ -339,7 +350,7 @@ class SolveLease {
  private:
   const pg_grid* g_;
   cudaStream_t st_;
-  std::unique_lock<std::mutex> lock_;
+  bool held_;  // the grid's buffers
   std::shared_ptr<SolveWorkspace> ws_;
 };
 

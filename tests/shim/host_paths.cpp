@@ -189,6 +189,58 @@ int slice_grids() {
   return 0;
 }
 
+// What grids keep between calls is given back: on request, with the grid, and
+// before an allocation is given up.
+int kept_buffers() {
+  pg_grid *a = grid(30, 20, 20), *b = grid(66, 20, 20);
+  const long N = pg_grid_npoints(b);
+  std::vector<double> r(8 * N), v(N), vec(2 * N), ev(2);
+  const std::vector<double> sigma(8, -0.1);
+  auto precondition = [&](pg_grid* g, int k) {
+    return pg_kinetic_precondition(g, r.data(), k, sigma.data(), PG_FP64, nullptr);
+  };
+  REQUIRE(pg_release_buffers() == 0);
+  const size_t bare = fake::kept_on(0);
+  REQUIRE(precondition(b, 4) == PG_OK);
+  const size_t kept = fake::kept_on(0) - bare;
+  REQUIRE(kept >= 8u * 8u * (size_t)N);
+  REQUIRE(precondition(b, 2) == PG_OK && fake::kept_on(0) - bare == kept);
+  REQUIRE(pg_release_buffers() == (long)kept && fake::kept_on(0) == bare);
+  // no room for a's scratch but b's
+  REQUIRE(precondition(b, 4) == PG_OK);
+  fake::state().memory = fake::state().in_use + 1000;
+  REQUIRE(precondition(a, 4) == PG_OK);
+  REQUIRE(precondition(b, 4) == PG_OK);
+  // nothing to give back: refused, and the grid is as it was
+  fake::state().memory = bare + 1000;
+  pg_release_buffers();
+  REQUIRE(precondition(a, 4) == PG_OOM);
+  fake::state().memory = (size_t)-1;
+  REQUIRE(precondition(a, 4) == PG_OK);
+  pg_release_buffers();
+  // the buffers of a solve
+  pg_solve_params p{};
+  p.nroots = 2;
+  p.maxsub = 8;
+  p.maxiter = 1;
+  p.ptol = 5;
+  p.corrflag = 1;
+  p.startvec = 1;
+  pg_solve(b, v.data(), &p, ev.data(), vec.data(), nullptr, nullptr);
+  const size_t solve = fake::kept_on(0);
+  REQUIRE(solve >= bare + 2u * 8u * 8u * (size_t)N);
+  fake::state().memory = fake::state().in_use + 1000;
+  REQUIRE(precondition(a, 4) == PG_OK);
+  REQUIRE(fake::kept_on(0) < solve);
+  fake::state().memory = (size_t)-1;
+  pg_solve(b, v.data(), &p, ev.data(), vec.data(), nullptr, nullptr);
+  pg_grid_destroy(b);
+  REQUIRE(precondition(a, 4) == PG_OK);
+  pg_grid_destroy(a);
+  REQUIRE(pg_release_buffers() == 0);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -199,6 +251,7 @@ int main(int argc, char** argv) {
       {"second_device", second_device},
       {"potential_tables", potential_tables},
       {"slice_grids", slice_grids},
+      {"kept_buffers", kept_buffers},
   };
   const auto it = cases.find(argc > 1 ? argv[1] : "");
   return it == cases.end() ? 2 : it->second();
