@@ -119,6 +119,19 @@ struct DevBuf {
   }
 };
 
+// Zeroes device memory, complete on return and for every stream: on a stream
+// of its own, since non-blocking streams do not wait for the legacy one and a
+// stream that is being captured would only record it.
+inline pg_status zero_now(void* p, size_t bytes) {
+  cudaStream_t st = nullptr;
+  PG_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  cudaError_t e = cudaMemsetAsync(p, 0, bytes, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  PG_CUDA_TRY(e);
+  return PG_OK;
+}
+
 // Programmatic dependent launch.  A kernel launched by launch_dependent may
 // be scheduled before the kernel ahead of it in the stream has finished; it
 // must call pdl_wait() before it touches global memory (the wait returns once

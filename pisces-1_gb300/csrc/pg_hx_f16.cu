@@ -639,8 +639,7 @@ static pg_status f16_counters(const pg_grid* g, cudaStream_t st, F16Counters** o
     }
     std::unique_ptr<DevBuf<unsigned>> b(new DevBuf<unsigned>());
     PG_TRY(b->alloc(sizeof(F16Counters) / sizeof(unsigned)));
-    // zeroed on the stream that uses it: other streams do not wait for the legacy one
-    PG_CUDA_TRY(cudaMemsetAsync(b->p, 0, sizeof(F16Counters), st));
+    PG_TRY(zero_now(b->p, sizeof(F16Counters)));
     it = g->fused_cnt.emplace(key, std::move(b)).first;
   }
   *out = reinterpret_cast<F16Counters*>(it->second->p);

@@ -919,8 +919,7 @@ static pg_status fused_counters(const pg_grid* g, cudaStream_t st, FusedCounters
     }
     std::unique_ptr<DevBuf<unsigned>> b(new DevBuf<unsigned>());
     PG_TRY(b->alloc(sizeof(FusedCounters) / sizeof(unsigned)));
-    // zeroed on the stream that uses it: other streams do not wait for the legacy one
-    PG_CUDA_TRY(cudaMemsetAsync(b->p, 0, sizeof(FusedCounters), st));
+    PG_TRY(zero_now(b->p, sizeof(FusedCounters)));
     it = g->fused_cnt.emplace(id, std::move(b)).first;
   }
   *out = reinterpret_cast<FusedCounters*>(it->second->p);

@@ -874,8 +874,7 @@ static pg_status kin_counters(const pg_grid* g, cudaStream_t st, KinCounters** o
     }
     std::unique_ptr<DevBuf<unsigned>> b(new DevBuf<unsigned>());
     PG_TRY(b->alloc(sizeof(KinCounters) / sizeof(unsigned)));
-    // zeroed on the stream that uses it: other streams do not wait for the legacy one
-    PG_CUDA_TRY(cudaMemsetAsync(b->p, 0, sizeof(KinCounters), st));
+    PG_TRY(zero_now(b->p, sizeof(KinCounters)));
     it = g->fused_cnt.emplace(key, std::move(b)).first;
   }
   *out = reinterpret_cast<KinCounters*>(it->second->p);

@@ -900,9 +900,7 @@ pg_status RedScratch::ensure(cudaStream_t st) {
   if (!partial.p) PG_TRY(partial.alloc((size_t)kRedBlocks * kMaxGramOut));
   if (!counter.p) {
     PG_TRY(counter.alloc(1));
-    // complete before any stream can use it (none waits for the legacy stream)
-    PG_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned), st));
-    PG_CUDA_TRY(cudaStreamSynchronize(st));
+    PG_TRY(zero_now(counter.p, sizeof(unsigned)));
   }
   return PG_OK;
 }

@@ -17,6 +17,7 @@ std::recursive_mutex m;
 std::map<cudaStream_t, std::vector<Copy>> pending;
 std::map<void*, std::pair<size_t, int>> device_blocks;
 std::map<const void*, size_t> pinned_sizes;
+std::set<cudaStream_t> own_streams;
 std::map<const void*, std::string>& names() {
   static std::map<const void*, std::string> n;
   return n;
@@ -32,6 +33,8 @@ void flush(cudaStream_t st) {
   for (auto& c : pending[st]) memcpy(c.dst, c.src, c.n);
   pending[st].clear();
 }
+
+bool captured(cudaStream_t st) { return fake::state().capturing && !own_streams.count(st); }
 
 cudaError_t launch(const void* f, dim3 grid, size_t smem, void** args) {
   std::lock_guard<std::recursive_mutex> l(m);
@@ -118,7 +121,7 @@ cudaError_t cudaMalloc(void** p, size_t n) {
     return cudaErrorMemoryAllocation;
   }
   *p = aligned_alloc(256, (n + 255) / 256 * 256);
-  memset(*p, 0, (n + 255) / 256 * 256);
+  memset(*p, 0xff, (n + 255) / 256 * 256);
   device_blocks[*p] = {n, s.device};
   s.in_use += n;
   return cudaSuccess;
@@ -161,20 +164,22 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
   memmove(d, s, n);
   return cudaSuccess;
 }
-cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
-  memset(d, v, n);
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t st) {
+  std::lock_guard<std::recursive_mutex> l(m);
+  if (captured(st)) fake::state().recorded += 1;
+  else memset(d, v, n);
   return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) {
   std::lock_guard<std::recursive_mutex> l(m);
-  if (fake::state().capturing) return cudaErrorStreamCaptureUnsupported;
+  if (captured(st)) return cudaErrorStreamCaptureUnsupported;
   fake::state().waits += 1;
   flush(st);
   if (fake::state().on_wait) fake::state().on_wait();
   return cudaSuccess;
 }
-cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
-  *s = fake::state().capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+cudaError_t cudaStreamIsCapturing(cudaStream_t st, cudaStreamCaptureStatus* s) {
+  *s = captured(st) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
@@ -210,6 +215,26 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 cudaError_t cudaStreamGetId(cudaStream_t st, unsigned long long* id) {
   *id = (unsigned long long)(size_t)st;
+  return cudaSuccess;
+}
+
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* st, unsigned) {
+  std::lock_guard<std::recursive_mutex> l(m);
+  *st = (cudaStream_t)malloc(1);
+  own_streams.insert(*st);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t st) {
+  std::lock_guard<std::recursive_mutex> l(m);
+  own_streams.erase(st);
+  free(st);
+  return cudaSuccess;
+}
+static int encode_stub(...) { return 0; }
+cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* q) {
+  *f = (void*)encode_stub;
+  if (q) *q = cudaDriverEntryPointSuccess;
   return cudaSuccess;
 }
 

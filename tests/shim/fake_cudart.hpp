@@ -23,7 +23,8 @@ struct State {
   int fail_mallocs = 0;          // the next cudaMalloc calls that fail
   size_t memory = (size_t)-1;    // device bytes in all; cudaMalloc fails past them
   size_t in_use = 0;
-  bool capturing = false;        // every stream is being captured: a wait is an error
+  bool capturing = false;        // every stream but the library's own is being captured: a wait is an error
+  int recorded = 0;              // memsets that a capture only records
   int waits = 0;                 // cudaStreamSynchronize calls
   // dynamic shared memory opted into, per device and kernel name
   std::map<std::pair<int, std::string>, int> opted_in;

@@ -241,6 +241,24 @@ int kept_buffers() {
   return 0;
 }
 
+// Work counters of a stream whose first use is captured: zero when the call
+// returns, not once the graph has run (the stream may be used before).
+int captured_counters() {
+  pg_grid* g = grid(32, 32, 32);
+  const long N = g ? pg_grid_npoints(g) : 1;
+  std::vector<double> buf(4 * N + 2);
+  double* x = buf.data() + ((size_t)buf.data() % 16 ? 1 : 0);
+  for (int kind : {3, 2}) {  // FP16 split, TF32 split
+    REQUIRE(pg_grid_set_hx_kernel(g, kind) == PG_OK);
+    fake::state().capturing = true;
+    REQUIRE(pg_hx_async(g, x + 2 * N, x, x + N, 1, PG_MIXED, nullptr) == PG_OK);
+    REQUIRE(fake::state().recorded == 0);
+    fake::state().capturing = false;
+  }
+  pg_grid_destroy(g);
+  return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -252,6 +270,7 @@ int main(int argc, char** argv) {
       {"potential_tables", potential_tables},
       {"slice_grids", slice_grids},
       {"kept_buffers", kept_buffers},
+      {"captured_counters", captured_counters},
   };
   const auto it = cases.find(argc > 1 ? argv[1] : "");
   return it == cases.end() ? 2 : it->second();

@@ -31,7 +31,7 @@ def program(pg, tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["scpol_upload", "hx_status", "hx_captured", "second_device", "potential_tables", "slice_grids",
-                                  "kept_buffers"])
+                                  "kept_buffers", "captured_counters"])
 def test_host_path(program, case):
     r = subprocess.run([program, case], env=dict(os.environ, MALLOC_PERTURB_="165"), capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
