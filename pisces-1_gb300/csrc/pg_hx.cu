@@ -18,46 +18,45 @@
 
 namespace {
 
-// One thread owns one grid point for up to four vectors (four independent
-// accumulators); operand loads are coalesced or warp-wide broadcasts.
+// One thread owns one grid point for four vectors (four independent
+// accumulators), in the last group of blocks for the REST that are left over;
+// operand loads are coalesced or warp-wide broadcasts.  Every vector of a body
+// exists: one left out by a predicate would take the FP64 pipe as long as any
+// other, and the predicates keep the loads from running ahead.  All groups are
+// one launch: on small grids the ones left over cost as much time as a group
+// of four, beside which they now run.
 template <int NV>
-__global__ void __launch_bounds__(256) k_hx_fp64(int nx, int ny, int nz, const double* __restrict__ tx,
-                                                 const double* __restrict__ ty, const double* __restrict__ tz,
-                                                 const double* __restrict__ v, const double* __restrict__ X,
-                                                 double* __restrict__ Y, int nvec) {
-  const long N = (long)nx * ny * nz;
-  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int v0 = blockIdx.y * NV;
-  if (g >= N) return;
+__device__ __forceinline__ void hx_point(int nx, int ny, int nz, const double* __restrict__ tx,
+                                         const double* __restrict__ ty, const double* __restrict__ tz,
+                                         const double* __restrict__ v, const double* __restrict__ Xv,
+                                         double* __restrict__ Yv, long N, long g) {
   const int i = (int)(g % nx);
   const long r = g / nx;
   const int j = (int)(r % ny);
   const int k = (int)(r / ny);
-  const int nv = nvec - v0 < NV ? nvec - v0 : NV;
-  const double* Xv = X + (long)v0 * N;
   double acc[NV];
   const double vg = v[g];
 #pragma unroll
-  for (int q = 0; q < NV; ++q) acc[q] = q < nv ? vg * Xv[(long)q * N + g] : 0.0;
+  for (int q = 0; q < NV; ++q) acc[q] = vg * Xv[(long)q * N + g];
   // x sweep: T[b][i] (coalesced over i), x[b,j,k] broadcast
   {
     const long base = (long)nx * (j + (long)ny * k);
+#pragma unroll 4
     for (int b = 0; b < nx; ++b) {
       const double t = tx[(long)b * nx + i];
 #pragma unroll
-      for (int q = 0; q < NV; ++q)
-        if (q < nv) acc[q] += t * Xv[(long)q * N + base + b];
+      for (int q = 0; q < NV; ++q) acc[q] += t * Xv[(long)q * N + base + b];
     }
   }
   // y sweep: Ty[j][b] broadcast, x[i,b,k] coalesced
   {
     const long base = i + (long)nx * ny * k;
     const double* trow = ty + (long)j * ny;
+#pragma unroll 4
     for (int b = 0; b < ny; ++b) {
       const double t = trow[b];
 #pragma unroll
-      for (int q = 0; q < NV; ++q)
-        if (q < nv) acc[q] += t * Xv[(long)q * N + base + (long)nx * b];
+      for (int q = 0; q < NV; ++q) acc[q] += t * Xv[(long)q * N + base + (long)nx * b];
     }
   }
   // z sweep: Tz[k][b] broadcast, x[i,j,b] coalesced
@@ -65,26 +64,56 @@ __global__ void __launch_bounds__(256) k_hx_fp64(int nx, int ny, int nz, const d
     const long base = i + (long)nx * j;
     const long sz = (long)nx * ny;
     const double* trow = tz + (long)k * nz;
+#pragma unroll 4
     for (int b = 0; b < nz; ++b) {
       const double t = trow[b];
 #pragma unroll
-      for (int q = 0; q < NV; ++q)
-        if (q < nv) acc[q] += t * Xv[(long)q * N + base + sz * b];
+      for (int q = 0; q < NV; ++q) acc[q] += t * Xv[(long)q * N + base + sz * b];
     }
   }
 #pragma unroll
-  for (int q = 0; q < NV; ++q)
-    if (q < nv) Y[(long)(v0 + q) * N + g] = acc[q];
+  for (int q = 0; q < NV; ++q) Yv[(long)q * N + g] = acc[q];
+}
+
+// Groups blockIdx.y < four take four vectors each, the next one the REST.
+template <int REST>
+__global__ void __launch_bounds__(256) k_hx_fp64(int nx, int ny, int nz, const double* __restrict__ tx,
+                                                 const double* __restrict__ ty, const double* __restrict__ tz,
+                                                 const double* __restrict__ v, const double* __restrict__ X,
+                                                 double* __restrict__ Y, int four) {
+  const long N = (long)nx * ny * nz;
+  const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (g >= N) return;
+  const long off = 4l * blockIdx.y * N;
+  if (REST == 0 || (int)blockIdx.y < four) hx_point<4>(nx, ny, nz, tx, ty, tz, v, X + off, Y + off, N, g);
+  else hx_point<REST == 0 ? 4 : REST>(nx, ny, nz, tx, ty, tz, v, X + off, Y + off, N, g);
 }
 
 // Y (mode) A x_axis X: one axis contraction in FP64, mode 0 write, 1 add.
 template <int NV>
+__device__ __forceinline__ void axis_point(int na, int idx, long stride, const double* __restrict__ A,
+                                           const double* __restrict__ Xv, double* __restrict__ Yv, long N, long g,
+                                           int mode) {
+  const long base = g - (long)idx * stride;
+  double acc[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) acc[q] = mode == 1 ? Yv[(long)q * N + g] : 0.0;
+  const double* arow = A + (long)idx * na;
+  for (int b = 0; b < na; ++b) {
+    const double t = arow[b];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) acc[q] += t * Xv[(long)q * N + base + (long)b * stride];
+  }
+#pragma unroll
+  for (int q = 0; q < NV; ++q) Yv[(long)q * N + g] = acc[q];
+}
+
+template <int REST>
 __global__ void __launch_bounds__(256) k_axis_fp64(int nx, int ny, int nz, int axis, const double* __restrict__ A,
-                                                   const double* __restrict__ X, double* __restrict__ Y, int nvec,
+                                                   const double* __restrict__ X, double* __restrict__ Y, int four,
                                                    int mode) {
   const long N = (long)nx * ny * nz;
   const long g = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int v0 = blockIdx.y * NV;
   if (g >= N) return;
   const int i = (int)(g % nx);
   const long r = g / nx;
@@ -93,21 +122,9 @@ __global__ void __launch_bounds__(256) k_axis_fp64(int nx, int ny, int nz, int a
   const int na = axis == 0 ? nx : (axis == 1 ? ny : nz);
   const int idx = axis == 0 ? i : (axis == 1 ? j : k);
   const long stride = axis == 0 ? 1 : (axis == 1 ? nx : (long)nx * ny);
-  const long base = g - (long)idx * stride;
-  const int nv = nvec - v0 < NV ? nvec - v0 : NV;
-  double acc[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) acc[q] = (q < nv && mode == 1) ? Y[(long)(v0 + q) * N + g] : 0.0;
-  const double* arow = A + (long)idx * na;
-  for (int b = 0; b < na; ++b) {
-    const double t = arow[b];
-#pragma unroll
-    for (int q = 0; q < NV; ++q)
-      if (q < nv) acc[q] += t * X[(long)(v0 + q) * N + base + (long)b * stride];
-  }
-#pragma unroll
-  for (int q = 0; q < NV; ++q)
-    if (q < nv) Y[(long)(v0 + q) * N + g] = acc[q];
+  const long off = 4l * blockIdx.y * N;
+  if (REST == 0 || (int)blockIdx.y < four) axis_point<4>(na, idx, stride, A, X + off, Y + off, N, g, mode);
+  else axis_point<REST == 0 ? 4 : REST>(na, idx, stride, A, X + off, Y + off, N, g, mode);
 }
 
 }  // namespace
@@ -117,17 +134,18 @@ namespace pg {
 pg_status tc_axis(const pg_grid* g, int a, const float* Ahi, const float* Alo, const double* v, const double* x,
                   double* y, int nvec, int mode, cudaStream_t st);
 
-// The in-order kernels over nvec vectors: groups of four, then the one to
-// three that are left with a kernel of their own (a vector left out by a
-// predicate takes the FP64 pipe as long as any other: an FP64 solve of 2
-// states on 64^3 31 ms with groups of four alone, 17 so; of 3 on 48^3 16 / 12).
+// Launches an in-order kernel over nvec vectors: launch(REST, blocks, four).
+// A launch for the groups of four and one for the rest took, for 5 vectors on
+// 12^3 / 28^3 / 64^3, 25.1 / 51.8 / 474 us, one launch of predicated groups 16.7 /
+// 50.6 / 716, and one launch with a body for the rest 16.6 / 31.3 / 417.
 template <typename F>
-static void by_vectors(int nvec, const F& launch) {
-  const int four = nvec / 4, v0 = 4 * four;
-  if (four > 0) launch(std::integral_constant<int, 4>(), 0, four);
-  if (nvec - v0 == 1) launch(std::integral_constant<int, 1>(), v0, 1);
-  if (nvec - v0 == 2) launch(std::integral_constant<int, 2>(), v0, 1);
-  if (nvec - v0 == 3) launch(std::integral_constant<int, 3>(), v0, 1);
+static void by_vectors(long N, int nvec, const F& launch) {
+  const int four = nvec / 4, rest = nvec % 4;
+  const dim3 blocks((unsigned)((N + 255) / 256), (unsigned)(four + (rest ? 1 : 0)));
+  if (rest == 0) launch(std::integral_constant<int, 0>(), blocks, four);
+  if (rest == 1) launch(std::integral_constant<int, 1>(), blocks, four);
+  if (rest == 2) launch(std::integral_constant<int, 2>(), blocks, four);
+  if (rest == 3) launch(std::integral_constant<int, 3>(), blocks, four);
 }
 
 pg_status axis_apply(const pg_grid* g, int axis, const SliceMat& S, const double* A64, const float* Ahi,
@@ -136,9 +154,8 @@ pg_status axis_apply(const pg_grid* g, int axis, const SliceMat& S, const double
   PG_ARG(g && x && y && x != y && axis >= 0 && axis < 3 && (mode == 0 || mode == 1), "axis_apply: bad arguments");
   if (precision == PG_MIXED) return tc_axis(g, axis, Ahi, Alo, nullptr, x, y, nvec, mode, st);
   if (!in_order) return slice_axis(g, axis, S, A64, nullptr, x, y, nvec, mode, st);
-  by_vectors(nvec, [&](auto nv, int v0, int groups) {
-    k_axis_fp64<nv.value><<<dim3((unsigned)((g->N + 255) / 256), (unsigned)groups), 256, 0, st>>>(
-        g->n[0], g->n[1], g->n[2], axis, A64, x + (long)v0 * g->N, y + (long)v0 * g->N, nvec - v0, mode);
+  by_vectors(g->N, nvec, [&](auto rest, dim3 blocks, int four) {
+    k_axis_fp64<rest.value><<<blocks, 256, 0, st>>>(g->n[0], g->n[1], g->n[2], axis, A64, x, y, four, mode);
   });
   return check_launch("k_axis_fp64");
 }
@@ -157,10 +174,9 @@ pg_status hx(const pg_grid* g, const double* v, const double* x, double* y, int 
   // where the slices would round T's small entries further than the chain of
   // multiply-adds rounds (a sine-DVR axis above about 750 points): the chain
   if (in_order || !g->t_sliced) {
-    by_vectors(nvec, [&](auto nv, int v0, int groups) {
-      k_hx_fp64<nv.value><<<dim3((unsigned)((g->N + 255) / 256), (unsigned)groups), 256, 0, st>>>(
-          g->n[0], g->n[1], g->n[2], g->t_dev[0].p, g->t_dev[1].p, g->t_dev[2].p, v, x + (long)v0 * g->N,
-          y + (long)v0 * g->N, nvec - v0);
+    by_vectors(g->N, nvec, [&](auto rest, dim3 blocks, int four) {
+      k_hx_fp64<rest.value><<<blocks, 256, 0, st>>>(g->n[0], g->n[1], g->n[2], g->t_dev[0].p, g->t_dev[1].p,
+                                                    g->t_dev[2].p, v, x, y, four);
     });
     return check_launch("k_hx_fp64");
   }
