@@ -63,16 +63,13 @@ inline pg_status check_launch(const char* what) {
   return PG_OK;
 }
 
-// Runs set() once for every device it is called on: a kernel's attributes
-// belong to the device that was current when they were set.
+// Runs set() once for every device it is called on, the current one: a
+// kernel's attributes belong to the device that was current when they were set.
 template <class Set>
-inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, const Set& set) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, int device, const Set& set) {
+  const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
   if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-  e = set();
+  const cudaError_t e = set();
   if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
   return e;
 }

@@ -12,6 +12,7 @@
 // out of a restart with signs that the rounding noise of the products
 // decides: with another product the states are the same to 1e-14, but a third
 // of them change sign, and a solve keeps the states it has always returned.
+#include <algorithm>
 #include <type_traits>
 
 #include "pg_slice.cuh"
@@ -160,6 +161,21 @@ pg_status axis_apply(const pg_grid* g, int axis, const SliceMat& S, const double
   return check_launch("k_axis_fp64");
 }
 
+// Whether the chain of multiply-adds is as fast as the slices, for this grid and
+// block.  Its one launch lasts as long as the FP64 pipe needs for a block of
+// 256 points on an SM, 78 ns for each multiply-add of a point, times the turns
+// its blocks take; the slices' three launches take 21 to 27 us on grids that
+// small, whatever their size (back to back, us, chain / slices: 8^3 x 1 9 / 21,
+// 12^3 x 8 17 / 21, 16^3 x 40 30 / 26).  Up to 36 multiply-adds a value, whose
+// roundings stay near the slices' few; longer chains round more (on 15x17x16
+// beyond four roundings of a value's terms) and are not taken for speed.
+static bool chain_is_shorter(const pg_grid* g, int nvec) {
+  const long blocks = (g->N + 255) / 256 * ((nvec + 3) / 4);
+  const long sms = sm_count(g->device);
+  const int terms = g->n[0] + g->n[1] + g->n[2];
+  return terms <= 36 && (long)terms * std::min(nvec, 4) * ((blocks + sms - 1) / sms) <= 250;
+}
+
 pg_status hx_mixed(const pg_grid* g, const double* v, const double* x, double* y, int nvec, cudaStream_t st,
                    bool check, bool unit);
 
@@ -171,9 +187,9 @@ pg_status hx(const pg_grid* g, const double* v, const double* x, double* y, int 
   PG_ARG(x != y, "pg_hx: X and Y must not alias");
   if (precision == PG_MIXED) return hx_mixed(g, v, x, y, nvec, st, false, unit);
   PG_ARG(precision == PG_FP64, "pg_hx: unknown precision %d", precision);
-  // where the slices would round T's small entries further than the chain of
-  // multiply-adds rounds (a sine-DVR axis above about 750 points): the chain
-  if (in_order || !g->t_sliced) {
+  // !t_sliced: the slices would round T's small entries further than the chain
+  // rounds (a sine-DVR axis above about 750 points)
+  if (in_order || !g->t_sliced || chain_is_shorter(g, nvec)) {
     by_vectors(g->N, nvec, [&](auto rest, dim3 blocks, int four) {
       k_hx_fp64<rest.value><<<blocks, 256, 0, st>>>(g->n[0], g->n[1], g->n[2], g->t_dev[0].p, g->t_dev[1].p,
                                                     g->t_dev[2].p, v, x, y, four);

@@ -928,7 +928,9 @@ inline bool pair_ok(long N, const double* P, const double* Q) {
 // Dynamic shared-memory opt-in, once per kernel and device.
 static pg_status opt_in_smem() {
   static std::atomic<unsigned long long> done{0};
-  PG_CUDA_TRY(once_per_device(done, [] {
+  int dev = 0;
+  PG_CUDA_TRY(cudaGetDevice(&dev));
+  PG_CUDA_TRY(once_per_device(done, dev, [] {
     cudaError_t e = cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_gram_df<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmemMax);

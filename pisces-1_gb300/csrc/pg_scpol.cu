@@ -466,7 +466,7 @@ pg_status scpol_add_points(const pg_grid* g, const pg_sites* t, const pg_scpol_m
                                                              m->damp_type, m->damp, E);
     PG_TRY(pg::check_launch("k_scpol_field"));
     int rows = 0;
-    PG_TRY(slice_rows(np, md.mat, md.inva, E, part, kRowDot, &rows, g->tc_err.p, st));
+    PG_TRY(slice_rows(g, np, md.mat, md.inva, E, part, kRowDot, &rows, st));
     k_scpol_finish<<<stride_blocks(np), 256, 0, st>>>(p0, np, list, rows, part, m->vpol_ww, v, vpol);
     PG_TRY(pg::check_launch("k_scpol_finish"));
   }
@@ -559,7 +559,7 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
                                                              g->x_dev[1].p, g->x_dev[2].p, m->npp, md.pos, md.epc,
                                                              2, m->damp, E.p);
     PG_TRY(pg::check_launch("k_scpol_field"));
-    PG_TRY(pg::slice_rows(np, md.mat, md.inva, E.p, MU.p, pg::kRowStore, nullptr, g->tc_err.p, st));
+    PG_TRY(pg::slice_rows(g, np, md.mat, md.inva, E.p, MU.p, pg::kRowStore, nullptr, st));
     const int sb = (int)((np + site_per - 1) / site_per);
     k_grad_sites<<<sb, 256, 0, st>>>(p0, np, site_per, g->n[0], g->n[1], g->x_dev[0].p, g->x_dev[1].p,
                                      g->x_dev[2].p, psi, MU.p, n, ns, srec.p, t->charge_damp, m->damp, spart.p);

@@ -482,9 +482,9 @@ constexpr int kSmemMost = 226 * 1024;
 
 template <int NU, bool kChunks>
 cudaError_t launch_slice(const SliceArgs& a, dim3 grid, size_t smem, const unsigned char* img, const double* A64,
-                         const double* v, const double* x, double* y, int* err, cudaStream_t st) {
+                         const double* v, const double* x, double* y, int* err, cudaStream_t st, int device) {
   static std::atomic<unsigned long long> done{0};
-  const cudaError_t attr = pg::once_per_device(done, [] {
+  const cudaError_t attr = pg::once_per_device(done, device, [] {
     return cudaFuncSetAttribute(k_slice_axis<NU, kChunks>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
   });
   if (attr != cudaSuccess) return attr;
@@ -583,23 +583,23 @@ pg_status slice_grid(pg_grid* g) {
   return PG_OK;
 }
 
-namespace {
-
-// SMs of the current device.
-int sm_count() {
+int sm_count(int device) {
   static std::atomic<int> known[64];
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 152;
-  if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 152;
-  if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
+  int n = 0;
+  const bool slot = device >= 0 && device < 64;
+  if (slot && (n = known[device].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) return 152;
+  if (slot) known[device].store(n, std::memory_order_relaxed);
   return n;
 }
+
+namespace {
 
 // Launches the contraction of nlines lines (stride inner); mode 3 writes
 // *rows rows of nlines partial dots.
 pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, const double* A64, bool trans,
-                       const double* v, const double* x, double* y, int mode, int* rows, int* err, cudaStream_t st) {
+                       const double* v, const double* x, double* y, int mode, int* rows, int* err, cudaStream_t st,
+                       int device) {
   SliceArgs a{};
   a.n = S.n;
   a.inner = inner;
@@ -633,7 +633,7 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
   // scheduler's warps), its digits do not (64^3 x 1: 44 us with the lines
   // first, 34 so; 80^3 x 1 62 / 48, 160x60x60 x 1 91 / 63).
   const long full = (nlines + kLines - 1) / kLines;
-  const int sms = sm_count();
+  const int sms = sm_count(device);
   const int groups = (int)std::max<long>(1, std::min<long>(S.nnc, sms / full));
   a.nc_per = (S.nnc + groups - 1) / groups;
   const int split = (S.nnc + a.nc_per - 1) / a.nc_per;
@@ -650,9 +650,9 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
     a.mode = h0 == 0 || mode == 3 ? mode : 1;
     a.out0 = (long)launches * split * nlines;
     cudaError_t e;
-    if (chunks) e = launch_slice<2, true>(a, grid, smem, S.img, A64, v, x, y, err, st);
-    else if (S.kc <= 32) e = launch_slice<1, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
-    else e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, err, st);
+    if (chunks) e = launch_slice<2, true>(a, grid, smem, S.img, A64, v, x, y, err, st, device);
+    else if (S.kc <= 32) e = launch_slice<1, false>(a, grid, smem, S.img, A64, v, x, y, err, st, device);
+    else e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, err, st, device);
     PG_CUDA_TRY(e);
     PG_TRY(check_launch("k_slice_axis"));
   }
@@ -666,7 +666,7 @@ pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double
                      const double* x, double* y, int nvec, int mode, cudaStream_t st) {
   PG_ARG(S.img && S.n == g->n[axis], "slice_axis: no operand images");
   const long inner = axis == 0 ? 1 : (axis == 1 ? g->n[0] : (long)g->n[0] * g->n[1]);
-  return slice_launch(g->N / S.n * nvec, inner, g->N, S, A64, false, v, x, y, mode, nullptr, g->tc_err.p, st);
+  return slice_launch(g->N / S.n * nvec, inner, g->N, S, A64, false, v, x, y, mode, nullptr, g->tc_err.p, st, g->device);
 }
 
 int slice_row_count(int n) {
@@ -700,9 +700,9 @@ pg_status slice_rows_matrix(const double* A64, unsigned char* img, SliceMat* S, 
   return check_launch("k_slice_matrix");
 }
 
-pg_status slice_rows(long nlines, const SliceMat& S, const double* A64, const double* x, double* y, SliceRows mode,
-                     int* rows, int* err, cudaStream_t st) {
-  return slice_launch(nlines, 1, nlines * S.n, S, A64, true, nullptr, x, y, mode, rows, err, st);
+pg_status slice_rows(const pg_grid* g, long nlines, const SliceMat& S, const double* A64, const double* x, double* y,
+                     SliceRows mode, int* rows, cudaStream_t st) {
+  return slice_launch(nlines, 1, nlines * S.n, S, A64, true, nullptr, x, y, mode, rows, g->tc_err.p, st, g->device);
 }
 
 }  // namespace pg

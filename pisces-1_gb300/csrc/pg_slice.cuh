@@ -142,6 +142,9 @@ __device__ __forceinline__ double slice_join(const float* acc, int e) {
   return __longlong_as_double(lz >= 32 ? 0ll : (long long)r);
 }
 
+// SMs of a device.
+int sm_count(int device);
+
 // The images of every matrix of a grid (t_dev, q_dev, qb_dev), made on the
 // device in one launch; equal matrices share one image.
 pg_status slice_grid(pg_grid* g);
@@ -154,7 +157,7 @@ pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double
 // Rows times a matrix: X is nlines x n (row-major), A n x n.
 // kRowStore: Y = X A.  kRowDot: Y holds *rows rows of nlines values whose sum
 // over the rows is x . (x A) for each line (at most slice_row_count(n)).
-// A64 and the images (slice_rows_matrix) on the device; err as tc_err.
+// A64 and the images (slice_rows_matrix) on the device; g gives the status word.
 enum SliceRows { kRowStore = 0, kRowDot = 3 };
 int slice_row_count(int n);
 // Shape and bytes of the images of an n x n matrix whose largest entry is big
@@ -163,7 +166,7 @@ int slice_row_count(int n);
 // as for entries outside the slices' range, every line goes by multiply-adds.
 size_t slice_rows_shape(int n, double big, double low, SliceMat* S);
 pg_status slice_rows_matrix(const double* A64, unsigned char* img, SliceMat* S, cudaStream_t st);
-pg_status slice_rows(long nlines, const SliceMat& S, const double* A64, const double* x, double* y, SliceRows mode,
-                     int* rows, int* err, cudaStream_t st);
+pg_status slice_rows(const pg_grid* g, long nlines, const SliceMat& S, const double* A64, const double* x, double* y,
+                     SliceRows mode, int* rows, cudaStream_t st);
 
 }  // namespace pg
