@@ -283,16 +283,15 @@ pg_status pg_water_default_tables(int nw, const double* sites, const double* cha
  * that a restart leaves with a sign decided by rounding may come out with the
  * other one in a caller's loop around pg_davidson_rci and pg_hx.
  * PG_MIXED: kinetic contractions as split FP16 or TF32
- * tensor-core products accumulated in FP32, V*X in FP64.  Waits for the stream
- * and returns PG_DEVICE_TIMEOUT if a completion wait inside a kernel of this
- * grid timed out (Y is then incomplete); in FP64 on a stream that is being
- * captured it queues its launches and returns, and pg_grid_check reports after
- * the graph has run.  nvec = 0 does
- * nothing and accepts null X and Y.  Replaces DVR::MatrixTimesVector applied
+ * tensor-core products accumulated in FP32, V*X in FP64; the call waits for the
+ * stream and returns PG_DEVICE_TIMEOUT if a completion wait inside a kernel
+ * timed out (Y is then incomplete).  In FP64 it returns once its launches are
+ * queued: where a wait times out, the kernel computes what is left by
+ * multiply-adds.  nvec = 0 does nothing and accepts null X and Y.  Replaces DVR::MatrixTimesVector applied
  * vector by vector (src/mtx.cpp:22-109, src/davdriver.cpp:67-78). */
 pg_status pg_hx(const pg_grid* g, const double* v_dev, const double* x_dev, double* y_dev, int nvec, int precision,
                 void* stream);
-/* pg_hx without the completion check: returns once the
+/* pg_hx without the completion check of the mixed form: returns once the
  * launches are queued (no host wait).  A tensor-core completion wait that
  * timed out is recorded in the grid's status word and reported by the next
  * pg_grid_check. */

@@ -271,7 +271,9 @@ extern "C" pg_status pg_kinetic_precondition(const pg_grid* g, double* R, int k,
   PG_TRY(pg::kinetic_precondition(g, R, k, sigma, reinterpret_cast<double*>(w), reinterpret_cast<double*>(w + wb),
                                   precision, st));
   // waits for the stream: the scratch is the next call's
-  return pg::check_tc_error(g, st);
+  if (precision == PG_MIXED) return pg::check_tc_error(g, st);
+  PG_CUDA_TRY(cudaStreamSynchronize(st));
+  return PG_OK;
 }
 
 extern "C" pg_status pg_grid_set_precond_kernel(pg_grid* g, int kind) {
@@ -992,7 +994,8 @@ pg_status solve_with(const pg_grid* g, const double* v, const pg_solve_params* p
   } else {
     PG_CUDA_TRY(cudaMemcpyAsync(evecs, B.p, sizeof(double) * N * nr, cudaMemcpyDeviceToDevice, st));
   }
-  PG_TRY(check_tc_error(g, st));  // waits for the stream
+  if (p->precision == PG_MIXED) PG_TRY(check_tc_error(g, st));  // waits for the stream
+  else PG_CUDA_TRY(cudaStreamSynchronize(st));
   if (stats) {
     memset(stats, 0, sizeof(*stats));
     stats->nconv = nconv;

@@ -470,7 +470,8 @@ pg_status scpol_add_points(const pg_grid* g, const pg_sites* t, const pg_scpol_m
     k_scpol_finish<<<stride_blocks(np), 256, 0, st>>>(p0, np, list, rows, part, m->vpol_ww, v, vpol);
     PG_TRY(pg::check_launch("k_scpol_finish"));
   }
-  return check_tc_error(g, st);  // waits for the stream
+  PG_CUDA_TRY(cudaStreamSynchronize(st));
+  return PG_OK;
 }
 
 }  // namespace pg
@@ -575,7 +576,7 @@ extern "C" pg_status pg_hf_gradient_grid(const pg_grid* g, const pg_sites* t, co
   std::vector<double> h(m1);
   PG_CUDA_TRY(cudaMemcpyAsync(h.data(), tot.p, sizeof(double) * m1, cudaMemcpyDeviceToHost, st));
   PG_CUDA_TRY(cudaMemcpyAsync(mcm, C.p, sizeof(double) * n * n, cudaMemcpyDeviceToHost, st));
-  PG_TRY(pg::check_tc_error(g, st));  // waits for the stream
+  PG_CUDA_TRY(cudaStreamSynchronize(st));
   std::memcpy(grad, h.data(), sizeof(double) * 3 * ns);
   std::memcpy(tmu, h.data() + 3 * ns, sizeof(double) * n);
   return PG_OK;

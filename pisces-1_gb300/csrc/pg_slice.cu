@@ -29,6 +29,20 @@
 
 namespace {
 
+// Polls of a barrier after which its waiters carry on by multiply-adds.
+#ifndef PG_SLICE_POLLS
+#define PG_SLICE_POLLS (1l << 26)
+#endif
+#ifndef PG_SLICE_POLLS_ISSUE
+#define PG_SLICE_POLLS_ISSUE (1l << 26)
+#endif
+template <long kPolls>
+__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity) {
+  for (long it = 0; it < kPolls; ++it)
+    if (mbar_try(bar, parity)) return true;
+  return false;
+}
+
 constexpr int kLines = 128;  // MMA M
 constexpr int kST = 512;     // threads that fill and read out
 constexpr int kTransMost = (kST / 32) * 32 * 5 * 8;  // transpose buffer: 32 lines x 4 columns per warp
@@ -67,17 +81,20 @@ struct SliceArgs {
 // waits for the matrix blocks and for the accumulators to be read: issued
 // by a thread that also reads out, two chunks of 64^3 took 5600 cycles before
 // its read-out began.
+// Every wait is bounded, and Y does not depend on them: where one runs out, the
+// outputs that it was for are computed by FP64 multiply-adds, as for lines
+// outside the slices' range.  Copies and products in flight are waited for
+// again before the block gives its memory back.
 template <int NU, bool kChunks>
 __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     k_slice_axis(const SliceArgs A, const unsigned char* __restrict__ img, const double* __restrict__ A64,
-                 const double* __restrict__ v, const double* __restrict__ x, double* y, int* __restrict__ err) {
+                 const double* __restrict__ v, const double* __restrict__ x, double* y) {
   constexpr int NS = pg::kSliceN;
   constexpr int kBuf = kChunks ? 1 : 2;  // matrix blocks and accumulator sets
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar_b[kBuf], bar_mma[kBuf], bar_read[kBuf];
   __shared__ uint32_t tmem_base;
   __shared__ int s_emax[kLines];
-  __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c_first = blockIdx.y * A.nc_per;
   const int c_end = c_first + A.nc_per < A.nnc ? c_first + A.nc_per : A.nnc;
@@ -96,7 +113,6 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
                  : "memory");
   };
   if (tid == 0) {
-    s_fail = 0;
     for (int b = 0; b < kBuf; ++b) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_b[b])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_mma[b])));
@@ -222,11 +238,7 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
   // lie side by side: at most 256 columns an instruction (one product at a
   // time reads the lines' digits once for each).
   auto issue = [&](int b, uint32_t parity, bool first) {
-    if (!mbar_wait(smem_u32(&bar_b[b]), parity)) {
-      s_fail = 1;
-      mbar_arrive(smem_u32(&bar_mma[b]));  // nothing was issued: release the others
-      return;
-    }
+    if (!wait_for<PG_SLICE_POLLS_ISSUE>(smem_u32(&bar_b[b]), parity)) return false;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint64_t dA = smem_desc(sA, lbo, sbo), dB = smem_desc(sB + (uint32_t)b * A.block_bytes, lbo, sbo);
     const uint32_t id0 = (1u << 4) | ((uint32_t)(kLines >> 4) << 24);
@@ -246,6 +258,13 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     }
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
         smem_u32(&bar_mma[b])));
+    return true;
+  };
+  // One thread: copies and products that it has issued, `loads` and `products`
+  // of them on the barriers of buffer b, are complete.
+  auto drain = [&](int b, int loads, int products) {
+    if (loads > 0) mbar_wait(smem_u32(&bar_b[b]), (uint32_t)((loads - 1) & 1));
+    if (products > 0) mbar_wait(smem_u32(&bar_mma[b]), (uint32_t)((products - 1) & 1));
   };
   // The four outputs of a read-out batch: four columns of the thread's own
   // line, or, where lines are contiguous and the batch is transposed, columns
@@ -292,20 +311,23 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
   // first column and address of this warp's first batch of N chunk c
   auto first_col = [&](int c) { return c * A.nc + 4 * wpart; };
   auto first_at = [&](int c) { return pbase + (long)first_col(c) * istep; };
-  auto readout = [&](int c, uint32_t tset, bool more) {
+  // mma false (the same for the lanes of a warp): without the accumulators
+  auto readout = [&](int c, uint32_t tset, bool more, bool mma) {
     if (!reads) return;
     const int em = s_emax[row];
-    const bool slow = is_slow(em);
+    const bool slow = is_slow(em) || !mma;
     const int emax = slow ? 0 : em;
     int i = first_col(c);
     long p = first_at(c);
     for (int bt = wpart; bt < nbatch; bt += 4, i += 16, p += 16 * istep) {
-      uint32_t r[pg::kSliceAcc][4];
+      uint32_t r[pg::kSliceAcc][4] = {};
+      if (mma) {
 #pragma unroll
-      for (int d = 0; d < pg::kSliceAcc; ++d)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(r[d][0]), "=r"(r[d][1]), "=r"(r[d][2]), "=r"(r[d][3])
-                     : "r"(trow + tset + (uint32_t)(d * A.nc + 4 * bt)));
+        for (int d = 0; d < pg::kSliceAcc; ++d)
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(r[d][0]), "=r"(r[d][1]), "=r"(r[d][2]), "=r"(r[d][3])
+                       : "r"(trow + tset + (uint32_t)(d * A.nc + 4 * bt)));
+      }
       double a0[4], b0[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) a0[q] = pa[q], b0[q] = pb[q];
@@ -384,27 +406,36 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
       prefetch(first_col(c_first), first_at(c_first));
       for (int c = c_first; c < c_end; ++c) {
         const int b = (c - c_first) & 1;
-        ok = mbar_wait(smem_u32(&bar_mma[b]), (uint32_t)((c - c_first) >> 1 & 1)) && !*(volatile int*)&s_fail && ok;
+        if (ok)
+          ok = __all_sync(0xffffffffu, wait_for<PG_SLICE_POLLS>(smem_u32(&bar_mma[b]),
+                                                               (uint32_t)((c - c_first) >> 1 & 1)));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         __syncwarp();
-        if (ok) readout(c, (uint32_t)b * (A.tmem_cols >> 1), c + 1 < c_end);
+        readout(c, (uint32_t)b * (A.tmem_cols >> 1), c + 1 < c_end, ok);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_read[b]));
+        // a warp that has given up is not counted: it may be chunks ahead
+        if (ok && lane == 0) mbar_arrive(smem_u32(&bar_read[b]));
       }
     } else if (lane == 0) {
-      for (int c = c_first; c < c_end; ++c) {
+      int loads[2] = {1, c_first + 1 < c_end ? 1 : 0}, products[2] = {0, 0};
+      for (int c = c_first; c < c_end && ok; ++c) {
         const int b = (c - c_first) & 1, use = (c - c_first) >> 1;
         if (use > 0) {
           // the matrix block is free once its products are done, the
           // accumulators once they are read
-          ok = mbar_wait(smem_u32(&bar_mma[b]), (uint32_t)((use - 1) & 1)) && ok;
+          ok = wait_for<PG_SLICE_POLLS_ISSUE>(smem_u32(&bar_mma[b]), (uint32_t)((use - 1) & 1));
+          if (!ok) break;
           load_b(c, 0, b);
-          ok = mbar_wait(smem_u32(&bar_read[b]), (uint32_t)((use - 1) & 1)) && ok;
+          ++loads[b];
+          ok = wait_for<PG_SLICE_POLLS_ISSUE>(smem_u32(&bar_read[b]), (uint32_t)((use - 1) & 1));
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        issue(b, (uint32_t)(use & 1), true);
+        ok = issue(b, (uint32_t)(use & 1), true);
+        if (ok) ++products[b];
       }
+      for (int b = 0; b < 2; ++b) drain(b, loads[b], products[b]);
     }
   } else {
     for (int h = 0; h < A.nch; ++h) {
@@ -412,31 +443,33 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
       chunk_emax();
       __syncthreads();
     }
-    uint32_t turn = 0;
-    for (int c = c_first; c < c_end && ok; ++c) {
+    int turn = 0, loads = 1, products = 0;
+    for (int c = c_first; c < c_end; ++c) {
       for (int h = 0; h < A.nch && ok; ++h, ++turn) {
         load_chunk(h);
         __syncthreads();  // the staging area is read
         convert();
         __syncthreads();
-        if (tid == 0) issue(0, turn & 1u, h == 0);
+        if (tid == 0) {
+          if (issue(0, (uint32_t)turn & 1u, h == 0)) ++products;
+        }
         if (h + 1 == A.nch) prefetch(first_col(c), first_at(c));
-        ok = __syncthreads_and(mbar_wait(smem_u32(&bar_mma[0]), turn & 1u) && !*(volatile int*)&s_fail) != 0;
+        ok = __syncthreads_and(wait_for<PG_SLICE_POLLS>(smem_u32(&bar_mma[0]), (uint32_t)turn & 1u)) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (tid == 0 && ok) {  // the next block while this one is read out
-          if (h + 1 < A.nch) load_b(c, h + 1, 0);
-          else if (c + 1 < c_end) load_b(c + 1, 0, 0);
+        if (tid == 0 && ok && (h + 1 < A.nch || c + 1 < c_end)) {  // the next block while this one is read out
+          load_b(h + 1 < A.nch ? c : c + 1, h + 1 < A.nch ? h + 1 : 0, 0);
+          ++loads;
         }
       }
-      if (!ok) break;
-      readout(c, 0u, false);
+      if (!ok) prefetch(first_col(c), first_at(c));
+      readout(c, 0u, false, ok);
       // the accumulators are read before products into them
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
+    if (tid == 0) drain(0, loads, products);
   }
-  if (!ok && lane == 0) atomicExch(err, 1);
   if (A.mode == 3) {
     // the four threads of a line, in order
     double* sd = reinterpret_cast<double*>(smem + A.off_t);
@@ -482,13 +515,14 @@ constexpr int kSmemMost = 226 * 1024;
 
 template <int NU, bool kChunks>
 cudaError_t launch_slice(const SliceArgs& a, dim3 grid, size_t smem, const unsigned char* img, const double* A64,
-                         const double* v, const double* x, double* y, int* err, cudaStream_t st, int device) {
+                         const double* v, const double* x, double* y, cudaStream_t st, int device) {
   static std::atomic<unsigned long long> done{0};
   const cudaError_t attr = pg::once_per_device(done, device, [] {
     return cudaFuncSetAttribute(k_slice_axis<NU, kChunks>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
   });
   if (attr != cudaSuccess) return attr;
-  return pg::launch_dependent(k_slice_axis<NU, kChunks>, grid, dim3(kST + (kChunks ? 0 : 32)), smem, st, a, img, A64, v, x, y, err);
+  return pg::launch_dependent(k_slice_axis<NU, kChunks>, grid, dim3(kST + (kChunks ? 0 : 32)), smem, st, a,
+                              img, A64, v, x, y);
 }
 
 }  // namespace
@@ -598,8 +632,7 @@ namespace {
 // Launches the contraction of nlines lines (stride inner); mode 3 writes
 // *rows rows of nlines partial dots.
 pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, const double* A64, bool trans,
-                       const double* v, const double* x, double* y, int mode, int* rows, int* err, cudaStream_t st,
-                       int device) {
+                       const double* v, const double* x, double* y, int mode, int* rows, cudaStream_t st, int device) {
   SliceArgs a{};
   a.n = S.n;
   a.inner = inner;
@@ -650,9 +683,9 @@ pg_status slice_launch(long nlines, long inner, long npts, const SliceMat& S, co
     a.mode = h0 == 0 || mode == 3 ? mode : 1;
     a.out0 = (long)launches * split * nlines;
     cudaError_t e;
-    if (chunks) e = launch_slice<2, true>(a, grid, smem, S.img, A64, v, x, y, err, st, device);
-    else if (S.kc <= 32) e = launch_slice<1, false>(a, grid, smem, S.img, A64, v, x, y, err, st, device);
-    else e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, err, st, device);
+    if (chunks) e = launch_slice<2, true>(a, grid, smem, S.img, A64, v, x, y, st, device);
+    else if (S.kc <= 32) e = launch_slice<1, false>(a, grid, smem, S.img, A64, v, x, y, st, device);
+    else e = launch_slice<2, false>(a, grid, smem, S.img, A64, v, x, y, st, device);
     PG_CUDA_TRY(e);
     PG_TRY(check_launch("k_slice_axis"));
   }
@@ -666,7 +699,7 @@ pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double
                      const double* x, double* y, int nvec, int mode, cudaStream_t st) {
   PG_ARG(S.img && S.n == g->n[axis], "slice_axis: no operand images");
   const long inner = axis == 0 ? 1 : (axis == 1 ? g->n[0] : (long)g->n[0] * g->n[1]);
-  return slice_launch(g->N / S.n * nvec, inner, g->N, S, A64, false, v, x, y, mode, nullptr, g->tc_err.p, st, g->device);
+  return slice_launch(g->N / S.n * nvec, inner, g->N, S, A64, false, v, x, y, mode, nullptr, st, g->device);
 }
 
 int slice_row_count(int n) {
@@ -702,7 +735,7 @@ pg_status slice_rows_matrix(const double* A64, unsigned char* img, SliceMat* S, 
 
 pg_status slice_rows(const pg_grid* g, long nlines, const SliceMat& S, const double* A64, const double* x, double* y,
                      SliceRows mode, int* rows, cudaStream_t st) {
-  return slice_launch(nlines, 1, nlines * S.n, S, A64, true, nullptr, x, y, mode, rows, g->tc_err.p, st, g->device);
+  return slice_launch(nlines, 1, nlines * S.n, S, A64, true, nullptr, x, y, mode, rows, st, g->device);
 }
 
 }  // namespace pg

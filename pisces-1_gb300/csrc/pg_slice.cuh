@@ -157,7 +157,7 @@ pg_status slice_axis(const pg_grid* g, int axis, const SliceMat& S, const double
 // Rows times a matrix: X is nlines x n (row-major), A n x n.
 // kRowStore: Y = X A.  kRowDot: Y holds *rows rows of nlines values whose sum
 // over the rows is x . (x A) for each line (at most slice_row_count(n)).
-// A64 and the images (slice_rows_matrix) on the device; g gives the status word.
+// A64 and the images (slice_rows_matrix) on the device of g.
 enum SliceRows { kRowStore = 0, kRowDot = 3 };
 int slice_row_count(int n);
 // Shape and bytes of the images of an n x n matrix whose largest entry is big
