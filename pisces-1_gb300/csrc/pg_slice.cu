@@ -12,15 +12,15 @@
 // Bounds: per point and axis about 40 integer operations to make the digits,
 // 95 to join the accumulators and one or two FP64 operations (V X, the sum
 // into Y), against n FP64 multiply-adds before; the FP64 pipe is about 60
-// times slower than the integer pipes here.  No one part sets the time: of
-// 23.4 us for an axis of 64^3 x 4 (a tile per CTA) the products cost 1.4 us
-// beside the rest, the joins 2.6, the digits 2.0; the others are the latencies
-// of the lines' loads, of each N chunk's read-out and of its sum into Y.
+// times slower than the integer pipes here.  No one part sets the time: of an
+// axis of 64^3 x 4 (a tile per CTA) the products cost 6 % beside the rest, the
+// joins 11 %, the digits 9 %; the others are the latencies of the lines' loads,
+// of each N chunk's read-out and of its sum into Y.
 //
 // H X, us, FP64 multiply-adds / slices of seven 9-bit digits (whose operands
-// and sums were not exact, pg_slice.cuh) / as here: 32^3 34.0 / 19.9 / 23.0,
-// 64^3 x 4 371 / 53.0 / 70.2, 83x90x71 x 6 1816 / 173 / 341, 96^3 x 8 3435 / 341
-// / 617, 160^3 x 16 (K chunks, two launches an axis) 63100 / 5505 / 12315.
+// and sums were not exact, pg_slice.cuh) / as here: 32^3 34.0 / 19.9 / 21.3,
+// 64^3 x 4 371 / 53.0 / 62.6, 83x90x71 x 6 1816 / 173 / 323, 96^3 x 8 3435 / 341
+// / 579, 160^3 x 16 (K chunks, two launches an axis) 63100 / 5505 / 11556.
 #include <algorithm>
 #include <cmath>
 
@@ -266,9 +266,10 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     if (loads > 0) mbar_wait(smem_u32(&bar_b[b]), (uint32_t)((loads - 1) & 1));
     if (products > 0) mbar_wait(smem_u32(&bar_mma[b]), (uint32_t)((products - 1) & 1));
   };
-  // The four outputs of a read-out batch: four columns of the thread's own
-  // line, or, where lines are contiguous and the batch is transposed, columns
-  // of neighbouring lines; addresses p + step[q].
+  // The four outputs of a read-out batch, joined two at a time (the accumulators
+  // of all four at once spilled: 64^3 x 4 73 us, so 63): four columns of the
+  // thread's own line, or, where lines are contiguous and the batch is
+  // transposed, columns of neighbouring lines; addresses p + step[q].
   const bool reads = 32 * (warp & 3) < A.lc;  // this warp's lanes hold lines
   const bool valid = row < lend;
   const long base = first_point(row);
@@ -320,30 +321,33 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     int i = first_col(c);
     long p = first_at(c);
     for (int bt = wpart; bt < nbatch; bt += 4, i += 16, p += 16 * istep) {
-      uint32_t r[pg::kSliceAcc][4] = {};
-      if (mma) {
-#pragma unroll
-        for (int d = 0; d < pg::kSliceAcc; ++d)
-          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                       : "=r"(r[d][0]), "=r"(r[d][1]), "=r"(r[d][2]), "=r"(r[d][3])
-                       : "r"(trow + tset + (uint32_t)(d * A.nc + 4 * bt)));
-      }
       double a0[4], b0[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) a0[q] = pa[q], b0[q] = pb[q];
       if (bt + 4 < nbatch) prefetch(i + 16, p + 16 * istep);
       else if (more) prefetch(first_col(c + 1), first_at(c + 1));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int d = 0; d < pg::kSliceAcc; ++d)  // the values are read after the wait
-        asm volatile("" : "+r"(r[d][0]), "+r"(r[d][1]), "+r"(r[d][2]), "+r"(r[d][3]));
       double k[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float a[pg::kSliceAcc];
+      for (int g = 0; g < 4; g += 2) {
+        uint32_t r[pg::kSliceAcc][2];
+        if (mma) {
 #pragma unroll
-        for (int d = 0; d < pg::kSliceAcc; ++d) a[d] = __uint_as_float(r[d][q]);
-        k[q] = pg::slice_join(a, A.scale + emax);
+          for (int d = 0; d < pg::kSliceAcc; ++d)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];"
+                         : "=r"(r[d][0]), "=r"(r[d][1])
+                         : "r"(trow + tset + (uint32_t)(d * A.nc + 4 * bt + g)));
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int d = 0; d < pg::kSliceAcc; ++d)  // the values are read after the wait
+          asm volatile("" : "+r"(r[d][0]), "+r"(r[d][1]));
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float a[pg::kSliceAcc];
+#pragma unroll
+          for (int d = 0; d < pg::kSliceAcc; ++d) a[d] = __uint_as_float(r[d][q]);
+          k[g + q] = pg::slice_join(a, A.scale + emax);
+        }
       }
       if (slow && valid) {
 #pragma unroll
