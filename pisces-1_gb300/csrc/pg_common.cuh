@@ -281,7 +281,7 @@ struct pg_grid {
   int t16_scale = 0;
   pg::DevBuf<double> x_dev[3];     // grid points on the device
   pg::StatusWord tc_err;           // set by the tensor-core kernels if a completion wait times out
-  bool same_t = false;             // the three axes share one kinetic matrix
+  bool same_t = false;             // the three axes share one kinetic matrix (slice_grid)
   // eigenbasis of the kinetic matrices (the orthonormal DST-I, symmetric),
   // for the kinetic preconditioner: FP64, TF32 hi/lo, and the eigenvalues
   pg::DevBuf<double> q_dev[3];

@@ -373,7 +373,6 @@ extern "C" pg_status pg_grid_create_dvr(const int n[3], const double L[3], int d
     delete g;
     return PG_OOM;
   }
-  g->same_t = n[0] == n[1] && n[0] == n[2] && g->t[0] == g->t[1] && g->t[0] == g->t[2];
   {
     const pg_status ss = pg::slice_grid(g);
     if (ss != PG_OK) {

@@ -23,6 +23,7 @@
 // / 579, 160^3 x 16 (K chunks, two launches an axis) 63100 / 5505 / 11556.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "pg_slice.cuh"
 #include "pg_tc16.cuh"
@@ -553,17 +554,25 @@ static void slice_shape(int n, SliceMat* S) {
 // further than r bits below the largest, which the slices round by 2^(r - 26)
 // of an FP64 rounding (kSliceGuard bits are to spare), two such roundings (T
 // and the line) against n.  The sine DVR keeps to this up to about 750 points.
-static bool slice_exact(const std::vector<double>& t) {
-  double big = 0, small = INFINITY;
-  for (double x : t) {
-    if (!std::isfinite(x)) return false;
-    const double a = fabs(x);
-    big = std::max(big, a);
-    if (a > 0) small = std::min(small, a);
+// big: the largest entry.
+static bool slice_exact(const std::vector<double>& t, double* big) {
+  // magnitudes compare as integers; the smallest above zero as bits - 1
+  uint64_t most = 0, least = ~0ull;
+  for (const double& x : t) {
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    u &= 0x7fffffffffffffffull;
+    most = std::max(most, u);
+    least = std::min(least, u - 1);
   }
-  if (big == 0) return true;
-  return big < 1e270 && small > 1e-270 &&
-         std::ilogb(big) - std::ilogb(small) <= kSliceGuard + std::ilogb(sqrt((double)t.size())) - 1;
+  double small;
+  memcpy(big, &most, 8);
+  if (most >= 0x7ff0000000000000ull) return false;
+  if (most == 0) return true;
+  ++least;
+  memcpy(&small, &least, 8);
+  return *big < 1e270 && small > 1e-270 &&
+         std::ilogb(*big) - std::ilogb(small) <= kSliceGuard + std::ilogb(sqrt((double)t.size())) - 1;
 }
 
 // T, Q^T and Q of the three axes; the host copies give the largest entry
@@ -572,16 +581,23 @@ pg_status slice_grid(pg_grid* g) {
   SliceBuild B{};
   SliceMat* S[9];
   int share[9], count = 0;
-  g->t_sliced = slice_exact(g->t[0]) && slice_exact(g->t[1]) && slice_exact(g->t[2]);
+  // an axis with the points and kinetic matrix of one before it has its images too
+  int like[3] = {-1, -1, -1};
+  double big[3];
+  g->t_sliced = true;
+  for (int a = 0; a < 3; ++a) {
+    for (int b = 0; b < a && like[a] < 0; ++b)
+      if (g->n[b] == g->n[a] && like[b] < 0 && g->t[b] == g->t[a]) like[a] = b;
+    if (like[a] >= 0) big[a] = big[like[a]];
+    else g->t_sliced &= slice_exact(g->t[a], &big[a]);
+  }
+  g->same_t = like[1] == 0 && like[2] == 0;
   size_t off[9], total = 0;
   for (int m = 0; m < 9; ++m) {
     const int a = m % 3;
     S[m] = m < 3 ? &g->t_sl[a] : (m < 6 ? &g->q_sl[a] : &g->qb_sl[a]);
     slice_shape(g->n[a], S[m]);
-    // an axis with the points and kinetic matrix of one before it has its images too
-    share[m] = -1;
-    for (int b = 0; b < a && share[m] < 0; ++b)
-      if (g->n[b] == g->n[a] && g->t[b] == g->t[a]) share[m] = m - a + b;
+    share[m] = like[a] >= 0 ? m - a + like[a] : -1;
     if (share[m] < 0 && m >= 6 && g->dvrtype != 3) share[m] = m - 3;  // the DST-I is symmetric
     while (share[m] >= 0 && share[share[m]] >= 0) share[m] = share[share[m]];
     if (m < 3 && !g->t_sliced) continue;  // no images of T
@@ -593,14 +609,9 @@ pg_status slice_grid(pg_grid* g) {
   int most = 0;
   for (int m = 0; m < 9; ++m) {
     const int a = m % 3;
-    double big = 1.0;
-    if (m < 3) {
-      big = 0;
-      for (double t : g->t[a]) big = std::max(big, fabs(t));
-      if (!g->t_sliced) continue;
-    }
+    if (m < 3 && !g->t_sliced) continue;
     int ex = 0;
-    frexp(big, &ex);  // big < 2^ex, its biased exponent ex + 1022
+    frexp(m < 3 ? big[a] : 1.0, &ex);  // big < 2^ex, its biased exponent ex + 1022
     S[m]->tau = kSliceN * kSliceP - 1 - ex;
     S[m]->img = g->sl_img.p + (share[m] < 0 ? off[m] : off[share[m]]);
     if (share[m] >= 0) continue;
