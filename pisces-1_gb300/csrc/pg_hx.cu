@@ -3,15 +3,17 @@
 // H = diag(V) + Tx (+) Ty (+) Tz: for every grid point and vector,
 //   y = v x + sum_b Tx[i,b] x[b,j,k] + sum_b Ty[j,b] x[i,b,k] + sum_b Tz[k,b] x[i,j,b]
 // (src/mtx.cpp:35-104 applies the same operator line by line with dspmv).
-// Three axis contractions from exact slices on the tensor cores
+// Three axis contractions from slices of both operands on the tensor cores
 // (pg_slice.cu): z with V X, then y and x added to Y.
 //
 // k_hx_fp64 and k_axis_fp64 are the same contractions as chains of FP64
-// multiply-adds in a fixed order, bound by that pipe (371 us against 54 at
-// 64^3 x 4).  They serve the FP64 solver of several roots, whose states come
-// out of a restart with signs that the rounding noise of the products
-// decides: with another product the states are the same to 1e-14, but a third
-// of them change sign, and a solve keeps the states it has always returned.
+// multiply-adds in a fixed order, bound by that pipe (344 us against 63 at
+// 64^3 x 4, the pipe 98 % active).  They serve the FP64 solver of several
+// roots, whose states come out of a restart with signs that the rounding noise
+// of the products decides: with another product the states are the same to
+// 1e-14, but a third of them change sign, and a solve keeps the states it has
+// always returned; and they serve grids that are very small, or whose T the
+// slices do not hold (chain_is_shorter, t_sliced).
 #include <algorithm>
 #include <type_traits>
 

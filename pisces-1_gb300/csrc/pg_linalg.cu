@@ -1,8 +1,10 @@
 // Deterministic skinny FP64 kernels for the Davidson subspace (see pg_linalg.cuh).
 //
-// Every reduction runs in two launches: blocks of the first write partial
-// sums (one per output), the second reduces the partials of each output with
-// one warp, in a fixed order.  No atomics, no dependence on scheduling.
+// Blocks write partial sums (one per output); the partials of each output are
+// reduced by one warp in a fixed order, by a second launch (Gram products) or
+// by the block that an arrival counter finds to be the last (norms, k_ritz_df,
+// and the coefficients of a Gram-Schmidt pass after its second launch).  Which
+// block that is does not change the sums: no dependence on scheduling.
 #include <algorithm>
 #include <cstdint>
 #include <mutex>

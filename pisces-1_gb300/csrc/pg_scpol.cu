@@ -9,8 +9,8 @@
 // (Potential::SelfConsistentPolarizability, src/Potential.cpp:1495-1628).
 //
 // Over the grid the dipoles are one dense product MU = E A (N x 3npp times
-// 3npp x 3npp), in FP64 precision on the tensor cores from exact slices
-// (pg_slice.cu; 8 waters on 48^3: 1.89 ms as FP64 multiply-adds, 0.15 ms so).
+// 3npp x 3npp), in FP64 precision on the tensor cores from slices of both
+// (pg_slice.cu; 8 waters on 48^3: 1.89 ms as FP64 multiply-adds, 0.32 ms so).
 // V_pol is that product's read-out: each CTA forms the row dots E . MU of its
 // points, and a second pass sums the few partial dots of a point in a fixed
 // order (no atomics; bit-stable).
