@@ -149,6 +149,14 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     return contig ? l * A.n : (l / A.inner) * A.inner * A.n + l % A.inner;
   };
   const int koct = A.kc >> 3;
+  // Octets of a K chunk that hold values, in whole K steps: of several, the last
+  // one may end early, and so may the last N chunk's batches (72^3 x 4 274 us with
+  // the padding, 245 so; one chunk is the axis itself, and a bound that is not
+  // the same for all its N chunks costs 64^3 x 4 63 -> 69).
+  auto octets = [&](int h) {
+    const int kn = A.n - (A.h0 + h) * A.kc;
+    return kChunks && kn < A.kc ? ((kn + 15) >> 4) << 1 : koct;
+  };
   const int k_end = (A.h0 + A.nch) * A.kc < A.n ? (A.h0 + A.nch) * A.kc : A.n;
 
   double val[NU][8];
@@ -207,14 +215,15 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
   const uint32_t lbo = 128, sbo = (uint32_t)koct * 128u;
   const uint32_t a_slice = (uint32_t)kLines * (uint32_t)A.kc * 2u;
   // digits: one 16-byte row of a core matrix per slice and octet
-  auto convert = [&] {
+  auto convert = [&](int h) {
+    const int ko = octets(h);
     const int em = s_emax[line];
     const bool slow = is_slow(em);
     const int emax = slow ? 0 : em;
 #pragma unroll
     for (int u = 0; u < NU; ++u) {
       const int o = part + parts * u;
-      if (o < koct) {
+      if (o < ko) {
         uint32_t w[NS][4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -238,18 +247,19 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
   // memory as one operand of (10 - i) nc rows, in accumulators i .. 9, which
   // lie side by side: at most 256 columns an instruction (one product at a
   // time reads the lines' digits once for each).
-  auto issue = [&](int b, uint32_t parity, bool first) {
+  auto issue = [&](int b, uint32_t parity, int h) {
     if (!wait_for<PG_SLICE_POLLS_ISSUE>(smem_u32(&bar_b[b]), parity)) return false;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint64_t dA = smem_desc(sA, lbo, sbo), dB = smem_desc(sB + (uint32_t)b * A.block_bytes, lbo, sbo);
     const uint32_t id0 = (1u << 4) | ((uint32_t)(kLines >> 4) << 24);
     const uint32_t d0 = tmem + (uint32_t)b * (A.tmem_cols >> 1);
-    for (int kk = 0; kk < (koct >> 1); ++kk) {
+    const int steps = octets(h) >> 1;
+    for (int kk = 0; kk < steps; ++kk) {
 #pragma unroll
       for (int i = 0; i < NS; ++i) {
         const uint64_t da = dA + (((uint32_t)i * a_slice + (uint32_t)kk * 256u) >> 4);
         const int all = (NS - i) * A.nc;
-        const uint32_t acc = (!first || kk > 0 || i > 0) ? 1u : 0u;
+        const uint32_t acc = (h > 0 || kk > 0 || i > 0) ? 1u : 0u;
         mma_f16(d0 + (uint32_t)(i * A.nc), da, dB + (uint32_t)kk * 16u,
                 id0 | ((uint32_t)((all < 256 ? all : 256) >> 3) << 17), acc);
         if (kChunks && all > 256)
@@ -321,7 +331,7 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
     const int emax = slow ? 0 : em;
     int i = first_col(c);
     long p = first_at(c);
-    for (int bt = wpart; bt < nbatch; bt += 4, i += 16, p += 16 * istep) {
+    for (int bt = wpart; bt < nbatch && (!kChunks || i < A.n); bt += 4, i += 16, p += 16 * istep) {
       double a0[4], b0[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) a0[q] = pa[q], b0[q] = pb[q];
@@ -404,7 +414,7 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
       load_chunk(0);
       chunk_emax();
       named_sync(1, kST);  // the maxima are complete, the staging area is read
-      convert();
+      convert(0);
     }
     __syncthreads();
     if (warp < kST / 32) {
@@ -437,7 +447,7 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        ok = issue(b, (uint32_t)(use & 1), true);
+        ok = issue(b, (uint32_t)(use & 1), 0);
         if (ok) ++products[b];
       }
       for (int b = 0; b < 2; ++b) drain(b, loads[b], products[b]);
@@ -453,10 +463,10 @@ __global__ void __launch_bounds__(kST + (kChunks ? 0 : 32), 1)
       for (int h = 0; h < A.nch && ok; ++h, ++turn) {
         load_chunk(h);
         __syncthreads();  // the staging area is read
-        convert();
+        convert(h);
         __syncthreads();
         if (tid == 0) {
-          if (issue(0, (uint32_t)turn & 1u, h == 0)) ++products;
+          if (issue(0, (uint32_t)turn & 1u, h)) ++products;
         }
         if (h + 1 == A.nch) prefetch(first_col(c), first_at(c));
         ok = __syncthreads_and(wait_for<PG_SLICE_POLLS>(smem_u32(&bar_mma[0]), (uint32_t)turn & 1u)) != 0;
