@@ -92,23 +92,28 @@ __global__ void __launch_bounds__(256) k_hx_fp64(int nx, int ny, int nz, const d
   else hx_point<REST == 0 ? 4 : REST>(nx, ny, nz, tx, ty, tz, v, X + off, Y + off, N, g);
 }
 
-// Y (mode) A x_axis X: one axis contraction in FP64, mode 0 write, 1 add.
+// Y (mode) A x_axis X: one axis contraction in FP64, mode 0 write, 1 add, for
+// vectors v0 .. v0 + nv - 1.  The bodies as above; the groups of four keep
+// their predicates (nv is not a constant there): without them the compiler runs
+// more loads ahead and the pass is slower (six passes, 96^3 x 8: 6.84 ms, 8.13).
 template <int NV>
 __device__ __forceinline__ void axis_point(int na, int idx, long stride, const double* __restrict__ A,
-                                           const double* __restrict__ Xv, double* __restrict__ Yv, long N, long g,
-                                           int mode) {
+                                           const double* __restrict__ X, double* __restrict__ Y, long N, long g,
+                                           int mode, int v0, int nv) {
   const long base = g - (long)idx * stride;
   double acc[NV];
 #pragma unroll
-  for (int q = 0; q < NV; ++q) acc[q] = mode == 1 ? Yv[(long)q * N + g] : 0.0;
+  for (int q = 0; q < NV; ++q) acc[q] = (q < nv && mode == 1) ? Y[(long)(v0 + q) * N + g] : 0.0;
   const double* arow = A + (long)idx * na;
   for (int b = 0; b < na; ++b) {
     const double t = arow[b];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) acc[q] += t * Xv[(long)q * N + base + (long)b * stride];
+    for (int q = 0; q < NV; ++q)
+      if (q < nv) acc[q] += t * X[(long)(v0 + q) * N + base + (long)b * stride];
   }
 #pragma unroll
-  for (int q = 0; q < NV; ++q) Yv[(long)q * N + g] = acc[q];
+  for (int q = 0; q < NV; ++q)
+    if (q < nv) Y[(long)(v0 + q) * N + g] = acc[q];
 }
 
 template <int REST>
@@ -125,9 +130,9 @@ __global__ void __launch_bounds__(256) k_axis_fp64(int nx, int ny, int nz, int a
   const int na = axis == 0 ? nx : (axis == 1 ? ny : nz);
   const int idx = axis == 0 ? i : (axis == 1 ? j : k);
   const long stride = axis == 0 ? 1 : (axis == 1 ? nx : (long)nx * ny);
-  const long off = 4l * blockIdx.y * N;
-  if (REST == 0 || (int)blockIdx.y < four) axis_point<4>(na, idx, stride, A, X + off, Y + off, N, g, mode);
-  else axis_point<REST == 0 ? 4 : REST>(na, idx, stride, A, X + off, Y + off, N, g, mode);
+  const int v0 = 4 * blockIdx.y, nv = 4 * four + REST - v0;
+  if (REST == 0 || (int)blockIdx.y < four) axis_point<4>(na, idx, stride, A, X, Y, N, g, mode, v0, nv < 4 ? nv : 4);
+  else axis_point<REST == 0 ? 4 : REST>(na, idx, stride, A, X, Y, N, g, mode, v0, REST);
 }
 
 }  // namespace
