@@ -927,8 +927,11 @@ inline bool pair_ok(long N, const double* P, const double* Q) {
   return N % 2 == 0 && ((uintptr_t)P % 16) == 0 && ((uintptr_t)Q % 16) == 0;
 }
 
-// Dynamic shared-memory opt-in, once per kernel and device.
-static pg_status opt_in_smem() {
+// Shared-memory opt-in of the Gram kernels for a launch with smem dynamic bytes,
+// once per kernel and device; launches within the default (48 KB with the
+// static part) do without the look at the device.
+static pg_status opt_in_smem(size_t smem) {
+  if (smem <= 40 * 1024) return PG_OK;
   static std::atomic<unsigned long long> done{0};
   int dev = 0;
   PG_CUDA_TRY(cudaGetDevice(&dev));
@@ -953,6 +956,7 @@ static pg_status launch_gram(long N, long chunk, int blocks, const double* P, in
   };
   int logT = 2;
   while (logT > 0 && smem(logT) > (size_t)kGramSmemMax) --logT;
+  PG_TRY(opt_in_smem(smem(logT)));
   PG_CUDA_TRY(launch_dependent(k_gram, dim3(blocks), dim3(kT), smem(logT), st, N, chunk, P, na, Q, nb, logT, partial,
                                skip));
   return check_launch("k_gram");
@@ -963,12 +967,12 @@ pg_status gram(long N, const double* P, int na, const double* Q, int nb, double*
   PG_ARG(na > 0 && nb > 0 && na * nb <= kMaxGramOut && na + nb <= 144, "gram: %d x %d outputs exceed the limits",
          na, nb);
   PG_TRY(rs.ensure(st));
-  PG_TRY(opt_in_smem());
   const long chunk = chunk_for(N, kRedBlocks, kTP);
   const int blocks = (int)((N + chunk - 1) / chunk);
   if (dfloat) {
     const GramGeom gg = gram_geometry(na, nb);
     PG_ARG(gg.nblk <= kT, "gram: %d output blocks", gg.nblk);  // at most ~160 within the limits above
+    PG_TRY(opt_in_smem(gg.smem));
     const long dchunk = chunk_for(N, kRedBlocks, gg.tp);
     const int dblocks = (int)((N + dchunk - 1) / dchunk);
     const double* Ps = Pt ? Pt : P;
@@ -1042,7 +1046,6 @@ pg_status combine(long N, const double* P, int na, const double* C, int ca, int 
   PG_ARG(nr > 0 && nr <= kMaxCombine && na >= 0 && na * nr <= 128 * kMaxCombine, "combine: bad sizes na=%d nr=%d",
          na, nr);
   PG_TRY(rs.ensure(st));
-  PG_TRY(opt_in_smem());
   const long chunk = chunk_for(N, kStreamBlocks, kT);
   const int blocks = (int)((N + chunk - 1) / chunk);
   if (dfloat) {
@@ -1320,12 +1323,12 @@ extern "C" pg_status pg_block_gram_noalloc(long n, const double* P, int np, cons
     }
     partial = g_noalloc_ptr[dev];
   }
-  PG_TRY(opt_in_smem());
   cudaStream_t st = as_stream(stream);
   const int no = np * nq;
   if (precision == PG_MIXED) {
     const GramGeom gg = gram_geometry(np, nq);
     PG_ARG(gg.nblk <= kT, "pg_block_gram_noalloc: %d output blocks", gg.nblk);
+    PG_TRY(opt_in_smem(gg.smem));
     const long chunk = chunk_for(n, pg::kRedBlocks, gg.tp);
     const int blocks = (int)((n + chunk - 1) / chunk);
     if (pair_ok(n, P, Q))
