@@ -19,8 +19,8 @@
 //
 // H X, us, FP64 multiply-adds / slices of seven 9-bit digits (whose operands
 // and sums were not exact, pg_slice.cuh) / as here: 32^3 34.0 / 19.9 / 21.3,
-// 64^3 x 4 371 / 53.0 / 62.6, 83x90x71 x 6 1816 / 173 / 323, 96^3 x 8 3435 / 341
-// / 579, 160^3 x 16 (K chunks, two launches an axis) 63100 / 5505 / 11556.
+// 64^3 x 4 344 / 53.0 / 62.8, 83x90x71 x 6 1816 / 173 / 307, 96^3 x 8 3320 / 341
+// / 581, 160^3 x 16 (K chunks, two launches an axis) 63100 / 5505 / 10360.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
